@@ -1,11 +1,11 @@
 // fp64.cu -- the double-precision state path (plan precision FULLMAG_FDM_PRECISION_DOUBLE).
 //
 // State, stage derivatives, fields, the FFT convolution and every reduction are FP64.
-// The structure is one kernel per operation, like the reference's FP64 backend, with
-// this engine's own pieces: a mixed-radix FP64 FFT on lines in shared memory (no
-// cuFFT), the real, octant-unique demag kernel of the FP32 path held in FP64, and the
-// FP64 GPU Newell builder when the caller passes no spectra.  This path exists for
-// accuracy, not speed: GB300 issues FP64 at a small fraction of its FP32 rate.
+// The passes are those of the FP32 path -- a fused row pass and the column passes of the
+// convolution, with this engine's own mixed-radix FP64 line transforms in shared memory (no
+// cuFFT), the real, octant-unique demag kernel held in FP64, and the FP64 GPU Newell builder
+// when the caller passes no spectra.  GB300 issues FP64 at a small fraction of its FP32 rate,
+// so the work per point is chosen for the fewest FP64 instructions.
 //
 // Reference behaviour restated (paths in mzrptu/fullmag):
 //   precision switch, plan validation          native/backends/fdm/src/api.cpp:97,324-395,533
@@ -42,7 +42,8 @@ constexpr int kT = 256;
 constexpr double kMu0d = 4.0 * M_PI * 1e-7;
 constexpr int kMaxRadixStages = 32;
 constexpr int kStats = 9;  // e_ex e_d e_ext e_uni e_cub | max|Heff|^2 max|Hd|^2 max|k|^2 max err^2
-constexpr int kRedBlocks = 1024;
+constexpr int kMaxBlocks = 1024;          // grid-stride conversions
+constexpr size_t kMaxSmem = 227 * 1024;   // shared memory of one CTA
 
 struct Plan64 {
     int n;
@@ -57,51 +58,204 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 __device__ __forceinline__ double2 zconj(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double2 ztw(const double2 *tw, int e, bool inv) {
-    const double2 w = tw[e];
-    return inv ? zconj(w) : w;
+template <bool INV>
+__device__ __forceinline__ double2 ztw(const double2 *tw, int e) {
+    const double2 w = __ldg(tw + e);
+    return INV ? zconj(w) : w;
+}
+// times -i (forward) or +i (inverse)
+template <bool INV>
+__device__ __forceinline__ double2 zmi(double2 a) {
+    return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
 
-// One line of length p.n in shared memory, transformed by the whole CTA with Stockham
-// stages (natural order in and out); returns the buffer holding the result.  Radix 4
-// and 2 have their own butterflies; any other radix R is an O(R^2) DFT read from the
-// table at stride n / R.  Contains __syncthreads: every thread of the CTA calls it.
-__device__ double2 *fft_line64(double2 *a, double2 *b, const Plan64 &p, bool inv) {
+// ---- FP64 line transforms ----
+// GB300 issues FP64 at 1/64 of its FP32 rate, so these passes are bound by the number of
+// FP64 instructions and by little else: shared-memory exchanges, index arithmetic and bank
+// conflicts of 16-byte elements hide behind them.  Hence radix-8 butterflies (10.5
+// instructions per point for three binary levels, twiddles included, against 7 for two with
+// radix 4), odd radices as folded symmetric sums (R-1)^2 + O(R) multiply-adds instead of
+// R^2 complex products, and half transforms where one half of a line is zero or unwanted.
+
+// R-point DFT in place.  HIN: the upper R/2 inputs are zero; HOUT: only the lower R/2
+// outputs are wanted.  tw: the table of the line's length n, W_R^e = tw[e n / R] (odd R).
+template <int R, bool INV, bool HIN, bool HOUT>
+__device__ __forceinline__ void dft64(double2 (&v)[R], const double2 *__restrict__ tw, int rs) {
+    if constexpr (R == 2) {
+        if constexpr (HIN) {
+            v[1] = v[0];
+        } else {
+            const double2 a = v[0], b = v[1];
+            v[0] = zadd(a, b);
+            if constexpr (!HOUT) v[1] = zsub(a, b);
+        }
+    } else if constexpr (R == 4) {
+        if constexpr (HIN) {
+            const double2 a = v[0], b = v[1], ib = zmi<INV>(b);
+            v[0] = zadd(a, b);
+            v[2] = zsub(a, b);
+            v[1] = zadd(a, ib);
+            v[3] = zsub(a, ib);
+        } else {
+            const double2 a0 = zadd(v[0], v[2]), a1 = zsub(v[0], v[2]);
+            const double2 b0 = zadd(v[1], v[3]), b1 = zmi<INV>(zsub(v[1], v[3]));
+            v[0] = zadd(a0, b0);
+            v[1] = zadd(a1, b1);
+            if constexpr (!HOUT) {
+                v[2] = zsub(a0, b0);
+                v[3] = zsub(a1, b1);
+            }
+        }
+    } else if constexpr (R == 8) {
+        const double h = 0.70710678118654752440;
+        double2 e[4], o[4];
+        if constexpr (HOUT) {
+            // decimation in time: y[t] = E[t] + W8^t O[t], t < 4
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                e[t] = v[2 * t];
+                o[t] = v[2 * t + 1];
+            }
+            dft64<4, INV, false, false>(e, tw, rs);
+            dft64<4, INV, false, false>(o, tw, rs);
+            const double2 q1 = zmi<INV>(o[1]), q3 = zmi<INV>(o[3]);
+            o[1] = make_double2(h * (o[1].x + q1.x), h * (o[1].y + q1.y));
+            o[2] = zmi<INV>(o[2]);
+            o[3] = make_double2(h * (q3.x - o[3].x), h * (q3.y - o[3].y));
+#pragma unroll
+            for (int t = 0; t < 4; ++t) v[t] = zadd(e[t], o[t]);
+        } else {
+            // decimation in frequency: even outputs from v[t] + v[t+4], odd ones from
+            // W8^t (v[t] - v[t+4])
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                e[t] = HIN ? v[t] : zadd(v[t], v[t + 4]);
+                o[t] = HIN ? v[t] : zsub(v[t], v[t + 4]);
+            }
+            const double2 q1 = zmi<INV>(o[1]), q3 = zmi<INV>(o[3]);
+            o[1] = make_double2(h * (o[1].x + q1.x), h * (o[1].y + q1.y));
+            o[2] = zmi<INV>(o[2]);
+            o[3] = make_double2(h * (q3.x - o[3].x), h * (q3.y - o[3].y));
+            dft64<4, INV, false, false>(e, tw, rs);
+            dft64<4, INV, false, false>(o, tw, rs);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                v[2 * t] = e[t];
+                v[2 * t + 1] = o[t];
+            }
+        }
+    } else {
+        // odd R: with s_t = v_t + v_{R-t}, d_t = v_t - v_{R-t},
+        //   X_q, X_{R-q} = v_0 + sum_t cos(2 pi q t / R) s_t  -+ i sum_t sin(2 pi q t / R) d_t
+        constexpr int H = (R - 1) / 2;
+        double2 s[H], d[H];
+        double2 x0 = v[0];
+        const double2 v0 = v[0];
+#pragma unroll
+        for (int t = 0; t < H; ++t) {
+            s[t] = zadd(v[1 + t], v[R - 1 - t]);
+            d[t] = zsub(v[1 + t], v[R - 1 - t]);
+            x0 = zadd(x0, s[t]);
+        }
+        v[0] = x0;
+#pragma unroll
+        for (int q = 1; q <= H; ++q) {
+            double2 c = v0, z = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int t = 0; t < H; ++t) {
+                const double2 w = __ldg(tw + ((q * (t + 1)) % R) * rs);  // (cos, -sin)
+                c.x += w.x * s[t].x;
+                c.y += w.x * s[t].y;
+                z.x += w.y * d[t].x;
+                z.y += w.y * d[t].y;
+            }
+            // i z for the forward transform (w.y = -sin), -i z for the inverse
+            const double2 iz = INV ? make_double2(z.y, -z.x) : make_double2(-z.y, z.x);
+            v[q] = zadd(c, iz);
+            v[R - q] = zsub(c, iz);
+        }
+    }
+}
+
+// One Stockham stage of radix R over nl lines of length n (line l at l * ls); twiddles on
+// every stage but the first (Ns == 1).
+template <int R, bool INV, bool HIN, bool HOUT>
+__device__ __forceinline__ void stage64(const double2 *__restrict__ in, double2 *__restrict__ out, int nl, int ls, int n,
+                                        int Ns, const double2 *__restrict__ tw) {
+    const int nb = n / R, tws = n / (Ns * R);
+    for (int idx = threadIdx.x; idx < nl * nb; idx += blockDim.x) {
+        const int l = idx / nb, j = idx - l * nb;
+        const int q = j / Ns, k = j - q * Ns;
+        const double2 *src = in + l * ls + j;
+        double2 *dst = out + l * ls + q * Ns * R + k;
+        double2 v[R];
+#pragma unroll
+        for (int t = 0; t < (HIN ? R / 2 : R); ++t) v[t] = src[t * nb];
+        if (!HIN && Ns > 1) {
+#pragma unroll
+            for (int t = 1; t < R; ++t) v[t] = zmul(v[t], ztw<INV>(tw, t * k * tws));
+        }
+        dft64<R, INV, HIN, HOUT>(v, tw, nb);
+#pragma unroll
+        for (int t = 0; t < (HOUT ? R / 2 : R); ++t) dst[t * Ns] = v[t];
+    }
+}
+
+// prime radix above 13 (caller spectra or periodic extents with such a factor): O(R^2)
+template <bool INV>
+__device__ __noinline__ void stage64_generic(const double2 *__restrict__ in, double2 *__restrict__ out, int nl, int ls, int n,
+                                             int Ns, int R, const double2 *__restrict__ tw) {
+    const int nb = n / R, tws = n / (Ns * R);
+    for (int idx = threadIdx.x; idx < nl * n; idx += blockDim.x) {
+        const int l = idx / n, r = idx - l * n;
+        const int q = r / nb, j = r - q * nb;  // output q of butterfly j
+        const int k = j % Ns, o = (j / Ns) * Ns * R + k;
+        const double2 *src = in + l * ls + j;
+        double2 acc = make_double2(0.0, 0.0);
+        int e = 0;  // (t q) mod R
+        for (int t = 0; t < R; ++t) {
+            double2 x = src[t * nb];
+            if (Ns > 1 && t) x = zmul(x, ztw<INV>(tw, t * k * tws));
+            acc = zadd(acc, zmul(x, ztw<INV>(tw, e * nb)));
+            e += q;
+            if (e >= R) e -= R;
+        }
+        out[l * ls + o + q * Ns] = acc;
+    }
+}
+
+// nl lines of length p.n in shared memory (natural order in and out) by the whole CTA;
+// returns the buffer that holds the result.  The radices run in plan order forwards and in
+// reverse order backwards, so radix[0] is the first forward and the last inverse stage:
+// with `prune` (an even radix[0], data in the lower half only) those two work on half
+// lines.  Contains __syncthreads: every thread of the CTA calls it; the caller has
+// synchronised the buffers.
+template <bool INV>
+__device__ __forceinline__ double2 *fft_lines64(double2 *a, double2 *b, int nl, int ls, const Plan64 &p, bool prune) {
     int Ns = 1;
     const int n = p.n;
     for (int s = 0; s < p.ns; ++s) {
-        const int R = p.radix[s], nb = n / R, tws = n / (Ns * R), rs = n / R;
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-            const int k = j % Ns, o = (j / Ns) * Ns * R + k;
-            if (R == 2) {
-                double2 v0 = a[j], v1 = a[j + nb];
-                if (Ns > 1) v1 = zmul(v1, ztw(p.tw, k * tws, inv));
-                b[o] = zadd(v0, v1);
-                b[o + Ns] = zsub(v0, v1);
-            } else if (R == 4) {
-                double2 v[4];
-                for (int t = 0; t < 4; ++t) {
-                    v[t] = a[j + t * nb];
-                    if (Ns > 1 && t) v[t] = zmul(v[t], ztw(p.tw, t * k * tws, inv));
-                }
-                const double2 a0 = zadd(v[0], v[2]), a1 = zsub(v[0], v[2]), b0 = zadd(v[1], v[3]);
-                const double2 d = zsub(v[1], v[3]);
-                const double2 b1 = inv ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);
-                b[o] = zadd(a0, b0);
-                b[o + 2 * Ns] = zsub(a0, b0);
-                b[o + Ns] = zadd(a1, b1);
-                b[o + 3 * Ns] = zsub(a1, b1);
-            } else {
-                for (int q = 0; q < R; ++q) {
-                    double2 acc = make_double2(0.0, 0.0);
-                    for (int t = 0; t < R; ++t) {
-                        double2 x = a[j + t * nb];
-                        if (Ns > 1 && t) x = zmul(x, ztw(p.tw, t * k * tws, inv));
-                        acc = zadd(acc, zmul(x, ztw(p.tw, ((t * q) % R) * rs, inv)));
-                    }
-                    b[o + q * Ns] = acc;
-                }
-            }
+        const int R = p.radix[INV ? p.ns - 1 - s : s];
+        const bool half = prune && (INV ? s == p.ns - 1 : s == 0);
+        switch (R) {
+            case 8:
+                if (half) stage64<8, INV, !INV, INV>(a, b, nl, ls, n, Ns, p.tw);
+                else stage64<8, INV, false, false>(a, b, nl, ls, n, Ns, p.tw);
+                break;
+            case 4:
+                if (half) stage64<4, INV, !INV, INV>(a, b, nl, ls, n, Ns, p.tw);
+                else stage64<4, INV, false, false>(a, b, nl, ls, n, Ns, p.tw);
+                break;
+            case 2:
+                if (half) stage64<2, INV, !INV, INV>(a, b, nl, ls, n, Ns, p.tw);
+                else stage64<2, INV, false, false>(a, b, nl, ls, n, Ns, p.tw);
+                break;
+            case 3: stage64<3, INV, false, false>(a, b, nl, ls, n, Ns, p.tw); break;
+            case 5: stage64<5, INV, false, false>(a, b, nl, ls, n, Ns, p.tw); break;
+            case 7: stage64<7, INV, false, false>(a, b, nl, ls, n, Ns, p.tw); break;
+            case 11: stage64<11, INV, false, false>(a, b, nl, ls, n, Ns, p.tw); break;
+            case 13: stage64<13, INV, false, false>(a, b, nl, ls, n, Ns, p.tw); break;
+            default: stage64_generic<INV>(a, b, nl, ls, n, Ns, R, p.tw); break;
         }
         __syncthreads();
         double2 *t = a;
@@ -112,30 +266,107 @@ __device__ double2 *fft_line64(double2 *a, double2 *b, const Plan64 &p, bool inv
     return a;
 }
 
-__device__ __forceinline__ void mirror(int k, int p, int &km, double &sg) {
-    if (k > p / 2) {
-        km = p - k;
-        sg = -1.0;
-    } else {
-        km = k;
-        sg = 1.0;
-    }
-}
-
 struct Conv64 {
     int nx, ny, nz, px, py, pz, nkx, nky, nkz, thin;
     long long n;
-    Plan64 plx, ply, plz;
-    const double *kern;    // octant kernel scaled by Ms / P
+    int half;              // px / 2 when the x lines are packed (two real samples per complex one), else 0
+    int xprune, yprune, zprune;  // half-line first / last stages (fft_lines64)
+    Plan64 plx, ply, plz;  // plx: length half (packed) or px
+    const double2 *xpost;  // packed: e^{-2 pi i k / px}, k <= half
+    const double *kern;    // octant kernel scaled by Ms / P, and by 1/2 with packed x lines
     const double2 *kernc;  // periodic grids: complex kernel K[c][kz][ky][kx] (full ky, kz), else NULL
 };
 
-// row (y, z) and component c: phi m along x, zero padded to px -> X[c][row][kx < nkx]
+// U independent loads per thread in flight before the first is stored
+template <int U, typename Load, typename Store>
+__device__ __forceinline__ void copy64(int total, Load ld, Store st) {
+    for (int base = threadIdx.x; base < total; base += U * blockDim.x) {
+        double2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int idx = base + u * (int)blockDim.x;
+            if (idx < total) v[u] = ld(idx);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int idx = base + u * (int)blockDim.x;
+            if (idx < total) st(idx, v[u]);
+        }
+    }
+}
+
+// ---- x lines of one batch: nl lines starting at line0 (line = 3 (row - row0) + c) ----
+// Packed lines carry z[j] = s[2j] + i s[2j+1]; the forward split stores twice the spectrum
+// (the factor is in the kernel), the inverse forms 2 Z[k] from X[k] and X[half - k].
+__device__ __forceinline__ double2 *x_inverse_lines(const Conv64 &C, const double2 *__restrict__ X, int row0, int line0, int nl,
+                                                    double2 *a, double2 *b, int ls) {
+    const size_t nrows = (size_t)C.ny * C.nz;
+    if (C.half) {
+        const int half = C.half;
+        for (int idx = threadIdx.x; idx < nl * half; idx += blockDim.x) {
+            const int l = idx / half, k = idx - l * half;
+            const int rr = (line0 + l) / 3, c = line0 + l - 3 * rr;
+            const double2 *src = X + (c * nrows + row0 + rr) * C.nkx;
+            const double2 p = src[k], q = src[half - k], w = __ldg(C.xpost + k);
+            const double2 d = make_double2(p.x - q.x, p.y + q.y);  // X[k] - conj X[half-k]
+            const double ox = d.x * w.x + d.y * w.y, oy = d.y * w.x - d.x * w.y;
+            a[l * ls + k] = make_double2((p.x + q.x) - oy, (p.y - q.y) + ox);
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < nl * C.px; idx += blockDim.x) {
+            const int l = idx / C.px, k = idx - l * C.px;
+            const int rr = (line0 + l) / 3, c = line0 + l - 3 * rr;
+            const double2 *src = X + (c * nrows + row0 + rr) * C.nkx;
+            a[l * ls + k] = k < C.nkx ? src[k] : zconj(src[C.px - k]);
+        }
+    }
+    __syncthreads();
+    return fft_lines64<true>(a, b, nl, ls, C.plx, C.xprune != 0);
+}
+
+// samples H[(line0 + l) * nx + x] -> X rows
+__device__ __forceinline__ void x_forward_lines(const Conv64 &C, double2 *__restrict__ X, const double *H, int row0, int line0,
+                                                int nl, double2 *a, double2 *b, int ls) {
+    const size_t nrows = (size_t)C.ny * C.nz;
+    const int nx = C.nx, len = C.half ? C.half : C.px;
+    const int lim = C.xprune ? len / 2 : len;  // the pruned first stage reads the lower half only
+    for (int idx = threadIdx.x; idx < nl * lim; idx += blockDim.x) {
+        const int l = idx / lim, j = idx - l * lim;
+        const double *h = H + (size_t)(line0 + l) * nx;
+        double2 v = make_double2(0.0, 0.0);
+        if (C.half) {
+            if (2 * j < nx) v.x = h[2 * j];
+            if (2 * j + 1 < nx) v.y = h[2 * j + 1];
+        } else if (j < nx) {
+            v.x = h[j];
+        }
+        a[l * ls + j] = v;
+    }
+    __syncthreads();
+    const double2 *r = fft_lines64<false>(a, b, nl, ls, C.plx, C.xprune != 0);
+    for (int idx = threadIdx.x; idx < nl * C.nkx; idx += blockDim.x) {
+        const int l = idx / C.nkx, k = idx - l * C.nkx;
+        const int rr = (line0 + l) / 3, c = line0 + l - 3 * rr;
+        double2 v;
+        if (C.half) {
+            const double2 p = r[l * ls + (k == C.half ? 0 : k)], q = r[l * ls + (k == 0 ? 0 : C.half - k)];
+            const double2 w = __ldg(C.xpost + k);
+            const double2 o = make_double2(p.y + q.y, q.x - p.x);  // -i (Z[k] - conj Z[half-k])
+            v = make_double2((p.x + q.x) + (w.x * o.x - w.y * o.y), (p.y - q.y) + (w.x * o.y + w.y * o.x));
+        } else {
+            v = r[l * ls + k];
+        }
+        X[(c * nrows + row0 + rr) * C.nkx + k] = v;
+    }
+}
+
+// Rows too long for the fused row pass's shared memory: one line per CTA, full-length lines.
 __global__ void x_forward64(const Conv64 C, const double *__restrict__ m, const double *__restrict__ phi,
                             double2 *__restrict__ X) {
     extern __shared__ double2 sm64[];
     double2 *a = sm64, *b = sm64 + C.px;
-    const int row = blockIdx.x, c = blockIdx.y, nrows = C.ny * C.nz;
+    const int row = blockIdx.x, c = blockIdx.y;
+    const size_t nrows = (size_t)C.ny * C.nz;
     const long long base = (long long)row * C.nx;
     for (int x = threadIdx.x; x < C.px; x += blockDim.x) {
         double v = 0.0;
@@ -146,52 +377,24 @@ __global__ void x_forward64(const Conv64 C, const double *__restrict__ m, const 
         a[x] = make_double2(v, 0.0);
     }
     __syncthreads();
-    const double2 *r = fft_line64(a, b, C.plx, false);
-    for (int k = threadIdx.x; k < C.nkx; k += blockDim.x) X[((long long)c * nrows + row) * C.nkx + k] = r[k];
+    const double2 *r = fft_lines64<false>(a, b, 1, C.px, C.plx, false);
+    for (int k = threadIdx.x; k < C.nkx; k += blockDim.x) X[(c * nrows + row) * C.nkx + k] = r[k];
 }
-
-// X[c][row][kx] -> H_d along x (real part of the inverse of the Hermitian-completed line);
-// zero at cells outside the body (mask, or phi <= 0 with a boundary tier)
-__global__ void x_inverse64(const Conv64 C, const double2 *__restrict__ X, double *__restrict__ hd,
-                            const uint8_t *__restrict__ mask, const double *__restrict__ phi) {
+__global__ void x_inverse64(const Conv64 C, const double2 *__restrict__ X, double *__restrict__ hd) {
     extern __shared__ double2 sm64[];
+    const int row = blockIdx.x, c = blockIdx.y;
     double2 *a = sm64, *b = sm64 + C.px;
-    const int row = blockIdx.x, c = blockIdx.y, nrows = C.ny * C.nz;
-    const double2 *src = X + ((long long)c * nrows + row) * C.nkx;
+    const size_t nrows = (size_t)C.ny * C.nz;
+    const double2 *src = X + (c * nrows + row) * C.nkx;
     for (int k = threadIdx.x; k < C.px; k += blockDim.x) a[k] = k < C.nkx ? src[k] : zconj(src[C.px - k]);
     __syncthreads();
-    const double2 *r = fft_line64(a, b, C.plx, true);
-    for (int x = threadIdx.x; x < C.nx; x += blockDim.x) {
-        const long long i = (long long)row * C.nx + x;
-        const bool act = (mask == nullptr || mask[i] != 0) && (phi == nullptr || phi[i] > 0.0);
-        hd[c * C.n + i] = act ? r[x].x : 0.0;
-    }
+    const double2 *r = fft_lines64<true>(a, b, 1, C.px, C.plx, false);
+    for (int x = threadIdx.x; x < C.nx; x += blockDim.x) hd[c * C.n + (long long)row * C.nx + x] = r[x].x;
 }
 
-// (c, z, kx): y < ny zero padded to py, forward -> Y[c][z][ky][kx]
-__global__ void y_forward64(const Conv64 C, const double2 *__restrict__ X, double2 *__restrict__ Y) {
-    extern __shared__ double2 sm64[];
-    double2 *a = sm64, *b = sm64 + C.py;
-    const int kx = blockIdx.x, z = blockIdx.y, c = blockIdx.z;
-    const double2 *src = X + (((long long)c * C.nz + z) * C.ny) * C.nkx + kx;
-    for (int y = threadIdx.x; y < C.py; y += blockDim.x) a[y] = y < C.ny ? src[(long long)y * C.nkx] : make_double2(0.0, 0.0);
-    __syncthreads();
-    const double2 *r = fft_line64(a, b, C.ply, false);
-    double2 *dst = Y + (((long long)c * C.nz + z) * C.py) * C.nkx + kx;
-    for (int ky = threadIdx.x; ky < C.py; ky += blockDim.x) dst[(long long)ky * C.nkx] = r[ky];
-}
-
-// (c, z, kx): inverse over ky, rows y < ny back into X
-__global__ void y_inverse64(const Conv64 C, const double2 *__restrict__ Y, double2 *__restrict__ X) {
-    extern __shared__ double2 sm64[];
-    double2 *a = sm64, *b = sm64 + C.py;
-    const int kx = blockIdx.x, z = blockIdx.y, c = blockIdx.z;
-    const double2 *src = Y + (((long long)c * C.nz + z) * C.py) * C.nkx + kx;
-    for (int ky = threadIdx.x; ky < C.py; ky += blockDim.x) a[ky] = src[(long long)ky * C.nkx];
-    __syncthreads();
-    const double2 *r = fft_line64(a, b, C.ply, true);
-    double2 *dst = X + (((long long)c * C.nz + z) * C.ny) * C.nkx + kx;
-    for (int y = threadIdx.x; y < C.ny; y += blockDim.x) dst[(long long)y * C.nkx] = r[y];
+// sign flip on the integer pipe
+__device__ __forceinline__ double zneg_if(bool neg, double v) {
+    return __longlong_as_double(__double_as_longlong(v) ^ (neg ? 0x8000000000000000ull : 0ull));
 }
 
 __device__ __forceinline__ double2 zmadd(double2 k, double2 m, double2 acc) {
@@ -216,80 +419,131 @@ __device__ __forceinline__ void multiply3(const Conv64 &C, double2 *mx, double2 
         *mz = make_double2(-hz.x, -hz.y);
         return;
     }
-    int kym, kzm;
-    double sy, sz;
-    mirror(ky, C.py, kym, sy);
+    const bool ny_ = ky > C.py / 2;  // mirrored frequencies: odd components change sign
+    const int kym = ny_ ? C.py - ky : ky;
+    const double2 a = *mx, b = *my, d = *mz;
     if (C.thin) {
         const long long kc = (long long)C.nky * C.nkx;
         const double *K = C.kern + (long long)kym * C.nkx + kx;
-        const double kxx = K[0], kyy = K[kc], kzz = K[2 * kc], kxy = sy * K[3 * kc];
-        const double2 a = *mx, b = *my, d = *mz;
+        const double kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc), kxy = zneg_if(ny_, __ldg(K + 3 * kc));
         *mx = make_double2(-(kxx * a.x + kxy * b.x), -(kxx * a.y + kxy * b.y));
         *my = make_double2(-(kxy * a.x + kyy * b.x), -(kxy * a.y + kyy * b.y));
         *mz = make_double2(-kzz * d.x, -kzz * d.y);
         return;
     }
-    mirror(kz, C.pz, kzm, sz);
+    const bool nz_ = kz > C.pz / 2;
+    const int kzm = nz_ ? C.pz - kz : kz;
     const long long kc = (long long)C.nkz * C.nky * C.nkx;
     const double *K = C.kern + ((long long)kzm * C.nky + kym) * C.nkx + kx;
-    const double kxx = K[0], kyy = K[kc], kzz = K[2 * kc];
-    const double kxy = sy * K[3 * kc], kxz = sz * K[4 * kc], kyz = sy * sz * K[5 * kc];
-    const double2 a = *mx, b = *my, d = *mz;
+    const double kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc);
+    const double kxy = zneg_if(ny_, __ldg(K + 3 * kc)), kxz = zneg_if(nz_, __ldg(K + 4 * kc)),
+                 kyz = zneg_if(ny_ != nz_, __ldg(K + 5 * kc));
     *mx = make_double2(-(kxx * a.x + kxy * b.x + kxz * d.x), -(kxx * a.y + kxy * b.y + kxz * d.y));
     *my = make_double2(-(kxy * a.x + kyy * b.x + kyz * d.x), -(kxy * a.y + kyy * b.y + kyz * d.y));
     *mz = make_double2(-(kxz * a.x + kyz * b.x + kzz * d.x), -(kxz * a.y + kyz * b.y + kzz * d.y));
 }
 
-// 3-D: (kx, ky): forward z of the three components, multiply, inverse, planes z < nz
-__global__ void z_convolve64(const Conv64 C, double2 *__restrict__ Y) {
-    extern __shared__ double2 sm64[];
-    const int kx = blockIdx.x, ky = blockIdx.y, L = C.pz;
-    double2 *a[3], *b[3];
-    for (int c = 0; c < 3; ++c) {
-        a[c] = sm64 + 2 * c * L;
-        b[c] = a[c] + L;
+// ---- column passes: a tile of tx kx columns per CTA ----
+struct Col64 {
+    Conv64 C;
+    const double2 *in;
+    double2 *out;
+    int tx;
+    int early;
+};
+
+// lines (c, col) at (c * ncol + col) * ls: elements e < cnt from src + c cs + e es + col,
+// zeros up to lim
+__device__ __forceinline__ void load_lines64(const double2 *__restrict__ src, size_t cs, size_t es, int nc, int cnt, int lim,
+                                             int ncol, double2 *a, int ls) {
+    copy64<4>(
+        nc * cnt * ncol,
+        [&](int idx) {
+            const int r = idx / ncol, col = idx - r * ncol, c = r / cnt, e = r - c * cnt;
+            return src[c * cs + e * es + col];
+        },
+        [&](int idx, double2 v) {
+            const int r = idx / ncol, col = idx - r * ncol, c = r / cnt, e = r - c * cnt;
+            a[(c * ncol + col) * ls + e] = v;
+        });
+    const int pad = lim - cnt;
+    for (int idx = threadIdx.x; idx < nc * ncol * pad; idx += blockDim.x) {
+        const int l = idx / pad;
+        a[l * ls + cnt + (idx - l * pad)] = make_double2(0.0, 0.0);
     }
-    const long long zs = (long long)C.py * C.nkx, cs = (long long)C.nz * zs;
-    for (int c = 0; c < 3; ++c)
-        for (int z = threadIdx.x; z < L; z += blockDim.x)
-            a[c][z] = z < C.nz ? Y[c * cs + z * zs + (long long)ky * C.nkx + kx] : make_double2(0.0, 0.0);
-    __syncthreads();
-    double2 *r[3];
-    for (int c = 0; c < 3; ++c) r[c] = fft_line64(a[c], b[c], C.plz, false);
-    for (int kz = threadIdx.x; kz < L; kz += blockDim.x) multiply3(C, r[0] + kz, r[1] + kz, r[2] + kz, kx, ky, kz);
-    __syncthreads();
-    double2 *q[3];
-    for (int c = 0; c < 3; ++c) q[c] = fft_line64(r[c], r[c] == a[c] ? b[c] : a[c], C.plz, true);
-    for (int c = 0; c < 3; ++c)
-        for (int z = threadIdx.x; z < C.nz; z += blockDim.x) Y[c * cs + z * zs + (long long)ky * C.nkx + kx] = q[c][z];
+}
+__device__ __forceinline__ void store_lines64(double2 *__restrict__ dst, size_t cs, size_t es, int nc, int cnt, int ncol,
+                                              const double2 *a, int ls) {
+    for (int idx = threadIdx.x; idx < nc * cnt * ncol; idx += blockDim.x) {
+        const int r = idx / ncol, col = idx - r * ncol, c = r / cnt, e = r - c * cnt;
+        dst[c * cs + e * es + col] = a[(c * ncol + col) * ls + e];
+    }
 }
 
-// thin film: (kx): forward y of the three components, 2-D multiply, inverse, rows y < ny
-__global__ void y_convolve64(const Conv64 C, double2 *__restrict__ X) {
+constexpr int kTC = 128;  // threads of a column pass
+__host__ __device__ inline int y_ls64(const Conv64 &C, int tx) { return C.py + (tx > 1 ? 1 : 0); }  // one line fills the limit
+
+// X[c][z][y < ny][kx] -> Y[c][z][ky][kx]
+__global__ void __launch_bounds__(kTC) y_forward64(const Col64 P) {
+    pdl_wait();
+    if (P.early) pdl_trigger();
     extern __shared__ double2 sm64[];
-    const int kx = blockIdx.x, L = C.py;
-    double2 *a[3], *b[3];
-    for (int c = 0; c < 3; ++c) {
-        a[c] = sm64 + 2 * c * L;
-        b[c] = a[c] + L;
-    }
-    const long long cs = (long long)C.ny * C.nkx;
-    for (int c = 0; c < 3; ++c)
-        for (int y = threadIdx.x; y < L; y += blockDim.x)
-            a[c][y] = y < C.ny ? X[c * cs + (long long)y * C.nkx + kx] : make_double2(0.0, 0.0);
+    const Conv64 &C = P.C;
+    const int kx0 = blockIdx.x * P.tx, ncol = min(P.tx, C.nkx - kx0), ls = y_ls64(C, P.tx);
+    const size_t cz = (size_t)blockIdx.z * C.nz + blockIdx.y;
+    double2 *a = sm64, *b = a + P.tx * ls;
+    load_lines64(P.in + cz * C.ny * C.nkx + kx0, 0, C.nkx, 1, C.ny, C.yprune ? C.py / 2 : C.py, ncol, a, ls);
     __syncthreads();
-    double2 *r[3];
-    for (int c = 0; c < 3; ++c) r[c] = fft_line64(a[c], b[c], C.ply, false);
-    for (int ky = threadIdx.x; ky < L; ky += blockDim.x) multiply3(C, r[0] + ky, r[1] + ky, r[2] + ky, kx, ky, 0);
-    __syncthreads();
-    double2 *q[3];
-    for (int c = 0; c < 3; ++c) q[c] = fft_line64(r[c], r[c] == a[c] ? b[c] : a[c], C.ply, true);
-    for (int c = 0; c < 3; ++c)
-        for (int y = threadIdx.x; y < C.ny; y += blockDim.x) X[c * cs + (long long)y * C.nkx + kx] = q[c][y];
+    const double2 *r = fft_lines64<false>(a, b, ncol, ls, C.ply, C.yprune != 0);
+    store_lines64(P.out + cz * C.py * C.nkx + kx0, 0, C.nkx, 1, C.py, ncol, r, ls);
 }
 
-// H_corr(t) = -sum_s dN(t, s) (phi_s Ms m_s), added to H_d at the target cells
-// (demag_boundary_fp64.cu:23-76); the tensor row of (t, s) is xx xy xz yy yz zz.
+// Y[c][z][ky][kx] -> X[c][z][y < ny][kx]
+__global__ void __launch_bounds__(kTC) y_inverse64(const Col64 P) {
+    pdl_wait();
+    if (P.early) pdl_trigger();
+    extern __shared__ double2 sm64[];
+    const Conv64 &C = P.C;
+    const int kx0 = blockIdx.x * P.tx, ncol = min(P.tx, C.nkx - kx0), ls = y_ls64(C, P.tx);
+    const size_t cz = (size_t)blockIdx.z * C.nz + blockIdx.y;
+    double2 *a = sm64, *b = a + P.tx * ls;
+    load_lines64(P.in + cz * C.py * C.nkx + kx0, 0, C.nkx, 1, C.py, C.py, ncol, a, ls);
+    __syncthreads();
+    const double2 *r = fft_lines64<true>(a, b, ncol, ls, C.ply, C.yprune != 0);
+    store_lines64(P.out + cz * C.ny * C.nkx + kx0, 0, C.nkx, 1, C.ny, ncol, r, ls);
+}
+
+// thin film (tile): forward y of the three components, multiply, inverse, rows y < ny;
+// 3-D (tile, ky): the same along z.  In place.
+template <bool THIN>
+__global__ void __launch_bounds__(kTC) convolve64(const Col64 P) {
+    pdl_wait();
+    if (P.early) pdl_trigger();
+    extern __shared__ double2 sm64[];
+    const Conv64 &C = P.C;
+    const int L = THIN ? C.py : C.pz, cnt = THIN ? C.ny : C.nz, ls = L + 1;
+    const bool prune = (THIN ? C.yprune : C.zprune) != 0;
+    const Plan64 &pl = THIN ? C.ply : C.plz;
+    const int kx0 = blockIdx.x * P.tx, ncol = min(P.tx, C.nkx - kx0), ky = THIN ? 0 : blockIdx.y;
+    const size_t es = THIN ? (size_t)C.nkx : (size_t)C.py * C.nkx, cs = cnt * es;
+    const size_t base = (size_t)ky * C.nkx + kx0;
+    double2 *a = sm64, *b = a + 3 * P.tx * ls;
+    load_lines64(P.in + base, cs, es, 3, cnt, prune ? L / 2 : L, ncol, a, ls);
+    __syncthreads();
+    double2 *r = fft_lines64<false>(a, b, 3 * ncol, ls, pl, prune);
+    for (int idx = threadIdx.x; idx < L * ncol; idx += blockDim.x) {
+        const int k = idx / ncol, col = idx - k * ncol;
+        double2 *q = r + col * ls + k;
+        multiply3(C, q, q + ncol * ls, q + 2 * ncol * ls, kx0 + col, THIN ? k : ky, THIN ? 0 : k);
+    }
+    __syncthreads();
+    const double2 *o = fft_lines64<true>(r, r == a ? b : a, 3 * ncol, ls, pl, prune);
+    store_lines64(P.out + base, cs, es, 3, cnt, ncol, o, ls);
+}
+
+// H_corr(t) = -sum_s dN(t, s) (phi_s Ms m_s) at the target cells, which the row pass adds to
+// H_d (demag_boundary_fp64.cu:23-76); the tensor row of (t, s) is xx xy xz yy yz zz.  hd is
+// zero before the launch.
 __global__ void demag_correction64(double *__restrict__ hd, const double *__restrict__ m, const double *__restrict__ phi,
                                    const int32_t *__restrict__ tidx, const int32_t *__restrict__ sidx,
                                    const double *__restrict__ tensor, double ms, long long n, uint32_t ntarget,
@@ -317,8 +571,10 @@ __global__ void demag_correction64(double *__restrict__ hd, const double *__rest
 struct Field64 {
     int nx, ny, nz;
     long long n;
-    const double *m, *hd;     // hd NULL: no demag
-    double *hex, *heff, *k;   // k NULL: not stored
+    const double *m;          // stage input; NULL: no right-hand side in this pass
+    const double *hcorr;      // sparse demag correction at m (zero elsewhere) or NULL
+    double *hex, *hd, *heff;  // observables; NULL: not written
+    double *k;                // NULL: not stored
     const uint8_t *mask;
     const uint8_t *region;    // ids (< 256) or NULL
     const double *lut;        // 256 x 256 stiffness table (J/m)
@@ -329,27 +585,29 @@ struct Field64 {
     double phi_floor, delta_min;
     int exchange;
     int per;                  // periodic axes (bit 0 x, 1 y, 2 z): neighbours wrap around
-    double a_ex, ms, dx, dy, dz;
+    double a_ex, dx, dy, dz;
+    double inv2[3];           // 1 / d^2
+    double ex_s;              // 2 / (mu0 Ms)
     int has_ext;
     double hext[3];
     int has_uni;
     double ku1, ku2, u[3];
+    double ku1c, ku2c;        // 2 Ku1 / (mu0 Ms), 4 Ku2 / (mu0 Ms)
     int has_cub;
     double kc1, kc2, kc3, c1[3], c2[3], c3[3];
+    double kc1c, kc2c, kc3c;  // -2 Kc1 / (mu0 Ms), -2 Kc2 / (mu0 Ms), -4 Kc3 / (mu0 Ms)
     double gbar, alpha, prec;
     double *partials;         // [block][kStats] or NULL
 };
 
 // exchange field at cell i (x, y, z); the neighbour offsets are +x -x +y -y +z -z
-__device__ void exchange64(const Field64 &P, long long i, int x, int y, int z, double e[3]) {
+__device__ __forceinline__ void exchange64(const Field64 &P, long long i, int x, int y, int z, double e[3]) {
     e[0] = e[1] = e[2] = 0.0;
     if (!P.exchange) return;
     const double *m = P.m;
     const long long n = P.n, nxy = (long long)P.nx * P.ny;
     const bool has[6] = {x + 1 < P.nx, x > 0, y + 1 < P.ny, y > 0, z + 1 < P.nz, z > 0};
     const long long off[6] = {1, -1, P.nx, -(long long)P.nx, nxy, -nxy};
-    const double inv2[6] = {1.0 / (P.dx * P.dx), 1.0 / (P.dx * P.dx), 1.0 / (P.dy * P.dy),
-                            1.0 / (P.dy * P.dy), 1.0 / (P.dz * P.dz), 1.0 / (P.dz * P.dz)};
     const double c0[3] = {m[i], m[n + i], m[2 * n + i]};
     const int ri = P.region ? P.region[i] : 0;
     if (P.tier == 0) {
@@ -360,7 +618,7 @@ __device__ void exchange64(const Field64 &P, long long i, int x, int y, int z, d
             long long j = has[q] ? i + off[q] : ((P.per >> (q >> 1)) & 1) ? i - off[q] * (ext[q >> 1] - 1) : i;
             if (P.mask && P.mask[j] == 0) j = i;
             if (j == i) continue;
-            const double w = (P.region ? P.lut[ri * FULLMAG_FDM_MAX_EXCHANGE_REGIONS + P.region[j]] : P.a_ex) * inv2[q];
+            const double w = (P.region ? P.lut[ri * FULLMAG_FDM_MAX_EXCHANGE_REGIONS + P.region[j]] : P.a_ex) * P.inv2[q >> 1];
             for (int c = 0; c < 3; ++c) e[c] += w * (m[c * n + j] - c0[c]);
         }
     } else if (P.tier == 1) {
@@ -370,7 +628,7 @@ __device__ void exchange64(const Field64 &P, long long i, int x, int y, int z, d
             const double f = P.face[q][i];
             if (!(f > 0.0) || !has[q]) continue;
             const long long j = i + off[q];
-            const double w = (P.region ? P.lut[ri * FULLMAG_FDM_MAX_EXCHANGE_REGIONS + P.region[j]] : P.a_ex) * f * inv2[q];
+            const double w = (P.region ? P.lut[ri * FULLMAG_FDM_MAX_EXCHANGE_REGIONS + P.region[j]] : P.a_ex) * f * P.inv2[q >> 1];
             for (int c = 0; c < 3; ++c) e[c] += w * (m[c * n + j] - c0[c]);
         }
     } else {
@@ -390,20 +648,19 @@ __device__ void exchange64(const Field64 &P, long long i, int x, int y, int z, d
             for (int c = 0; c < 3; ++c) e[c] += w * (mj[c] - c0[c]);
         }
     }
-    double s = 2.0 / (kMu0d * P.ms);
+    double s = P.ex_s;
     if (P.tier > 0) s /= fmax(P.phi[i], P.phi_floor);
     for (int c = 0; c < 3; ++c) e[c] *= s;
 }
 
 // exchange energy pairs of cell i with its forward neighbours (reductions_fp64.cu:123-210)
-__device__ double exchange_pairs64(const Field64 &P, long long i, int x, int y, int z, double phi_i) {
+__device__ __forceinline__ double exchange_pairs64(const Field64 &P, long long i, int x, int y, int z, double phi_i) {
     if (!P.exchange) return 0.0;
     const double *m = P.m;
     const long long n = P.n, nxy = (long long)P.nx * P.ny;
     const bool has[3] = {x + 1 < P.nx, y + 1 < P.ny, z + 1 < P.nz};
     const long long off[3] = {1, P.nx, nxy};
     const int ext[3] = {P.nx, P.ny, P.nz};
-    const double inv2[3] = {1.0 / (P.dx * P.dx), 1.0 / (P.dy * P.dy), 1.0 / (P.dz * P.dz)};
     const int ri = P.region ? P.region[i] : 0;
     double e = 0.0;
     for (int a = 0; a < 3; ++a) {
@@ -420,7 +677,7 @@ __device__ double exchange_pairs64(const Field64 &P, long long i, int x, int y, 
             const double dm = m[c * n + j] - m[c * n + i];
             s2 += dm * dm;
         }
-        e += A * phi_i * s2 * inv2[a];
+        e += A * phi_i * s2 * P.inv2[a];
     }
     return e;
 }
@@ -444,130 +701,181 @@ __device__ __forceinline__ void block_stats(double (&v)[kStats], double *out) {
     }
 }
 
-// H_eff, the right-hand side and (optionally) the statistics of one evaluation
-__global__ void __launch_bounds__(kT) field64(const Field64 P) {
+// One fused pass over `rows` x-rows per CTA: inverse x-transform of the demag field at the
+// stage input, exchange, local terms, torque, statistics, the adaptive error norm, the next
+// stage input N(m0 + dt sum_j c_j k_j) and its forward x-transform.  The step is then a
+// chain of two launches per evaluation on films and four on volumes; FP64 issue bounds it.
+// 200x100x1 Heun: 511 us per step as one kernel per operation with strided radix-4 columns.
+struct Row64 {
+    Field64 f;
+    Conv64 C;
+    const double2 *x_in;  // NULL: no demag field from a spectrum in this pass
+    double2 *x_out;       // NULL: no forward transform
+    const double *hd_in;  // H_d from memory (rows too long for the fused transform) or NULL
+    int rows;             // rows per CTA
+    int lb;               // x lines transformed at a time: 3 rows or 1
+    const double *m0;     // NULL: no combination
+    int nk;
+    const double *kk[8];  // NULL entry: the derivative of this pass
+    double c[8];
+    double dt;
+    double *m_next;
+    const double *m_fwd;  // forward-transform source without a combination
+    int ne;               // error terms (0: none); NULL entry: the derivative of this pass
+    const double *ek[8];
+    double ec[8];
+    int early;
+};
+
+__host__ __device__ inline int row_ls64(const Conv64 &C) { return (C.half ? C.half : C.px) + 1; }
+
+__global__ void __launch_bounds__(kT, 2) row64(const Row64 R) {
+    pdl_wait();
+    if (R.early) pdl_trigger();
+    extern __shared__ double2 sm64[];
+    const Field64 &P = R.f;
+    const int nx = P.nx, nrows = P.ny * P.nz, row0 = blockIdx.x * R.rows, rows = min(R.rows, nrows - row0);
+    const bool fft = R.x_in || R.x_out;
+    const int ls = fft ? row_ls64(R.C) : 0, lb = min(R.lb, rows * 3);
+    double2 *a = sm64, *b = a + R.lb * ls;
+    double *H = reinterpret_cast<double *>(b + R.lb * ls);  // line (row, c): H_d in, next input out
+    if (R.x_in) {
+        for (int l0 = 0; l0 < rows * 3; l0 += lb) {
+            const int nl = min(lb, rows * 3 - l0);
+            const double2 *r = x_inverse_lines(R.C, R.x_in, row0, l0, nl, a, b, ls);
+            for (int idx = threadIdx.x; idx < nl * nx; idx += blockDim.x) {
+                const int l = idx / nx, x = idx - l * nx;
+                const double2 *q = r + l * ls;
+                H[(size_t)l0 * nx + idx] = R.C.half ? ((x & 1) ? q[x >> 1].y : q[x >> 1].x) : q[x].x;
+            }
+            __syncthreads();
+        }
+    }
     double st[kStats] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     const long long n = P.n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % P.nx), y = (int)((i / P.nx) % P.ny), z = (int)(i / ((long long)P.nx * P.ny));
+    for (int idx = threadIdx.x; idx < rows * nx; idx += blockDim.x) {
+        const int rr = idx / nx, x = idx - rr * nx, row = row0 + rr, z = row / P.ny, y = row - z * P.ny;
+        const long long i = (long long)row * nx + x;
         const double phi_i = P.phi ? P.phi[i] : 1.0;
-        const bool act = (P.mask == nullptr || P.mask[i] != 0) && (P.tier == 0 || phi_i > 0.0);
-        double h[3] = {0, 0, 0}, ex[3] = {0, 0, 0}, hd[3] = {0, 0, 0}, k[3] = {0, 0, 0};
-        if (act) {
-            const double m0[3] = {P.m[i], P.m[n + i], P.m[2 * n + i]};
-            exchange64(P, i, x, y, z, ex);
-            if (P.hd)
-                for (int c = 0; c < 3; ++c) hd[c] = P.hd[c * n + i];
-            for (int c = 0; c < 3; ++c) h[c] = ex[c] + hd[c] + (P.has_ext ? P.hext[c] : 0.0);
-            double e_uni = 0.0, e_cub = 0.0;
-            const double inv_mu0ms = 1.0 / (kMu0d * P.ms);
-            if (P.has_uni) {
-                const double mu = m0[0] * P.u[0] + m0[1] * P.u[1] + m0[2] * P.u[2];
-                const double cf = 2.0 * inv_mu0ms * (P.ku1 * mu + 2.0 * P.ku2 * mu * mu * mu);
-                for (int c = 0; c < 3; ++c) h[c] += cf * P.u[c];
-                e_uni = P.ku1 * mu * mu + P.ku2 * mu * mu * mu * mu;
+        double *hl = H + (size_t)rr * 3 * nx + x;
+        double k[3] = {0, 0, 0};
+        if (P.m) {
+            const bool act = (P.mask == nullptr || P.mask[i] != 0) && (P.tier == 0 || phi_i > 0.0);
+            double h[3] = {0, 0, 0}, ex[3] = {0, 0, 0}, hd[3] = {0, 0, 0};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (act) hd[c] = R.x_in ? hl[c * nx] : R.hd_in ? R.hd_in[c * n + i] : 0.0;
+                if (P.hcorr) hd[c] += P.hcorr[c * n + i];
+                if (P.hd) P.hd[c * n + i] = hd[c];
             }
-            if (P.has_cub) {
-                const double a1 = m0[0] * P.c1[0] + m0[1] * P.c1[1] + m0[2] * P.c1[2];
-                const double a2 = m0[0] * P.c2[0] + m0[1] * P.c2[1] + m0[2] * P.c2[2];
-                const double a3 = m0[0] * P.c3[0] + m0[1] * P.c3[1] + m0[2] * P.c3[2];
-                const double s1 = a1 * a1, s2 = a2 * a2, s3 = a3 * a3;
-                const double sig = s1 * s2 + s2 * s3 + s1 * s3;
-                const double k1c = -2.0 * P.kc1 * inv_mu0ms, k2c = -2.0 * P.kc2 * inv_mu0ms, k3c = -4.0 * P.kc3 * inv_mu0ms;
-                const double g1 = k1c * a1 * (s2 + s3) + k2c * a1 * s2 * s3 + k3c * sig * a1 * (s2 + s3);
-                const double g2 = k1c * a2 * (s1 + s3) + k2c * a2 * s1 * s3 + k3c * sig * a2 * (s1 + s3);
-                const double g3 = k1c * a3 * (s1 + s2) + k2c * a3 * s1 * s2 + k3c * sig * a3 * (s1 + s2);
-                for (int c = 0; c < 3; ++c) h[c] += g1 * P.c1[c] + g2 * P.c2[c] + g3 * P.c3[c];
-                e_cub = P.kc1 * sig + P.kc2 * s1 * s2 * s3 + P.kc3 * sig * sig;
+            if (act) {
+                const double m0[3] = {P.m[i], P.m[n + i], P.m[2 * n + i]};
+                exchange64(P, i, x, y, z, ex);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) h[c] = ex[c] + hd[c] + (P.has_ext ? P.hext[c] : 0.0);
+                double e_uni = 0.0, e_cub = 0.0;
+                if (P.has_uni) {
+                    const double mu = m0[0] * P.u[0] + m0[1] * P.u[1] + m0[2] * P.u[2], mu2 = mu * mu;
+                    const double cf = mu * (P.ku1c + P.ku2c * mu2);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) h[c] += cf * P.u[c];
+                    e_uni = mu2 * (P.ku1 + P.ku2 * mu2);
+                }
+                if (P.has_cub) {
+                    const double a1 = m0[0] * P.c1[0] + m0[1] * P.c1[1] + m0[2] * P.c1[2];
+                    const double a2 = m0[0] * P.c2[0] + m0[1] * P.c2[1] + m0[2] * P.c2[2];
+                    const double a3 = m0[0] * P.c3[0] + m0[1] * P.c3[1] + m0[2] * P.c3[2];
+                    const double s1 = a1 * a1, s2 = a2 * a2, s3 = a3 * a3;
+                    const double sig = s1 * s2 + s2 * s3 + s1 * s3;
+                    const double w = P.kc1c + P.kc3c * sig;
+                    const double g1 = a1 * (w * (s2 + s3) + P.kc2c * s2 * s3);
+                    const double g2 = a2 * (w * (s1 + s3) + P.kc2c * s1 * s3);
+                    const double g3 = a3 * (w * (s1 + s2) + P.kc2c * s1 * s2);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) h[c] += g1 * P.c1[c] + g2 * P.c2[c] + g3 * P.c3[c];
+                    e_cub = P.kc1 * sig + P.kc2 * s1 * s2 * s3 + P.kc3 * sig * sig;
+                }
+                const double p0 = m0[1] * h[2] - m0[2] * h[1], p1 = m0[2] * h[0] - m0[0] * h[2], p2 = m0[0] * h[1] - m0[1] * h[0];
+                const double q0 = m0[1] * p2 - m0[2] * p1, q1 = m0[2] * p0 - m0[0] * p2, q2 = m0[0] * p1 - m0[1] * p0;
+                k[0] = -P.gbar * (P.prec * p0 + P.alpha * q0);
+                k[1] = -P.gbar * (P.prec * p1 + P.alpha * q1);
+                k[2] = -P.gbar * (P.prec * p2 + P.alpha * q2);
+                if (P.partials) {
+                    st[0] += exchange_pairs64(P, i, x, y, z, phi_i);
+                    st[1] += phi_i * (m0[0] * hd[0] + m0[1] * hd[1] + m0[2] * hd[2]);
+                    if (P.has_ext) st[2] += phi_i * (m0[0] * P.hext[0] + m0[1] * P.hext[1] + m0[2] * P.hext[2]);
+                    st[3] += phi_i * e_uni;
+                    st[4] += phi_i * e_cub;
+                    st[5] = fmax(st[5], h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
+                    st[6] = fmax(st[6], hd[0] * hd[0] + hd[1] * hd[1] + hd[2] * hd[2]);
+                    st[7] = fmax(st[7], k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
+                }
             }
-            const double p0 = m0[1] * h[2] - m0[2] * h[1], p1 = m0[2] * h[0] - m0[0] * h[2], p2 = m0[0] * h[1] - m0[1] * h[0];
-            const double q0 = m0[1] * p2 - m0[2] * p1, q1 = m0[2] * p0 - m0[0] * p2, q2 = m0[0] * p1 - m0[1] * p0;
-            k[0] = -P.gbar * (P.prec * p0 + P.alpha * q0);
-            k[1] = -P.gbar * (P.prec * p1 + P.alpha * q1);
-            k[2] = -P.gbar * (P.prec * p2 + P.alpha * q2);
-            if (P.partials) {
-                st[0] += exchange_pairs64(P, i, x, y, z, phi_i);
-                st[1] += phi_i * (m0[0] * hd[0] + m0[1] * hd[1] + m0[2] * hd[2]);
-                if (P.has_ext) st[2] += phi_i * (m0[0] * P.hext[0] + m0[1] * P.hext[1] + m0[2] * P.hext[2]);
-                st[3] += phi_i * e_uni;
-                st[4] += phi_i * e_cub;
-                st[5] = fmax(st[5], h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
-                st[6] = fmax(st[6], hd[0] * hd[0] + hd[1] * hd[1] + hd[2] * hd[2]);
-                st[7] = fmax(st[7], k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
+            if (R.ne > 0) {
+                double e2 = 0.0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    double s = 0.0;
+                    for (int t = 0; t < R.ne; ++t) s += R.ec[t] * (R.ek[t] ? R.ek[t][c * n + i] : k[c]);
+                    s *= R.dt;
+                    e2 += s * s;
+                }
+                st[8] = fmax(st[8], e2);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (P.hex) P.hex[c * n + i] = ex[c];
+                if (P.heff) P.heff[c * n + i] = h[c];
+                if (P.k) P.k[c * n + i] = k[c];
             }
         }
-        for (int c = 0; c < 3; ++c) {
-            P.hex[c * n + i] = ex[c];
-            P.heff[c * n + i] = h[c];
-            if (P.k) P.k[c * n + i] = k[c];
+        double v[3] = {0, 0, 0};
+        if (R.m0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double s = 0.0;
+                for (int t = 0; t < R.nk; ++t) s += R.c[t] * (R.kk[t] ? R.kk[t][c * n + i] : k[c]);
+                v[c] = R.m0[c * n + i] + R.dt * s;
+            }
+            const double nn = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+            const double inv = nn > 0.0 ? 1.0 / sqrt(nn) : 0.0;  // a zero vector stays zero
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                v[c] *= inv;
+                R.m_next[c * n + i] = v[c];
+            }
+        } else if (R.m_fwd) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = R.m_fwd[c * n + i];
+        }
+        if (R.x_out) {  // the convolution's input is phi m with a boundary tier
+#pragma unroll
+            for (int c = 0; c < 3; ++c) hl[c * nx] = P.phi ? v[c] * phi_i : v[c];
         }
     }
     if (P.partials) block_stats(st, P.partials);
-}
-
-// out = N(m0 + dt sum_j c_j k_j) (a zero vector stays zero)
-struct Comb64 {
-    long long n;
-    const double *m0;
-    int nk;
-    const double *k[8];
-    double c[8];
-    double dt;
-    double *out;
-};
-__global__ void combine64(const Comb64 C) {
-    const long long n = C.n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double v[3];
-        for (int c = 0; c < 3; ++c) {
-            double s = 0.0;
-            for (int t = 0; t < C.nk; ++t) s += C.c[t] * C.k[t][c * n + i];
-            v[c] = C.m0[c * n + i] + C.dt * s;
-        }
-        const double nn = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-        const double inv = nn > 0.0 ? 1.0 / nn : 0.0;
-        for (int c = 0; c < 3; ++c) C.out[c * n + i] = v[c] * inv;
-    }
-}
-
-// max over cells of |dt sum_j e_j k_j|^2 into partials[block * kStats + 8]
-__global__ void __launch_bounds__(kT) error64(const Comb64 C, double *partials) {
-    double st[kStats] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const long long n = C.n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double e2 = 0.0;
-        for (int c = 0; c < 3; ++c) {
-            double s = 0.0;
-            for (int t = 0; t < C.nk; ++t) s += C.c[t] * C.k[t][c * n + i];
-            s *= C.dt;
-            e2 += s * s;
-        }
-        st[8] = fmax(st[8], e2);
-    }
-    block_stats(st, partials);
-}
-
-// sums / maxima of the block partials in a fixed order (one CTA)
-__global__ void finalize64(const double *partials, int nblocks, double *out, int with_err) {
-    __shared__ double sh[kT][kStats];
-    for (int s = 0; s < kStats; ++s) {
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-            const double v = partials[b * kStats + s];
-            acc = s < 5 ? acc + v : fmax(acc, v);
-        }
-        sh[threadIdx.x][s] = acc;
-    }
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o)
-            for (int s = 0; s < kStats; ++s)
-                sh[threadIdx.x][s] = s < 5 ? sh[threadIdx.x][s] + sh[threadIdx.x + o][s] : fmax(sh[threadIdx.x][s], sh[threadIdx.x + o][s]);
+    if (R.x_out) {
         __syncthreads();
+        for (int l0 = 0; l0 < rows * 3; l0 += lb) {
+            x_forward_lines(R.C, R.x_out, H, row0, l0, min(lb, rows * 3 - l0), a, b, ls);
+            __syncthreads();
+        }
     }
-    if (threadIdx.x == 0)
-        for (int s = 0; s < kStats; ++s)
-            if (s < 8 || with_err) out[s] = sh[0][s];
+}
+
+// sums / maxima of the block partials in a fixed order (one CTA of kT threads)
+__global__ void __launch_bounds__(kT) finalize64(const double *__restrict__ partials, int nblocks, double *__restrict__ out,
+                                                 int early) {
+    pdl_wait();
+    if (early) pdl_trigger();
+    double v[kStats] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+#pragma unroll
+        for (int s = 0; s < kStats; ++s) {
+            const double w = partials[(size_t)b * kStats + s];
+            v[s] = s < 5 ? v[s] + w : fmax(v[s], w);
+        }
+    block_stats(v, out);
 }
 
 __global__ void aos_to_soa64(const double *__restrict__ in, double *__restrict__ out, const uint8_t *__restrict__ mask,
@@ -583,14 +891,15 @@ __global__ void soa_to_aos64(const double *__restrict__ in, double *__restrict__
         for (int c = 0; c < 3; ++c) out[3 * i + c] = in[c * n + i];
 }
 
-unsigned blocks_for(long long n) { return (unsigned)std::min<long long>((n + kT - 1) / kT, kRedBlocks); }
+unsigned blocks_for(long long n) { return (unsigned)std::min<long long>((n + kT - 1) / kT, kMaxBlocks); }
 
-// radices 4, 2, 3, 5, 7, then any remaining prime
+// radices 8 (4 or 2 for the remainder) first, then odd primes: the even radix in front
+// carries the half-line stages
 bool make_plan64(int n, std::vector<double2> &tw, std::vector<size_t> &off, Plan64 &p) {
     p.n = n;
     p.ns = 0;
     int r = n;
-    for (int f : {4, 2, 3, 5, 7}) {
+    for (int f : {8, 4, 2, 3, 5, 7}) {
         while (r % f == 0) {
             if (p.ns >= kMaxRadixStages) return false;
             p.radix[p.ns++] = f;
@@ -613,6 +922,40 @@ bool make_plan64(int n, std::vector<double2> &tw, std::vector<size_t> &off, Plan
     return true;
 }
 
+// FP64 instructions per point of a transform of length n (twiddles included); 0 when n has
+// a prime factor above 13, for which there is no butterfly
+double fft_cost64(int n) {
+    const struct {
+        int r;
+        double c;
+    } cost[] = {{8, 10.5}, {4, 7.0}, {2, 4.0}, {3, 8.0}, {5, 12.0}, {7, 15.0}, {11, 19.0}, {13, 21.0}};
+    double s = 0.0;
+    for (const auto &f : cost)
+        while (n % f.r == 0) {
+            n /= f.r;
+            s += f.c;
+        }
+    return n == 1 ? std::max(s, 1.0) : 0.0;
+}
+
+// Padded extent of an open axis of n cells when the engine builds the tensor: 2n, the
+// reference's, when its factors are all 2..13; else the even extent above it whose
+// transform issues the fewest instructions (a prime factor R > 13 costs 4R of them per
+// point, so 2 x 157 takes 30 times the instructions of 320)
+int pad_extent64(int n) {
+    if (fft_cost64(2 * n) > 0.0) return 2 * n;
+    int best = 2 * n;
+    double bc = 1e30;
+    for (int p = 2 * n + 2; p <= 2 * n + 2 + n / 2; p += 2) {
+        const double c = fft_cost64(p) * p;
+        if (c > 0.0 && c < bc) {
+            bc = c;
+            best = p;
+        }
+    }
+    return best;
+}
+
 // One FP64 line of length p per CTA along an axis of layout [outer][p][inner] (real
 // input in_re with zero imaginary part, or complex c_in), forward transform
 // e^{-2 pi i k a / p}, the first nout outputs written to out[outer][nout][inner].
@@ -626,7 +969,7 @@ __global__ void fft_axis64_kernel(const double *__restrict__ in_re, const double
     for (int i = threadIdx.x; i < p; i += blockDim.x)
         a[i] = in_re ? make_double2(in_re[base + (long long)i * inner], 0.0) : c_in[base + (long long)i * inner];
     __syncthreads();
-    const double2 *r = fft_line64(a, b, plan, false);
+    const double2 *r = fft_lines64<false>(a, b, 1, p, plan, false);
     for (int k = threadIdx.x; k < nout; k += blockDim.x) out[(o * nout + k) * inner + q] = r[k];
 }
 
@@ -680,6 +1023,7 @@ struct Fp64Engine {
     std::vector<void *> allocs;
     double *S[2] = {nullptr, nullptr}, *K[7] = {}, *A[2] = {nullptr, nullptr};
     double *hex = nullptr, *hd = nullptr, *heff = nullptr, *staging = nullptr;
+    double *hcorr = nullptr;         // sparse demag correction (n targets among 3 n values)
     double *partials = nullptr, *dstats = nullptr, *hstats = nullptr;
     uint8_t *mask = nullptr, *region = nullptr;
     double *lut = nullptr, *phi = nullptr, *face[6] = {}, *delta[6] = {};
@@ -690,6 +1034,11 @@ struct Fp64Engine {
     double *kern = nullptr;
     double2 *kernc = nullptr;  // periodic grids: the complex image-sum kernel
     double2 *twid = nullptr;
+    // launch shapes (choose_shapes)
+    int rows = 1, lb = 3;            // rows per CTA of the row pass, x lines transformed at a time
+    bool fused_x = true;             // the row pass holds the x-transforms
+    int tx_y = 1, tx_c = 1;          // kx columns per CTA of the y passes and of the convolution pass
+    bool early = false;              // programmatic early launch on small grids (engine.h)
     // state
     int cur = 0;
     double time = 0.0;
@@ -733,26 +1082,153 @@ struct Fp64Engine {
     bool setup(const fullmag_fdm_plan_desc *plan);
     bool upload(const double *m_xyz);
 
-    // ---- one evaluation: H_d by the FFT convolution, then the field kernel ----
-    bool demag_field(const double *m) {
+    // ---- one evaluation: the spectrum of its input lies in X, the column passes turn it into
+    // the field's, and the row pass that evaluates it also forms and transforms the next input ----
+    bool columns() {
         if (!demag) return true;
         const Conv64 &C = conv;
-        const int nrows = ny * nz;
-        const size_t smx = sizeof(double2) * 2 * C.px, smy = sizeof(double2) * 2 * C.py;
-        x_forward64<<<dim3(nrows, 3), kT, smx, stream>>>(C, m, tier > 0 ? phi : nullptr, X);
+        Col64 P{};
+        P.C = C;
+        P.early = early;
+        auto tiles = [&](int tx) { return (unsigned)((C.nkx + tx - 1) / tx); };
+        cudaError_t e;
         if (C.thin) {
-            y_convolve64<<<C.nkx, kT, 3 * smy, stream>>>(C, X);
+            P.tx = tx_c;
+            P.in = X;
+            P.out = X;
+            e = launch_pdl(convolve64<true>, dim3(tiles(tx_c)), dim3(kTC), conv_smem(tx_c), stream, P);
         } else {
-            y_forward64<<<dim3(C.nkx, nz, 3), kT, smy, stream>>>(C, X, Y);
-            z_convolve64<<<dim3(C.nkx, C.py), kT, sizeof(double2) * 6 * C.pz, stream>>>(C, Y);
-            y_inverse64<<<dim3(C.nkx, nz, 3), kT, smy, stream>>>(C, Y, X);
+            P.tx = tx_y;
+            P.in = X;
+            P.out = Y;
+            e = launch_pdl(y_forward64, dim3(tiles(tx_y), nz, 3), dim3(kTC), y_smem(tx_y), stream, P);
+            P.tx = tx_c;
+            P.in = Y;
+            if (e == cudaSuccess) e = launch_pdl(convolve64<false>, dim3(tiles(tx_c), C.py), dim3(kTC), conv_smem(tx_c), stream, P);
+            P.tx = tx_y;
+            P.out = X;
+            if (e == cudaSuccess) e = launch_pdl(y_inverse64, dim3(tiles(tx_y), nz, 3), dim3(kTC), y_smem(tx_y), stream, P);
         }
-        x_inverse64<<<dim3(nrows, 3), kT, smx, stream>>>(C, X, hd, mask, tier > 0 ? phi : nullptr);
-        // the correction's source weights phi_s are the volume fractions whenever the plan has them
-        if (corr_targets > 0)
-            demag_correction64<<<std::max(1u, std::min(1024u, (corr_targets + kT - 1) / kT)), kT, 0, stream>>>(
-                hd, m, phi, ctidx, csidx, ctensor, ms, n, corr_targets, corr_stencil);
-        return !fail("demag kernels", cudaGetLastError());
+        return !fail("demag column passes", e);
+    }
+    size_t conv_smem(int tx) const { return sizeof(double2) * 6 * (size_t)tx * ((conv.thin ? conv.py : conv.pz) + 1); }
+    size_t y_smem(int tx) const { return sizeof(double2) * 2 * (size_t)tx * y_ls64(conv, tx); }
+    size_t row_smem(int r, int l) const {
+        if (!demag) return 0;
+        return sizeof(double2) * 2 * (size_t)l * row_ls64(conv) + sizeof(double) * 3 * (size_t)r * nx;
+    }
+
+    // Tiles by the number of CTAs: FP64 issue is the bound, so a pass is as long as the SM
+    // with the most lines.  Rows: one per CTA until 2 x 152 CTAs are there, then up to about
+    // 256 cells; columns: the tile with the least ceil(CTAs / 152) x tile, the widest of equals
+    // (64-byte segments from 4 columns on).
+    bool choose_shapes() {
+        constexpr size_t kSoft = 100 * 1024, kHard = kMaxSmem, kRow = kMaxSmem - 1024;  // row pass: static statistics
+        const int nrows = ny * nz;
+        rows = 1;
+        lb = 3;
+        fused_x = true;
+        if (demag) {
+            if (row_smem(1, 3) > kRow) lb = 1;
+            fused_x = row_smem(1, lb) <= kRow;
+        }
+        if (!demag || row_smem(1, 3) <= kSoft) {
+            while (rows < 8 && rows * nx < 256 && nrows / (2 * rows) >= 304 && row_smem(2 * rows, 6 * rows) <= kSoft) rows *= 2;
+            lb = 3 * rows;
+        }
+        if (!demag) return true;
+        auto pick = [&](long long outer, auto smem) {
+            int best = 1;
+            long long bc = 1LL << 60;
+            for (int tx : {1, 2, 4, 8}) {
+                if (tx > 1 && (tx > conv.nkx || smem(tx) > kSoft)) break;
+                const long long ctas = ((conv.nkx + tx - 1) / tx) * outer, c = ((ctas + 151) / 152) * tx;
+                if (c <= bc + bc / 16) {
+                    best = tx;
+                    bc = std::min(c, bc);
+                }
+            }
+            return best;
+        };
+        tx_c = pick(conv.thin ? 1 : conv.py, [&](int tx) { return conv_smem(tx); });
+        tx_y = conv.thin ? 1 : pick(3LL * nz, [&](int tx) { return y_smem(tx); });
+        return conv_smem(tx_c) <= kHard && (conv.thin || y_smem(tx_y) <= kHard) &&
+               (fused_x || sizeof(double2) * 2 * (size_t)conv.px <= kHard);
+    }
+
+    // the sparse correction at m, for the row pass that evaluates m
+    bool correction(const double *m) {
+        if (!demag || corr_targets == 0) return true;
+        if (fail("correction memset", cudaMemsetAsync(hcorr, 0, sizeof(double) * 3 * n, stream))) return false;
+        // the source weights phi_s are the volume fractions whenever the plan has them
+        demag_correction64<<<std::max(1u, std::min(1024u, (corr_targets + kT - 1) / kT)), kT, 0, stream>>>(
+            hcorr, m, phi, ctidx, csidx, ctensor, ms, n, corr_targets, corr_stencil);
+        return !fail("demag correction", cudaGetLastError());
+    }
+
+    // one row pass: evaluation at m (NULL: none) into k, combination into out (NULL: none) or
+    // the transform of fwd, statistics with the final evaluation of a step
+    struct Terms {
+        int nk = 0;
+        const int *kidx = nullptr;  // -1: the derivative of this pass
+        const double *coef = nullptr;
+    };
+    bool row_pass(const double *m, double *k, bool stats, const Terms &comb, double dt, double *out, const double *fwd,
+                  const Terms &err_terms) {
+        Row64 R{};
+        R.f = field_base();
+        R.C = conv;
+        R.early = early;
+        const bool to_x = demag && (out || fwd);
+        if (m) {
+            fields_ok = false;
+            if (!correction(m)) return false;
+            R.f.m = m;
+            R.f.k = k;
+            if (corr_targets > 0 && demag) R.f.hcorr = hcorr;
+            if (stats) {
+                R.f.partials = partials;
+                R.f.hex = hex;
+                R.f.hd = demag ? hd : nullptr;
+                R.f.heff = heff;
+            }
+            if (demag && !fused_x) {
+                x_inverse64<<<dim3(ny * nz, 3), kT, sizeof(double2) * 2 * conv.px, stream>>>(conv, X, hd);
+                R.hd_in = hd;
+            } else if (demag) {
+                R.x_in = X;
+            }
+        }
+        if (to_x && fused_x) R.x_out = X;
+        R.rows = rows;
+        R.lb = lb;
+        R.dt = dt;
+        if (out) {
+            R.m0 = S[cur];
+            R.m_next = out;
+            R.nk = comb.nk;
+            for (int t = 0; t < comb.nk; ++t) {
+                R.kk[t] = comb.kidx[t] < 0 ? nullptr : K[comb.kidx[t]];
+                R.c[t] = comb.coef[t];
+            }
+        }
+        R.m_fwd = fwd;
+        R.ne = err_terms.nk;
+        for (int t = 0; t < err_terms.nk; ++t) {
+            R.ek[t] = err_terms.kidx[t] < 0 ? nullptr : K[err_terms.kidx[t]];
+            R.ec[t] = err_terms.coef[t];
+        }
+        const unsigned nb = (unsigned)((ny * nz + rows - 1) / rows);
+        const bool fft = R.x_in || R.x_out;
+        if (fail("row pass", launch_pdl(row64, dim3(nb), dim3(kT), fft ? row_smem(rows, lb) : 0, stream, R))) return false;
+        if (to_x && !fused_x) {
+            x_forward64<<<dim3(ny * nz, 3), kT, sizeof(double2) * 2 * conv.px, stream>>>(conv, out ? out : fwd,
+                                                                                        tier > 0 ? phi : nullptr, X);
+            if (fail("x forward", cudaGetLastError())) return false;
+        }
+        if (stats && fail("finalize", launch_pdl(finalize64, dim3(1), dim3(kT), 0, stream, partials, (int)nb, dstats, (int)early)))
+            return false;
+        return (out || fwd) ? columns() : true;
     }
 
     Field64 field_base() const {
@@ -761,9 +1237,6 @@ struct Fp64Engine {
         P.ny = ny;
         P.nz = nz;
         P.n = n;
-        P.hd = demag ? hd : nullptr;
-        P.hex = hex;
-        P.heff = heff;
         P.mask = mask;
         P.region = region;
         P.lut = lut;
@@ -777,11 +1250,20 @@ struct Fp64Engine {
         P.delta_min = delta_min;
         P.exchange = exchange;
         P.per = per;
+        const double inv_mu0ms = 1.0 / (kMu0d * ms);
         P.a_ex = a_ex;
-        P.ms = ms;
         P.dx = dx;
         P.dy = dy;
         P.dz = dz;
+        P.inv2[0] = 1.0 / (dx * dx);
+        P.inv2[1] = 1.0 / (dy * dy);
+        P.inv2[2] = 1.0 / (dz * dz);
+        P.ex_s = 2.0 / (kMu0d * ms);
+        P.ku1c = 2.0 * inv_mu0ms * ku1;
+        P.ku2c = 4.0 * inv_mu0ms * ku2;
+        P.kc1c = -2.0 * kc1 * inv_mu0ms;
+        P.kc2c = -2.0 * kc2 * inv_mu0ms;
+        P.kc3c = -4.0 * kc3 * inv_mu0ms;
         P.has_ext = has_ext;
         for (int c = 0; c < 3; ++c) {
             P.hext[c] = hext[c];
@@ -803,52 +1285,21 @@ struct Fp64Engine {
         return P;
     }
 
-    // RHS at m into k (when non-null); with stats the statistics land in dstats[0..7]
-    bool eval(const double *m, double *k, bool stats) {
-        fields_ok = false;
-        if (!demag_field(m)) return false;
-        Field64 P = field_base();
-        P.m = m;
-        P.k = k;
-        P.partials = stats ? partials : nullptr;
-        const unsigned nb = blocks_for(n);
-        field64<<<nb, kT, 0, stream>>>(P);
-        if (stats) finalize64<<<1, kT, 0, stream>>>(partials, (int)nb, dstats, 0);
-        return !fail("field kernels", cudaGetLastError());
+    // first stage input of a step, N(m0 + dt sum c_j k_j), and its transforms
+    bool first(int nk, const int *kidx, const double *coef, double dt, double *out) {
+        return row_pass(nullptr, nullptr, false, {nk, kidx, coef}, dt, out, nullptr, {});
     }
-
-    bool combine(const double *m0, int nk, const int *kidx, const double *coef, const double *kcur, double dt, double *out) {
-        Comb64 C{};
-        C.n = n;
-        C.m0 = m0;
-        C.nk = nk;
-        for (int t = 0; t < nk; ++t) {
-            C.k[t] = kidx[t] < 0 ? kcur : K[kidx[t]];
-            C.c[t] = coef[t];
-        }
-        C.dt = dt;
-        C.out = out;
-        combine64<<<blocks_for(n), kT, 0, stream>>>(C);
-        return !fail("combine", cudaGetLastError());
+    // derivative at m (into k, NULL: not stored) and the next input (index -1: this derivative)
+    bool stage(const double *m, double *k, int nk, const int *kidx, const double *coef, double dt, double *out) {
+        return row_pass(m, k, false, {nk, kidx, coef}, dt, out, nullptr, {});
     }
-
-    bool error_norm(int nk, const int *kidx, const double *coef, double dt) {
-        Comb64 C{};
-        C.n = n;
-        C.nk = nk;
-        for (int t = 0; t < nk; ++t) {
-            C.k[t] = K[kidx[t]];
-            C.c[t] = coef[t];
-        }
-        C.dt = dt;
-        const unsigned nb = blocks_for(n);
-        error64<<<nb, kT, 0, stream>>>(C, partials);
-        finalize64<<<1, kT, 0, stream>>>(partials, (int)nb, dstats + kStats, 1);
-        return !fail("error norm", cudaGetLastError());
+    // derivative at the proposed state with the statistics and optional error terms
+    bool final_eval(const double *m, double *k, double dt, int ne = 0, const int *eidx = nullptr, const double *ecoef = nullptr) {
+        return row_pass(m, k, true, {}, dt, nullptr, nullptr, {ne, eidx, ecoef});
     }
 
     bool read_stats() {
-        if (fail("stats copy", cudaMemcpyAsync(hstats, dstats, sizeof(double) * 2 * kStats, cudaMemcpyDeviceToHost, stream)) ||
+        if (fail("stats copy", cudaMemcpyAsync(hstats, dstats, sizeof(double) * kStats, cudaMemcpyDeviceToHost, stream)) ||
             fail("stream sync", cudaStreamSynchronize(stream)))
             return false;
         return true;
@@ -874,7 +1325,8 @@ struct Fp64Engine {
 
     // k1 = f(S[cur]) with the statistics and observables of the committed state
     bool eval_state() {
-        if (!eval(S[cur], K[0], true) || !read_stats()) return false;
+        if (demag && !row_pass(nullptr, nullptr, false, {}, 0.0, nullptr, S[cur], {})) return false;
+        if (!final_eval(S[cur], K[0], 0.0) || !read_stats()) return false;
         memcpy(raw, hstats, sizeof(raw));
         fill_stats(raw);
         k1_valid = true;
@@ -901,25 +1353,25 @@ struct Fp64Engine {
     int rk_fixed(double dt, fullmag_fdm_interrupt_poll_fn poll, void *user) {
         const int nxt = 1 - cur;
         if (integrator == FULLMAG_FDM_INTEGRATOR_RK4) {
-            const int k0[1] = {0}, k1[1] = {1}, k2[1] = {2}, kall[4] = {0, 1, 2, 3};
+            const int k0[1] = {0}, self[1] = {-1}, kall[4] = {0, 1, 2, -1};
             const double h[1] = {0.5}, one[1] = {1.0}, b[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
-            if (!combine(S[cur], 1, k0, h, nullptr, dt, A[0]) || !eval(A[0], K[1], false)) return -1;
+            if (!first(1, k0, h, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 1;
-            if (!combine(S[cur], 1, k1, h, nullptr, dt, A[1]) || !eval(A[1], K[2], false)) return -1;
+            if (!stage(A[0], K[1], 1, self, h, dt, A[1])) return -1;
             if (poll_hit(poll, user)) return 1;
-            if (!combine(S[cur], 1, k2, one, nullptr, dt, A[0]) || !eval(A[0], K[3], false)) return -1;
+            if (!stage(A[1], K[2], 1, self, one, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 1;
-            if (!combine(S[cur], 4, kall, b, nullptr, dt, S[nxt])) return -1;
+            if (!stage(A[0], nullptr, 4, kall, b, dt, S[nxt])) return -1;
         } else {  // Heun
-            const int k0[1] = {0}, kb[2] = {0, 1};
+            const int k0[1] = {0}, kb[2] = {0, -1};
             const double one[1] = {1.0}, half[2] = {0.5, 0.5};
-            if (!combine(S[cur], 1, k0, one, nullptr, dt, A[0]) || !eval(A[0], K[1], false)) return -1;
+            if (!first(1, k0, one, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 1;
-            if (!combine(S[cur], 2, kb, half, nullptr, dt, S[nxt])) return -1;
+            if (!stage(A[0], nullptr, 2, kb, half, dt, S[nxt])) return -1;
         }
         // k1 of the next step (the combination above was the last reader of K[0])
         k1_valid = false;
-        if (!eval(S[nxt], K[0], true) || !read_stats()) return -1;
+        if (!final_eval(S[nxt], K[0], dt) || !read_stats()) return -1;
         commit(dt);
         return 0;
     }
@@ -932,13 +1384,13 @@ struct Fp64Engine {
             static const double a2[1] = {0.5}, a3[1] = {0.75};
             static const double b[3] = {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0};
             static const double e[4] = {-5.0 / 72.0, 1.0 / 12.0, 1.0 / 9.0, -1.0 / 8.0};
-            const int k0[1] = {0}, k1[1] = {1}, kb[3] = {0, 1, 2}, ke[4] = {0, 1, 2, 3};
-            if (!combine(S[cur], 1, k0, a2, nullptr, dt, A[0]) || !eval(A[0], K[1], false)) return -1;
+            const int k0[1] = {0}, self[1] = {-1}, kb[3] = {0, 1, -1}, ke[4] = {0, 1, 2, -1};
+            if (!first(1, k0, a2, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 1, k1, a3, nullptr, dt, A[1]) || !eval(A[1], K[2], false)) return -1;
+            if (!stage(A[0], K[1], 1, self, a3, dt, A[1])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 3, kb, b, nullptr, dt, S[nxt]) || !eval(S[nxt], K[3], true)) return -1;
-            if (!error_norm(4, ke, e, dt)) return -1;
+            if (!stage(A[1], K[2], 3, kb, b, dt, S[nxt])) return -1;
+            if (!final_eval(S[nxt], K[3], dt, 4, ke, e)) return -1;
             kfin = 3;
         } else {
             static const double a21[1] = {1.0 / 5.0};
@@ -949,30 +1401,29 @@ struct Fp64Engine {
             static const double b[5] = {35.0 / 384.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0};
             static const double e[6] = {71.0 / 57600.0, -71.0 / 16695.0, 71.0 / 1920.0, -17253.0 / 339200.0, 22.0 / 525.0,
                                         -1.0 / 40.0};
-            const int k1[1] = {0}, k2[2] = {0, 1}, k3[3] = {0, 1, 2}, k4[4] = {0, 1, 2, 3}, k5[5] = {0, 1, 2, 3, 4};
-            const int kb[5] = {0, 2, 3, 4, 5}, ke[6] = {0, 2, 3, 4, 5, 6};
-            if (!combine(S[cur], 1, k1, a21, nullptr, dt, A[0]) || !eval(A[0], K[1], false)) return -1;
+            const int k1[1] = {0}, k2[2] = {0, -1}, k3[3] = {0, 1, -1}, k4[4] = {0, 1, 2, -1}, k5[5] = {0, 1, 2, 3, -1};
+            const int kb[5] = {0, 2, 3, 4, -1}, ke[6] = {0, 2, 3, 4, 5, -1};
+            if (!first(1, k1, a21, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 2, k2, a3, nullptr, dt, A[1]) || !eval(A[1], K[2], false)) return -1;
+            if (!stage(A[0], K[1], 2, k2, a3, dt, A[1])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 3, k3, a4, nullptr, dt, A[0]) || !eval(A[0], K[3], false)) return -1;
+            if (!stage(A[1], K[2], 3, k3, a4, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 4, k4, a5, nullptr, dt, A[1]) || !eval(A[1], K[4], false)) return -1;
+            if (!stage(A[0], K[3], 4, k4, a5, dt, A[1])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 5, k5, a6, nullptr, dt, A[0]) || !eval(A[0], K[5], false)) return -1;
+            if (!stage(A[1], K[4], 5, k5, a6, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 2;
-            if (!combine(S[cur], 5, kb, b, nullptr, dt, S[nxt]) || !eval(S[nxt], K[6], true)) return -1;
-            if (!error_norm(6, ke, e, dt)) return -1;
+            if (!stage(A[0], K[5], 5, kb, b, dt, S[nxt])) return -1;
+            if (!final_eval(S[nxt], K[6], dt, 6, ke, e)) return -1;
             kfin = 6;
         }
         if (!read_stats()) return -1;
-        const double er = sqrt(hstats[kStats + 8]);
+        const double er = sqrt(hstats[8]);
         const double ex = integrator == FULLMAG_FDM_INTEGRATOR_RK23 ? 1.0 / 3.0 : 0.2;
         if (er <= max_error || dt <= dt_min) {
             double dtn = dt_max;
             if (er > 0.0) dtn = std::min(std::max(headroom * dt * pow(max_error / er, ex), dt_min), dt_max);
-            if (fail("fsal copy", cudaMemcpyAsync(K[0], K[kfin], sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, stream)))
-                return -1;
+            std::swap(K[0], K[kfin]);  // first same as last
             commit(dt);
             cur_stats.suggested_next_dt = dtn;
             next_dt = dtn;
@@ -1002,13 +1453,14 @@ struct Fp64Engine {
         } else {
             const int kp[3] = {abm_hist[0], abm_hist[1], abm_hist[2]};
             const double cp[3] = {23.0 / 12.0, -16.0 / 12.0, 5.0 / 12.0};
-            if (!combine(S[cur], 3, kp, cp, nullptr, dt, A[0]) || !eval(A[0], K[abm_kf], false)) return -1;
+            if (!first(3, kp, cp, dt, A[0])) return -1;
             if (poll_hit(poll, user)) return 1;
-            const int kc[3] = {abm_kf, abm_hist[0], abm_hist[1]};
+            const int kc[3] = {-1, abm_hist[0], abm_hist[1]};
             const double cc[3] = {5.0 / 12.0, 8.0 / 12.0, -1.0 / 12.0};
-            if (!combine(S[cur], 3, kc, cc, nullptr, dt, S[nxt])) return -1;
+            if (!stage(A[0], K[abm_kf], 3, kc, cc, dt, S[nxt])) return -1;
             if (poll_hit(poll, user)) return 1;
-            if (!eval(S[nxt], K[0], true) || !read_stats()) return -1;
+            k1_valid = false;
+            if (!final_eval(S[nxt], K[0], dt) || !read_stats()) return -1;
             const int freed = abm_hist[2];
             abm_hist[2] = abm_hist[1];
             abm_hist[1] = abm_hist[0];
@@ -1144,11 +1596,11 @@ bool Fp64Engine::setup(const fullmag_fdm_plan_desc *plan) {
         if (!alloc(S[s], v3) || !alloc(A[s], v3)) return false;
     for (int s = 0; s < 7; ++s)
         if (!alloc(K[s], v3)) return false;
-    if (!alloc(hex, v3) || !alloc(hd, v3) || !alloc(heff, v3) || !alloc(staging, v3) || !alloc(partials, kRedBlocks * kStats) ||
-        !alloc(dstats, 2 * kStats))
+    if (!alloc(hex, v3) || !alloc(hd, v3) || !alloc(heff, v3) || !alloc(staging, v3) ||
+        !alloc(partials, (size_t)ny * nz * kStats) || !alloc(dstats, kStats) || (corr_targets > 0 && !alloc(hcorr, v3)))
         return false;
     if (fail("cudaMemsetAsync", cudaMemsetAsync(hd, 0, sizeof(double) * v3, stream))) return false;
-    if (fail("cudaMallocHost", cudaMallocHost((void **)&hstats, sizeof(double) * 2 * kStats))) return false;
+    if (fail("cudaMallocHost", cudaMallocHost((void **)&hstats, sizeof(double) * kStats))) return false;
     if (plan->active_mask) {
         has_mask = true;
         mask_host.assign(plan->active_mask, plan->active_mask + n);
@@ -1201,6 +1653,10 @@ bool Fp64Engine::setup(const fullmag_fdm_plan_desc *plan) {
         // periodic axes (fdm_fft.rs:140-160): unpadded, and the backend builds the tensor
         C.px = (per & 1) ? nx : 2 * nx;
         C.py = (per & 2) ? ny : 2 * ny;
+        if (plan->demag_kernel_spectrum_len == 0) {
+            if (!(per & 1)) C.px = pad_extent64(nx);
+            if (!(per & 2)) C.py = pad_extent64(ny);
+        }
         if (per && plan->demag_kernel_spectrum_len != 0)
             return err = "periodic boundaries: the backend builds the image-sum demag tensor, the plan must carry no spectra",
                    false;
@@ -1222,36 +1678,60 @@ bool Fp64Engine::setup(const fullmag_fdm_plan_desc *plan) {
                        false;
         }
         C.thin = thin;
-        C.pz = thin ? 1 : (per & 4) ? nz : 2 * nz;
+        C.pz = thin ? 1 : (per & 4) ? nz : given ? 2 * nz : pad_extent64(nz);
         C.nkx = C.px / 2 + 1;
         C.nky = C.py / 2 + 1;
         C.nkz = C.pz / 2 + 1;
+        // an even x extent is transformed at half its length, two real samples per complex one;
+        // rows too long for the fused row pass take full lines of a pass of their own
+        C.half = C.px % 2 == 0 ? C.px / 2 : 0;
+        if (!choose_shapes()) {
+            C.px = (per & 1) ? nx : 2 * nx;  // the least padding, then again
+            C.py = (per & 2) ? ny : 2 * ny;
+            C.pz = thin ? 1 : (per & 4) ? nz : 2 * nz;
+            C.nkx = C.px / 2 + 1;
+            C.nky = C.py / 2 + 1;
+            C.nkz = C.pz / 2 + 1;
+            C.half = C.px % 2 == 0 ? C.px / 2 : 0;
+            if (!choose_shapes()) return err = "grid too large for the double-precision FFT lines", false;
+        }
+        if (!fused_x) C.half = 0;
         std::vector<double2> tw;
         std::vector<size_t> off;
-        if (!make_plan64(C.px, tw, off, C.plx) || !make_plan64(C.py, tw, off, C.ply) ||
-            (!thin && !make_plan64(C.pz, tw, off, C.plz)))
+        if (!make_plan64(C.half ? C.half : C.px, tw, off, C.plx) || !make_plan64(C.py, tw, off, C.ply) ||
+            !make_plan64(C.pz, tw, off, C.plz))
             return err = "FFT length has too many factors", false;
+        auto even = [](const Plan64 &p) { return p.ns > 0 && p.radix[0] % 2 == 0; };
+        C.xprune = C.half && 2 * ((nx + 1) / 2) <= C.half && even(C.plx);
+        C.yprune = 2 * ny <= C.py && even(C.ply);
+        C.zprune = 2 * nz <= C.pz && even(C.plz);
+        const size_t post = tw.size();
+        for (int k = 0; k <= C.half; ++k) {
+            const double a = 2.0 * M_PI * (double)k / (double)C.px;
+            tw.push_back(make_double2(cos(a), -sin(a)));
+        }
         if (!put(twid, tw.data(), tw.size())) return false;
         C.plx.tw = twid + off[0];
         C.ply.tw = twid + off[1];
-        if (!thin) C.plz.tw = twid + off[2];
+        C.plz.tw = twid + off[2];
+        C.xpost = twid + post;
         const int ncomp = thin ? 4 : 6;
         const size_t kper = per ? (size_t)C.pz * C.py * C.nkx : (size_t)C.nkz * C.nky * C.nkx;
         if (per ? !alloc(kernc, ncomp * kper) : !alloc(kern, ncomp * kper)) return false;
         if (!alloc(X, 3 * (size_t)nz * ny * C.nkx)) return false;
         if (!thin && !alloc(Y, 3 * (size_t)nz * C.py * C.nkx)) return false;
-        const size_t smz = sizeof(double2) * 6 * std::max(C.pz, thin ? C.py : 1);
-        const size_t smx = sizeof(double2) * 2 * std::max(C.px, C.py);
-        if (smz > 227 * 1024 || smx > 227 * 1024) return err = "grid too large for the double-precision FFT lines", false;
-        const void *big[] = {(const void *)z_convolve64, (const void *)y_convolve64, (const void *)x_forward64,
-                             (const void *)x_inverse64, (const void *)y_forward64, (const void *)y_inverse64};
+        const void *big[] = {(const void *)row64, (const void *)convolve64<true>, (const void *)convolve64<false>,
+                             (const void *)x_forward64, (const void *)x_inverse64, (const void *)y_forward64,
+                             (const void *)y_inverse64};
         for (const void *f : big)
-            if (fail("cudaFuncSetAttribute", cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024)))
+            if (fail("cudaFuncSetAttribute", cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                  (int)(f == big[0] ? kMaxSmem - 1024 : kMaxSmem))))
                 return false;
+        const double xs = C.half ? 0.5 : 1.0;  // the packed split stores twice the spectrum (exact)
         if (given) {
             const double *src[6] = {plan->demag_kernel_xx_spectrum, plan->demag_kernel_yy_spectrum, plan->demag_kernel_zz_spectrum,
                                     plan->demag_kernel_xy_spectrum, plan->demag_kernel_xz_spectrum, plan->demag_kernel_yz_spectrum};
-            const double scale = ms / ((double)C.px * C.py * C.pz);
+            const double scale = xs * ms / ((double)C.px * C.py * C.pz);
             std::vector<double> h(ncomp * kper);
             for (int c = 0; c < ncomp; ++c)
                 for (int kz = 0; kz < C.nkz; ++kz)
@@ -1278,13 +1758,16 @@ bool Fp64Engine::setup(const fullmag_fdm_plan_desc *plan) {
             g.nkz = C.nkz;
             g.thin = thin;
             g.per = per;
-            if (per ? !newell_periodic_spectrum_gpu(g, dx, dy, dz, ms, images, nullptr, kernc, stream, err)
-                    : !newell_spectrum_gpu64(g, dx, dy, dz, ms, kern, stream, err))
+            if (per ? !newell_periodic_spectrum_gpu(g, dx, dy, dz, xs * ms, images, nullptr, kernc, stream, err)
+                    : !newell_spectrum_gpu64(g, dx, dy, dz, xs * ms, kern, stream, err))
                 return false;
         }
         C.kern = kern;
         C.kernc = kernc;
+    } else if (!choose_shapes()) {
+        return err = "grid too large", false;
     }
+    early = n <= 65536;
     return true;
 }
 
