@@ -3189,7 +3189,9 @@ struct BatchRound {
     long long max_n3 = 0;
     void *d_blob = nullptr;     // descriptors and work tables
     cudaGraphExec_t exec = nullptr;
-    static constexpr int kRounds = 16;  // rounds per graph launch
+    static constexpr int kRounds = 16;  // most rounds enqueued between two looks at the state
+    std::vector<char> host_blob;        // what d_blob holds: a round of the same descriptors is used again
+    bool synced = true;                 // the engines have taken over the device step control
 
     void release() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -3204,6 +3206,8 @@ struct BatchRound {
         d_stats = nullptr;
         if (d_blob) cudaFree(d_blob);
         d_blob = nullptr;
+        host_blob.clear();
+        members.clear();
         if (h_state) cudaFreeHost(h_state);
         h_state = nullptr;
         if (d_state) cudaFree(d_state);
@@ -3267,7 +3271,7 @@ struct FdmBatch {
     // hands every member's device step control back to its engine: time, accepted steps,
     // statistics of the last accepted step, next step size.
     bool sync_states(std::string &err) {
-        if (!round.exec) return true;
+        if (!round.exec || round.synced) return true;
         const int n = (int)round.members.size();
         const unsigned gx = (unsigned)std::min<long long>((round.max_n3 + 255) / 256, 64);
         batch_commit_all_kernel<<<dim3(gx, n), 256, 0, bstream>>>(round.d_com, round.d_ctl);
@@ -3285,24 +3289,44 @@ struct FdmBatch {
             next_dt[i] = st.next_dt;
             st.steps = 0;
         }
-        return cudaMemcpyAsync(round.d_state, round.h_state, sizeof(BatchState) * n, cudaMemcpyHostToDevice, bstream) ==
-                   cudaSuccess &&
-               cudaStreamSynchronize(bstream) == cudaSuccess;
+        round.synced = true;
+        return true;
+    }
+
+    // Enqueues rounds until the step control is worth a look -- as many as the slowest member
+    // needs at its current step size, at most kRounds -- and reads it.  Returns the rounds, 0 on
+    // failure.  One captured round is launched that many times: sixteen in one graph made the
+    // graph, and every rebuild of it, sixteen times as large.
+    int run_rounds() {
+        double need = 1.0;
+        for (size_t k = 0; k < round.members.size(); ++k) {
+            const BatchState &st = round.h_state[k];
+            if (!st.done && st.next_dt > 0.0) need = std::max(need, std::ceil((st.t_end - st.time) / st.next_dt - 1e-6));
+        }
+        const int r = (int)std::min(need, (double)BatchRound::kRounds);
+        round.synced = false;
+        for (int i = 0; i < r; ++i)
+            if (cudaGraphLaunch(round.exec, bstream) != cudaSuccess) return 0;
+        if (cudaMemcpyAsync(round.h_state, round.d_state, sizeof(BatchState) * round.members.size(), cudaMemcpyDeviceToHost,
+                            bstream) != cudaSuccess ||
+            cudaStreamSynchronize(bstream) != cudaSuccess)
+            return 0;
+        return r;
     }
 
     bool build_round(const std::vector<size_t> &act, double t_end, std::string &err) {
         // the old round's pending commits and step control go back to the engines first
         if (!sync_states(err)) return false;
         if (bstream) cudaStreamSynchronize(bstream);
-        round.release();
         const int n = (int)act.size();
+        if (round.members != act) round.release();
         round.members = act;
-        if (cudaMallocHost((void **)&round.h_ctl, sizeof(BatchCtl) * n) != cudaSuccess ||
+        if (!round.h_ctl && (cudaMallocHost((void **)&round.h_ctl, sizeof(BatchCtl) * n) != cudaSuccess ||
             cudaMallocHost((void **)&round.h_stats, sizeof(double) * kNumStats * n) != cudaSuccess ||
             cudaMallocHost((void **)&round.h_state, sizeof(BatchState) * n) != cudaSuccess ||
             cudaMalloc((void **)&round.d_ctl, sizeof(BatchCtl) * n) != cudaSuccess ||
             cudaMalloc((void **)&round.d_stats, sizeof(double) * kNumStats * n) != cudaSuccess ||
-            cudaMalloc((void **)&round.d_state, sizeof(BatchState) * n) != cudaSuccess) {
+            cudaMalloc((void **)&round.d_state, sizeof(BatchState) * n) != cudaSuccess)) {
             err = "batch round allocation failed";
             return false;
         }
@@ -3375,11 +3399,6 @@ struct FdmBatch {
         for (int k = 0; k < NK * NC; ++k) { o_cw[k] = off; off += al(sizeof(int2) * col_work[k].size()); }
         o_fin = off; off += al(sizeof(FinDesc) * n);
         o_com = off; off += al(sizeof(CommitDesc) * n);
-        if (cudaMalloc(&round.d_blob, off) != cudaSuccess) {
-            err = "batch descriptor allocation failed";
-            return false;
-        }
-        char *blob = (char *)round.d_blob;
         std::vector<char> hb(off);
         for (int s = 0; s < 7; ++s) memcpy(hb.data() + o_rows[s], rows[s].data(), sizeof(RowPass) * rows[s].size());
         for (int k = 0; k < NK * NC; ++k) memcpy(hb.data() + o_cols[k], cols[k].data(), sizeof(ColPass) * cols[k].size());
@@ -3387,12 +3406,28 @@ struct FdmBatch {
         for (int k = 0; k < NK * NC; ++k) memcpy(hb.data() + o_cw[k], col_work[k].data(), sizeof(int2) * col_work[k].size());
         memcpy(hb.data() + o_fin, fin.data(), sizeof(FinDesc) * n);
         memcpy(hb.data() + o_com, com.data(), sizeof(CommitDesc) * n);
-        if (cudaMemcpy(blob, hb.data(), off, cudaMemcpyHostToDevice) != cudaSuccess ||
+        // a call that continues with the same descriptors replays the round it has: only the
+        // step control is new (capturing and instantiating a round takes milliseconds)
+        const bool same = round.exec && hb == round.host_blob;
+        if (!same) {
+            if (round.exec) cudaGraphExecDestroy(round.exec);
+            round.exec = nullptr;
+            if (round.d_blob) cudaFree(round.d_blob);
+            round.d_blob = nullptr;
+            if (cudaMalloc(&round.d_blob, off) != cudaSuccess) {
+                err = "batch descriptor allocation failed";
+                return false;
+            }
+            round.host_blob = std::move(hb);
+        }
+        char *blob = (char *)round.d_blob;
+        if ((!same && cudaMemcpy(blob, round.host_blob.data(), off, cudaMemcpyHostToDevice) != cudaSuccess) ||
             cudaMemcpy(round.d_ctl, round.h_ctl, sizeof(BatchCtl) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(round.d_state, round.h_state, sizeof(BatchState) * n, cudaMemcpyHostToDevice) != cudaSuccess) {
             err = "batch descriptor upload failed";
             return false;
         }
+        if (same) return true;
         round.d_com = (const CommitDesc *)(blob + o_com);
         // capture the round
         long long max_n3 = 0;
@@ -3419,12 +3454,11 @@ struct FdmBatch {
             err = "batch capture failed";
             return false;
         }
-        // kRounds rounds, each: the previous round's commits, the seven passes of an attempt
-        // for every member, the statistics, and the device step control; then the control
-        // state goes to the host once
+        // one round: the previous round's commits, the seven passes of an attempt for every
+        // member, the statistics, and the device step control
         bool ok = true;
         round.max_n3 = max_n3;
-        for (int r = 0; r < BatchRound::kRounds && ok; ++r) {
+        {
             const unsigned gx = (unsigned)std::min<long long>((max_n3 + 255) / 256, 64);
             batch_commit_all_kernel<<<dim3(gx, n), 256, 0, bstream>>>((const CommitDesc *)(blob + o_com), round.d_ctl);
             ok = cudaGetLastError() == cudaSuccess;
@@ -3445,9 +3479,6 @@ struct FdmBatch {
                 ok = cudaGetLastError() == cudaSuccess;
             }
         }
-        if (ok)
-            ok = cudaMemcpyAsync(round.h_state, round.d_state, sizeof(BatchState) * n, cudaMemcpyDeviceToHost, bstream) ==
-                 cudaSuccess;
         const cudaError_t ce = cudaStreamEndCapture(bstream, &graph);
         if (!ok || ce != cudaSuccess || !graph) {
             if (graph) cudaGraphDestroy(graph);
@@ -3505,11 +3536,11 @@ uint32_t fullmag_fdm_batch_size(fullmag_fdm_batch *batch) {
 // t_end stay in the round's work tables with step size 0, which makes their row and
 // column CTAs return at once, until the round is rebuilt without them (when a tenth
 // of its members have finished).  Returns 1 when not batchable.
-// Batched DP45 rounds: each graph launch runs BatchRound::kRounds rounds with the step
-// control on the device (batch_control_kernel); the host reads the control state once per
-// launch to see which problems reached t_end, and rebuilds the round for the remaining
-// ones when fewer than 90 % of its members are still running.  Time to solution is taken
-// at the end of the launch in which a problem finished.
+// Batched DP45 rounds: each look at the state follows up to BatchRound::kRounds rounds with the step
+// control on the device (batch_control_kernel); the host reads the control state after them
+// to see which problems reached t_end, and rebuilds the round for the remaining
+// ones when fewer than half of its members are still running.  Time to solution is taken
+// at the end of the rounds in which a problem finished.
 static int batch_step_until_batched(FdmBatch *b, double t_end, double dt0, uint64_t *out_steps, uint64_t *out_wall_ns) {
     const size_t n = b->items.size();
     const auto t0 = std::chrono::steady_clock::now();
@@ -3526,7 +3557,6 @@ static int batch_step_until_batched(FdmBatch *b, double t_end, double dt0, uint6
         b->last_error = err0;
         return FULLMAG_FDM_ERR_CUDA;
     }
-    b->round.release();
     for (size_t i = 0; i < n; ++i) {
         Engine *e = b->items[i];
         steps0[i] = e->step_count;
@@ -3543,16 +3573,19 @@ static int batch_step_until_batched(FdmBatch *b, double t_end, double dt0, uint6
     }
     bool built = false;
     while (!active.empty()) {
-        if (!built || active.size() * 10 < b->round.members.size() * 9) {
+        // a finished member's CTAs leave at once: a new round pays when half of them do
+        if (!built || active.size() * 2 < b->round.members.size()) {
             std::string err;
             if (!b->build_round(active, t_end, err)) {
+                b->round.release();
                 if (!built) return 1;  // not batchable: caller falls back
                 b->last_error = err;
                 return FULLMAG_FDM_ERR_CUDA;
             }
             built = true;
         }
-        if (cudaGraphLaunch(b->round.exec, b->bstream) != cudaSuccess || cudaStreamSynchronize(b->bstream) != cudaSuccess) {
+        const int rounds = b->run_rounds();
+        if (rounds == 0) {
             b->last_error = "batch round launch failed";
             return FULLMAG_FDM_ERR_CUDA;
         }
@@ -3562,7 +3595,7 @@ static int batch_step_until_batched(FdmBatch *b, double t_end, double dt0, uint6
         for (size_t k = 0; k < mem.size(); ++k) {
             const size_t i = mem[k];
             if (done[i]) continue;
-            b->items[i]->launches += (uint64_t)BatchRound::kRounds * (7 + (b->items[i]->demag ? 6 : 0) + 1);
+            b->items[i]->launches += (uint64_t)rounds * (7 + (b->items[i]->demag ? 6 : 0) + 1);
             if (b->round.h_state[k].done) {
                 done[i] = 1;
                 if (out_wall_ns) out_wall_ns[i] = (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(now - t0).count();
