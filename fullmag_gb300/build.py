@@ -16,7 +16,11 @@ PKG = Path(__file__).resolve().parent
 SRC = PKG / "csrc"
 OUT = PKG / "_build"
 LIB = OUT / "libfullmag_fdm.so"
-SOURCES = ["row_pass.cu", "columns.cu", "engine.cu", "newell.cu", "adjoint.cu", "noalloc.cu", "extra_field.cu", "fp64.cu"]
+SOURCES = ["row_pass.cu", "row_pass_batched.cu", "columns.cu", "columns_z.cu", "columns_conv.cu", "columns_batched.cu", "engine.cu",
+           "newell.cu", "adjoint.cu", "noalloc.cu", "extra_field.cu", "fp64.cu"]
+# kernels per transform length, compiled in groups (FM_GROUP) so that they build in parallel
+GROUPED = ["row_pass_lengths.cu", "columns_lengths.cu"]
+GROUPS = range(7)
 # the cuFFT + unfused measurement baseline: a separate library, never linked into the product
 PLAIN_SOURCES = ["plain_baseline.cu"]
 PLAIN_LIB = OUT / "libfullmag_fdm_plain.so"
@@ -35,7 +39,7 @@ def _stale() -> bool:
     if not LIB.exists() or not PLAIN_LIB.exists():
         return True
     t = min(LIB.stat().st_mtime, PLAIN_LIB.stat().st_mtime)
-    deps = [SRC / s for s in SOURCES + PLAIN_SOURCES if (SRC / s).exists()]
+    deps = [SRC / s for s in SOURCES + GROUPED + PLAIN_SOURCES if (SRC / s).exists()]
     deps += list(SRC.glob("*.cuh")) + list(SRC.glob("*.h")) + [PKG.parent / "include" / "fullmag_fdm.h"]
     return any(d.stat().st_mtime > t for d in deps)
 
@@ -45,11 +49,13 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return LIB
     OUT.mkdir(parents=True, exist_ok=True)
     cc = nvcc()
-    srcs = [s for s in SOURCES + PLAIN_SOURCES if (SRC / s).exists()]
+    # the largest units first
+    units = [(s, g) for s in GROUPED for g in GROUPS] + [(s, None) for s in SOURCES + PLAIN_SOURCES if (SRC / s).exists()]
 
-    def compile_one(s: str) -> Path:
-        obj = OUT / (Path(s).stem + ".o")
-        cmd = [cc, *FLAGS, *ARCH, "-c", str(SRC / s), "-o", str(obj)]
+    def compile_one(unit) -> Path:
+        s, group = unit
+        obj = OUT / (Path(s).stem + ("" if group is None else f"_{group}") + ".o")
+        cmd = [cc, *FLAGS, *([] if group is None else [f"-DFM_GROUP={group}"]), *ARCH, "-c", str(SRC / s), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed on {s}:\n{r.stderr}")
@@ -57,8 +63,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             print(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=len(srcs)) as ex:
-        objs = dict(zip(srcs, ex.map(compile_one, srcs)))
+    with ThreadPoolExecutor(max_workers=max(4, os.cpu_count() or 4)) as ex:
+        objs = dict(zip(units, ex.map(compile_one, units)))
 
     def link(out: Path, parts, libs):
         tmp = out.with_name(out.name + ".tmp")
@@ -68,10 +74,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             raise RuntimeError(f"link of {out.name} failed:\n{r.stderr}")
         os.replace(tmp, out)
 
-    link(LIB, [objs[s] for s in SOURCES if s in objs], ["-lcudart"])
+    link(LIB, [o for (s, _), o in objs.items() if s not in PLAIN_SOURCES], ["-lcudart"])
     # the plain baseline builds its tensor with newell.cu, whose periodic builder uses the
     # FP64 line transforms of fp64.cu
-    link(PLAIN_LIB, [objs[s] for s in PLAIN_SOURCES if s in objs] + [objs["newell.cu"], objs["fp64.cu"]],
+    link(PLAIN_LIB, [objs[(s, None)] for s in [*PLAIN_SOURCES, "newell.cu", "fp64.cu"] if (s, None) in objs],
          ["-lcufft", "-lcudart"])
     return LIB
 

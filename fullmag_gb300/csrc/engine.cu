@@ -516,13 +516,31 @@ struct Engine {
             if (smooth_enough(m)) return m;
         }
     }
-    // Padded extent >= n when the engine builds the tensor: the next power of two.
-    // It is at most 2x the 2,3,5,7-smooth extent, and the compile-time radix-16/8/4
-    // path it selects runs several times faster per point than the generic radices.
-    static int pad_extent(int n, bool even) {
+    // Padded extent >= n when the engine builds the tensor: the next power of two, or the
+    // next length of the two-level transforms (two_level_length) where there is one.  They
+    // run at the speed per point of the powers of two, several times faster than the runtime
+    // radices, on up to half the points per axis.
+    static int pow2_extent(int n) {
         int p2 = 1;
-        while (p2 < std::max(n, even ? 2 : 1)) p2 <<= 1;
+        while (p2 < n) p2 <<= 1;
         return p2;
+    }
+    static int pad_extent(int n) {
+        const int p2 = pow2_extent(n);
+        for (int m = n; m < p2; ++m)
+            if (two_level_length(m)) return m;
+        return p2;
+    }
+    // x: the half length is the one transformed
+    static int pad_x(int nx) { return 2 * pad_extent(nx); }
+    // y of a 3-D grid: at least the shortest two-level length (the fused y+z pass)
+    static int pad_y(int ny, bool thin) { return thin ? pad_extent(2 * ny - 1) : std::max(16, pad_extent(2 * ny - 1)); }
+    // z: every even length up to 16 (the register z passes take them); beyond those, the
+    // z pass over the periodic kernel is the general one, fast at powers of two only
+    static int pad_z(int nz, bool periodic) {
+        if (nz == 1) return 1;
+        const int n = 2 * nz <= 16 ? 2 * nz : pad_extent(2 * nz - 1);
+        return periodic && !z_register_length_ok(n) ? pow2_extent(2 * nz - 1) : n;
     }
 
     bool setup(const fullmag_fdm_plan_desc *plan);
@@ -672,7 +690,7 @@ struct Engine {
     // tx_z doubles as the tile of the fused y+z pass when the (y, z) plane of a kx
     // column fits in shared memory (use_yz)
     int tx_yf = 1, tx_z = 1, tx_yi = 1, tx_2d = 1;
-    int z_pair = 0;  // 1: the z pass runs the packed ky-pair kernel (tile 8)
+    int z_pair = 0;  // z pass: 1 the packed ky-pair kernel (tile 8), 2 the register kernel, 0 the others
     int split_yf = 0, split_z = 0, split_yi = 0;  // radix split of each two-level column pass
     bool use_yz = false;
     int row_blocks = 1;  // CTAs of the row pass at the current rows-per-CTA
@@ -1911,8 +1929,8 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
         }
         thin = g.nz == 1;
         use_gpu_newell = demag;
-        g.px = (g.per & 1) ? g.nx : pad_extent(2 * g.nx - 1, true);
-        g.py = (g.per & 2) ? g.ny : pad_extent(2 * g.ny - 1, false);
+        g.px = (g.per & 1) ? g.nx : pad_x(g.nx);
+        g.py = (g.per & 2) ? g.ny : pad_y(g.ny, thin);
     } else if (demag) {
         const uint64_t len3 = 2ull * (uint64_t)(2 * g.nx) * (2 * g.ny) * (2 * g.nz);
         const uint64_t len2 = 2ull * (uint64_t)(2 * g.nx) * (2 * g.ny);
@@ -1938,12 +1956,22 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
                 use_gpu_newell = true;
         }
         if (use_gpu_newell) {
-            g.px = pad_extent(2 * g.nx - 1, true);
-            g.py = pad_extent(2 * g.ny - 1, false);
+            g.px = pad_x(g.nx);
+            g.py = pad_y(g.ny, thin);
         }
     }
     g.thin = thin ? 1 : 0;
-    g.pz = thin ? 1 : (g.per & 4) ? g.nz : (use_gpu_newell ? pad_extent(2 * g.nz - 1, false) : 2 * g.nz);
+    g.pz = thin ? 1 : (g.per & 4) ? g.nz : (use_gpu_newell ? pad_z(g.nz, g.per != 0) : 2 * g.nz);
+    if (use_gpu_newell && !g.per && !thin && !z_register_length_ok(g.pz)) {
+        // a (y, z) plane that fits the general fused y+z pass keeps the powers of two it is fast at
+        Grid t = g;
+        t.py = pow2_extent(2 * g.ny - 1);
+        t.pz = pow2_extent(2 * g.nz - 1);
+        if (yz_convolve_smem(t, 1) <= 200u * 1024u) {
+            g.py = t.py;
+            g.pz = t.pz;
+        }
+    }
     if (g.px < 2) g.px = 2;
     g.half = g.px / 2;
     g.nkx = g.half + 1;
@@ -2161,10 +2189,13 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     tx_2d = col_tile(g, 3, g.py);
     {
         const char *no_yz = std::getenv("FULLMAG_FDM_NO_FUSED_YZ");
-        use_yz = demag && !thin && !g.per && !(no_yz && *no_yz && *no_yz != '0') && yz_convolve_smem(g, 1) <= 200u * 1024u;
+        // beyond pz = 8 the fused pass needs two CTAs per SM to be worth it
+        const size_t yz_limit = (z_register_length_ok(g.pz) && g.pz > 8 ? 100u : 200u) * 1024u;
+        use_yz = demag && !thin && !g.per && !(no_yz && *no_yz && *no_yz != '0') && yz_convolve_smem(g, 1) <= yz_limit;
+        z_pair = demag && !thin && !use_yz && z_convolve_register_ok(g) ? 2 : 0;
         if (use_yz) {
             tx_z = 1;
-            while (tx_z < 8 && yz_convolve_smem(g, 2 * tx_z) <= 200u * 1024u) tx_z *= 2;
+            while (tx_z < 8 && yz_convolve_smem(g, 2 * tx_z) <= yz_limit) tx_z *= 2;
         }
     }
     const size_t vec = sizeof(float) * 3 * (size_t)g.n;
@@ -2352,7 +2383,7 @@ bool Engine::autotune() {
             tx_z = std::max(1, v[2]);
             tx_yi = std::max(1, v[3]);
             tx_2d = std::max(1, v[4]);
-            z_pair = v[5] && z_convolve_pair_ok(g, tx_z) ? 1 : 0;
+            z_pair = v[5] == 2 && z_convolve_register_ok(g) ? 2 : v[5] && z_convolve_pair_ok(g, tx_z) ? 1 : 0;
             split_yf = v[6] != 0;
             split_z = v[7] != 0;
             split_yi = v[8] != 0;
@@ -2439,25 +2470,30 @@ bool Engine::autotune() {
             };
             tx_yf = tune(tx_yf, split_yf, two_splits(g.py), ysm,
                          [&](int tx, int sp) { return launch_y_forward(cp(plan_y, tx, sp, X, Y), stream) == cudaSuccess; });
-            tx_z = tune(tx_z, split_z, two_splits(g.pz), [&](int tx) { return z_convolve_smem(g, tx); },
-                        [&](int tx, int sp) { return launch_z_convolve(cp(plan_z, tx, sp, Y, Y), stream) == cudaSuccess; });
-            // the packed ky-pair z pass (tile 8) against the best unpaired launch;
-            // FULLMAG_FDM_Z_PAIR=0 or 1 forces the choice
-            z_pair = 0;
-            const char *zp_env = std::getenv("FULLMAG_FDM_Z_PAIR");
-            if (z_convolve_pair_ok(g, 8) && zp_env && zp_env[0] == '1') {
-                tx_z = 8;
-                z_pair = 1;
-                split_z = 0;
-            } else if (z_convolve_pair_ok(g, 8) && !(zp_env && zp_env[0] == '0')) {
-                ColPass best = cp(plan_z, tx_z, split_z, Y, Y), paired = col_pass(plan_z, 8, Y, Y);
-                paired.pipe = 1;
-                const float t_best = time_ms([&] { return launch_z_convolve(best, stream) == cudaSuccess; });
-                const float t_pair = time_ms([&] { return launch_z_convolve(paired, stream) == cudaSuccess; });
-                if (t_pair < t_best) {
+            // pz <= 24: the register z pass moves its bytes once with no shared memory
+            if (z_convolve_register_ok(g)) {
+                z_pair = 2;
+            } else {
+                tx_z = tune(tx_z, split_z, two_splits(g.pz), [&](int tx) { return z_convolve_smem(g, tx); },
+                            [&](int tx, int sp) { return launch_z_convolve(cp(plan_z, tx, sp, Y, Y), stream) == cudaSuccess; });
+                // the packed ky-pair z pass (tile 8) against the best unpaired launch;
+                // FULLMAG_FDM_Z_PAIR=0 or 1 forces the choice
+                z_pair = 0;
+                const char *zp_env = std::getenv("FULLMAG_FDM_Z_PAIR");
+                if (z_convolve_pair_ok(g, 8) && zp_env && zp_env[0] == '1') {
                     tx_z = 8;
                     z_pair = 1;
                     split_z = 0;
+                } else if (z_convolve_pair_ok(g, 8) && !(zp_env && zp_env[0] == '0')) {
+                    ColPass best = cp(plan_z, tx_z, split_z, Y, Y), paired = col_pass(plan_z, 8, Y, Y);
+                    paired.pipe = 1;
+                    const float t_best = time_ms([&] { return launch_z_convolve(best, stream) == cudaSuccess; });
+                    const float t_pair = time_ms([&] { return launch_z_convolve(paired, stream) == cudaSuccess; });
+                    if (t_pair < t_best) {
+                        tx_z = 8;
+                        z_pair = 1;
+                        split_z = 0;
+                    }
                 }
             }
             tx_yi = tune(tx_yi, split_yi, two_splits(g.py), ysm,
@@ -3250,8 +3286,8 @@ struct FdmBatch {
 
     // Enqueues launch(id, stream) for every id as parallel branches that fork from and
     // join back into bstream (inside a capture: graph nodes with no edges between them).
-    template <typename F>
-    bool fan_out(const std::vector<int> &ids, F &&launch) {
+    template <typename T, typename F>
+    bool fan_out(const std::vector<T> &ids, F &&launch) {
         if (ids.empty()) return true;
         if (ids.size() == 1) return launch(ids[0], bstream) == cudaSuccess;
         const int ns = std::min<int>((int)ids.size(), kSide);
@@ -3330,19 +3366,28 @@ struct FdmBatch {
             err = "batch round allocation failed";
             return false;
         }
-        // Work is bucketed by shared-memory class so one large member does not set the
-        // occupancy of every CTA: row buckets rb, column groups (kind, class).
-        constexpr int NC = 5;
+        // Work is bucketed by kernel (class of the row pass, kind of the column pass) and by
+        // shared-memory class, so one large member does not set the occupancy of every CTA.
         auto smem_class = [](size_t b) {
             return b <= 24u * 1024u ? 0 : b <= 48u * 1024u ? 1 : b <= 96u * 1024u ? 2 : b <= 150u * 1024u ? 3 : 4;
         };
+        constexpr int NC = 8;
+        struct RowBucket {
+            int cls = 0;
+            size_t smem = 0, offset = 0;
+            std::vector<int2> work;
+        };
+        struct ColBucket {
+            int kind = 0;
+            size_t smem = 0, offset = 0, work_offset = 0;
+            std::vector<ColPass> passes;
+            std::vector<int2> work;
+        };
         std::vector<RowPass> rows[7];
-        constexpr int NK = 4;  // column kernel kinds (col_batched_kind)
-        std::vector<ColPass> cols[NK * NC];
-        std::vector<int2> row_work[NC], col_work[NK * NC];
+        std::map<int, RowBucket> row_buckets;  // x class, smem class
+        std::map<int, ColBucket> col_buckets;  // kind, smem class
         std::vector<FinDesc> fin(n);
         std::vector<CommitDesc> com(n);
-        size_t row_smem[NC] = {0, 0, 0, 0, 0}, col_smem[NK * NC] = {};
         std::vector<RowPass> rec;
         std::vector<int> kinds;
         for (int k = 0; k < n; ++k) {
@@ -3368,23 +3413,24 @@ struct FdmBatch {
                 rows[s].push_back(rec[s]);
                 rs = std::max(rs, row_pass_smem(rec[s]));
             }
-            const int rb = smem_class(rs);
-            row_smem[rb] = std::max(row_smem[rb], rs);
+            const int cls = row_pass_class(e->g, e->demag);
+            RowBucket &rb = row_buckets[cls * NC + smem_class(rs)];
+            rb.cls = cls;
+            rb.smem = std::max(rb.smem, rs);
             const int nb = row_pass_blocks(rec[0]);
-            for (int b = 0; b < nb; ++b) row_work[rb].push_back(make_int2(k, b));
+            for (int b = 0; b < nb; ++b) rb.work.push_back(make_int2(k, b));
             if (e->demag) {
-                const int kind = kinds[0];
                 const bool thin = e->g.thin != 0;
                 const int tx = thin ? e->tx_2d : e->tx_z;
                 const size_t cs = thin ? y_convolve_2d_smem(e->g, tx) : yz_convolve_smem(e->g, tx);
-                const int cg = kind * NC + smem_class(cs);
+                ColBucket &cb = col_buckets[kinds[0] * NC + smem_class(cs)];
+                cb.kind = kinds[0];
+                cb.smem = std::max(cb.smem, cs);
                 ColPass c = e->col_pass(e->plan_y, tx, e->X, e->X);
                 c.skip_dt = &round.d_ctl[k].dt;
-                const int idx = (int)cols[cg].size();
-                cols[cg].push_back(c);
                 const int ntiles = (e->g.nkx + tx - 1) / tx;
-                for (int t = 0; t < ntiles; ++t) col_work[cg].push_back(make_int2(idx, t));
-                col_smem[cg] = std::max(col_smem[cg], cs);
+                for (int t = 0; t < ntiles; ++t) cb.work.push_back(make_int2((int)cb.passes.size(), t));
+                cb.passes.push_back(c);
             }
             fin[k] = FinDesc{e->partials, nb, 0};
             com[k] = CommitDesc{e->S[0], e->S[1], e->K[0], e->K[6], 3 * e->g.n};
@@ -3392,18 +3438,27 @@ struct FdmBatch {
         // one device blob for every descriptor array
         size_t off = 0;
         auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-        size_t o_rows[7], o_cols[NK * NC], o_rw[NC], o_cw[NK * NC], o_fin, o_com;
-        for (int s = 0; s < 7; ++s) { o_rows[s] = off; off += al(sizeof(RowPass) * rows[s].size()); }
-        for (int k = 0; k < NK * NC; ++k) { o_cols[k] = off; off += al(sizeof(ColPass) * cols[k].size()); }
-        for (int k = 0; k < NC; ++k) { o_rw[k] = off; off += al(sizeof(int2) * row_work[k].size()); }
-        for (int k = 0; k < NK * NC; ++k) { o_cw[k] = off; off += al(sizeof(int2) * col_work[k].size()); }
+        auto place = [&](size_t bytes) {
+            const size_t at = off;
+            off += al(bytes);
+            return at;
+        };
+        size_t o_rows[7], o_fin, o_com;
+        for (int s = 0; s < 7; ++s) o_rows[s] = place(sizeof(RowPass) * rows[s].size());
+        for (auto &b : row_buckets) b.second.offset = place(sizeof(int2) * b.second.work.size());
+        for (auto &b : col_buckets) {
+            b.second.offset = place(sizeof(ColPass) * b.second.passes.size());
+            b.second.work_offset = place(sizeof(int2) * b.second.work.size());
+        }
         o_fin = off; off += al(sizeof(FinDesc) * n);
         o_com = off; off += al(sizeof(CommitDesc) * n);
         std::vector<char> hb(off);
         for (int s = 0; s < 7; ++s) memcpy(hb.data() + o_rows[s], rows[s].data(), sizeof(RowPass) * rows[s].size());
-        for (int k = 0; k < NK * NC; ++k) memcpy(hb.data() + o_cols[k], cols[k].data(), sizeof(ColPass) * cols[k].size());
-        for (int k = 0; k < NC; ++k) memcpy(hb.data() + o_rw[k], row_work[k].data(), sizeof(int2) * row_work[k].size());
-        for (int k = 0; k < NK * NC; ++k) memcpy(hb.data() + o_cw[k], col_work[k].data(), sizeof(int2) * col_work[k].size());
+        for (auto &b : row_buckets) memcpy(hb.data() + b.second.offset, b.second.work.data(), sizeof(int2) * b.second.work.size());
+        for (auto &b : col_buckets) {
+            memcpy(hb.data() + b.second.offset, b.second.passes.data(), sizeof(ColPass) * b.second.passes.size());
+            memcpy(hb.data() + b.second.work_offset, b.second.work.data(), sizeof(int2) * b.second.work.size());
+        }
         memcpy(hb.data() + o_fin, fin.data(), sizeof(FinDesc) * n);
         memcpy(hb.data() + o_com, com.data(), sizeof(CommitDesc) * n);
         // a call that continues with the same descriptors replays the round it has: only the
@@ -3433,22 +3488,25 @@ struct FdmBatch {
         long long max_n3 = 0;
         for (auto &c : com) max_n3 = std::max(max_n3, c.n3);
         // set the shared-memory limits outside the capture
-        size_t max_row = 0, max_col = 0;
-        for (int k = 0; k < NC; ++k) max_row = std::max(max_row, row_smem[k]);
-        for (int k = 0; k < NK * NC; ++k) max_col = std::max(max_col, col_smem[k]);
-        launch_row_pass_batched((const RowPass *)(blob + o_rows[0]), (const int2 *)(blob + o_rw[0]), 0, max_row, bstream);
-        for (int kd = 0; kd < NK; ++kd)
-            launch_col_batched((const ColPass *)(blob + o_cols[0]), (const int2 *)(blob + o_cw[0]), 0, kd, max_col, bstream);
+        std::vector<const RowBucket *> row_ids;
+        std::vector<const ColBucket *> col_ids;
+        for (auto &b : row_buckets) {
+            row_ids.push_back(&b.second);
+            for (bool lean : {false, true})
+                launch_row_pass_batched(nullptr, nullptr, 0, b.second.cls, lean, b.second.smem, bstream);
+        }
+        for (auto &b : col_buckets) {
+            col_ids.push_back(&b.second);
+            launch_col_batched(nullptr, nullptr, 0, b.second.kind, b.second.smem, bstream);
+        }
+        // the largest launches first, so that the small ones run beside them
+        std::stable_sort(row_ids.begin(), row_ids.end(), [](auto *a, auto *b) { return a->work.size() > b->work.size(); });
+        std::stable_sort(col_ids.begin(), col_ids.end(), [](auto *a, auto *b) { return a->work.size() > b->work.size(); });
         cudaGetLastError();
         if (!ensure_branches()) {
             err = "batch stream or event creation failed";
             return false;
         }
-        std::vector<int> row_ids, col_ids;
-        for (int rb = 0; rb < NC; ++rb)
-            if (!row_work[rb].empty()) row_ids.push_back(rb);
-        for (int cg = 0; cg < NK * NC; ++cg)
-            if (!col_work[cg].empty()) col_ids.push_back(cg);
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(bstream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             err = "batch capture failed";
@@ -3463,14 +3521,15 @@ struct FdmBatch {
             batch_commit_all_kernel<<<dim3(gx, n), 256, 0, bstream>>>((const CommitDesc *)(blob + o_com), round.d_ctl);
             ok = cudaGetLastError() == cudaSuccess;
             for (int s = 0; s < 7 && ok; ++s) {
-                ok = fan_out(row_ids, [&](int rb, cudaStream_t st) {
-                    return launch_row_pass_batched((const RowPass *)(blob + o_rows[s]), (const int2 *)(blob + o_rw[rb]),
-                                                   (int)row_work[rb].size(), row_smem[rb], st);
+                // passes 1 to 5 are intermediate stages (0 has no right-hand side, 6 the statistics)
+                ok = fan_out(row_ids, [&](const RowBucket *rb, cudaStream_t st) {
+                    return launch_row_pass_batched((const RowPass *)(blob + o_rows[s]), (const int2 *)(blob + rb->offset),
+                                                   (int)rb->work.size(), rb->cls, s > 0 && s < 6, rb->smem, st);
                 });
                 if (ok && s < 6)
-                    ok = fan_out(col_ids, [&](int cg, cudaStream_t st) {
-                        return launch_col_batched((const ColPass *)(blob + o_cols[cg]), (const int2 *)(blob + o_cw[cg]),
-                                                  (int)col_work[cg].size(), cg / NC, col_smem[cg], st);
+                    ok = fan_out(col_ids, [&](const ColBucket *cb, cudaStream_t st) {
+                        return launch_col_batched((const ColPass *)(blob + cb->offset), (const int2 *)(blob + cb->work_offset),
+                                                  (int)cb->work.size(), cb->kind, cb->smem, st);
                     });
             }
             if (ok) ok = launch_finalize_batched((const FinDesc *)(blob + o_fin), n, round.d_stats, bstream) == cudaSuccess;

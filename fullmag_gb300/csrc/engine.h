@@ -170,7 +170,7 @@ struct ColPass {
     const float *kern;       // demag kernel (multiply passes)
     int inverse;
     const double *skip_dt;   // batched rounds: the problem's step size; <= 0 skips its tiles
-    int pipe;                // z pass: 1 = the packed ky-pair kernel (tile 8)
+    int pipe;                // z pass: 1 = the packed ky-pair kernel (tile 8), 2 = the register kernel
     int split;               // two-level passes: 0 the default radix split N1 x N2, 1 the alternative
     int early;               // let the next kernel launch early (pdl_trigger)
 };
@@ -192,8 +192,10 @@ bool newell_periodic_spectrum_gpu(const Grid &g, double dx, double dy, double dz
 // K[c][kz][ky][kx] -> K[c][kz][kx][ky] (the fused y+z path's layout), out of place
 cudaError_t launch_kern_ky_fast(const float *in, float *out, int ncomp, int nkz, int nky, int nkx, cudaStream_t s);
 size_t z_convolve_smem(const Grid &g, int tx);
-// the packed ky-pair z pass exists for this grid at tile tx
+// the packed ky-pair z pass exists for this grid at tile tx / the register z pass exists
 bool z_convolve_pair_ok(const Grid &g, int tx);
+bool z_convolve_register_ok(const Grid &g);
+bool z_register_length_ok(int pz);  // z lengths of the register z passes
 size_t y_pass_smem(const Grid &g, int tx);
 size_t y_convolve_2d_smem(const Grid &g, int tx);
 
@@ -285,13 +287,20 @@ struct FinDesc {
     int nblocks;
     int pad;
 };
-cudaError_t launch_row_pass_batched(const RowPass *ps, const int2 *work, int nwork, size_t smem, cudaStream_t s);
+// The work table of one launch holds problems of one class of x lengths and passes that are
+// all intermediate stages (lean) or not; nwork 0 only prepares the kernel.
+cudaError_t launch_row_pass_batched(const RowPass *ps, const int2 *work, int nwork, int cls, bool lean, size_t smem,
+                                    cudaStream_t s);
+int row_pass_length(const Grid &g, bool demag);  // x half length of the row-pass instance, 0: the general one
+int row_pass_class(const Grid &g, bool demag);   // its class: 0 general, 1 up to 64, 2 up to 256, 3 longer
 cudaError_t launch_col_batched(const ColPass *ps, const int2 *work, int nwork, int kind, size_t smem, cudaStream_t s);
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s);
 cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early = 0);
 int row_pass_blocks(const RowPass &p);
-// Kernel of the batched column pass for a grid: 0 thin film pruned, 1 fused y+z pruned,
-// 2 thin film general, 3 fused y+z general.
+// Kernel of the batched column pass for a grid: 3 k + c with k = 0 thin film two-level, 1 fused
+// y+z two-level, 2 its longer z lengths and c the class of py (0 up to 64, 1 up to 256, 2
+// longer); 9 thin film general, 10 fused y+z general.  nwork 0 only prepares the kernel.
+constexpr int kColBatchedKinds = 11;
 int col_batched_kind(const Grid &g);
 int col_tile(const Grid &g, int lines_per_col, int len);
 

@@ -43,8 +43,33 @@ __device__ __forceinline__ float2 plane_b(cp2 v) { return make_float2(v.re.y, v.
 __device__ __forceinline__ float4 pstore(cp2 v) { return make_float4(v.re.x, v.re.y, v.im.x, v.im.y); }
 __device__ __forceinline__ cp2 pload(float4 f) { return {make_float2(f.x, f.y), make_float2(f.z, f.w)}; }
 
+__device__ __forceinline__ cp2 vadd(cp2 a, cp2 b) { return padd(a, b); }
+__device__ __forceinline__ cp2 vsub(cp2 a, cp2 b) { return psub(a, b); }
+__device__ __forceinline__ cp2 vscale(float c, cp2 a) { return {__fmul2_rn(pb(c), a.re), __fmul2_rn(pb(c), a.im)}; }
+__device__ __forceinline__ cp2 vfma(float c, cp2 a, cp2 b) {
+    return {__ffma2_rn(pb(c), a.re, b.re), __ffma2_rn(pb(c), a.im, b.im)};
+}
+__device__ __forceinline__ cp2 vmul_mi(cp2 a, bool inv) { return pmul_mi(a, inv); }
+
 template <int R>
 __device__ __forceinline__ void pdft(cp2 *v, bool inv);
+template <int R>
+__device__ __forceinline__ void dft_v(cp2 *v, bool inv) {
+    pdft<R>(v, inv);
+}
+
+template <>
+__device__ __forceinline__ void pdft<3>(cp2 *v, bool inv) {
+    dft_odd<3>(v, inv);
+}
+template <>
+__device__ __forceinline__ void pdft<5>(cp2 *v, bool inv) {
+    dft_odd<5>(v, inv);
+}
+template <>
+__device__ __forceinline__ void pdft<7>(cp2 *v, bool inv) {
+    dft_odd<7>(v, inv);
+}
 
 template <>
 __device__ __forceinline__ void pdft<2>(cp2 *v, bool) {
@@ -115,6 +140,11 @@ __device__ __forceinline__ void pdft<16>(cp2 *v, bool inv) {
 #pragma unroll
         for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = b[k2];
     }
+}
+
+template <>
+__device__ __forceinline__ void pdft<6>(cp2 *v, bool inv) {
+    dft_coprime<2, 3>(v, inv);
 }
 
 // Pruned two-level forms of half_dft_store / half_idft_load (fft_smem.cuh) on pairs; the

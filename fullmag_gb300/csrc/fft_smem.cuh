@@ -13,6 +13,9 @@
 // arithmetic folded to shifts and masks.  Other lengths use the runtime path
 // with radices 8, 4, 2 and an O(R^2) loop for any other prime factor.  Twiddles are FP64-computed host-side and stored as
 // float2 e^{-2 pi i e / n}; the inverse conjugates them.
+//
+// The passes over engine-built tensors take the two-level transforms further down at the
+// lengths of two_level_length (2^a times 1, 5/4, 3/2 or 7/4).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -78,7 +81,10 @@ __device__ __forceinline__ void ff_add(float &hi, float &lo, float v) {
     hi = s;
     lo += e;
 }
-__host__ __device__ constexpr int skewed_len(int n) { return n + (n >> 4) + 1; }
+__host__ __device__ constexpr int skewed_len(int n) {
+    // odd, so that neighbouring lines start in different banks
+    return (n + (n >> 4) + 1) | 1;
+}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -91,8 +97,111 @@ __device__ __forceinline__ float2 mul_mi(float2 a, bool inv) {
     return inv ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
+// ---- butterflies of radix 3, 5, 7 and of two coprime factors, on one complex line
+// (float2) or on a pair of lines (cp2, fft_pair.cuh) ----
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return cadd(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return csub(a, b); }
+__device__ __forceinline__ float2 vscale(float c, float2 a) { return make_float2(c * a.x, c * a.y); }
+__device__ __forceinline__ float2 vfma(float c, float2 a, float2 b) {
+    return make_float2(fmaf(c, a.x, b.x), fmaf(c, a.y, b.y));
+}
+__device__ __forceinline__ float2 vmul_mi(float2 a, bool inv) { return mul_mi(a, inv); }
+
+// cos and sin of 2 pi m / P for P = 3, 5, 7 (m < P)
+template <int P>
+__device__ __forceinline__ constexpr float odd_cos(int m) {
+    constexpr float c3 = -0.5f;
+    constexpr float c5[2] = {0.30901699437494742410f, -0.80901699437494742410f};
+    constexpr float c7[3] = {0.62348980185873353053f, -0.22252093395631440429f, -0.90096886790241912624f};
+    const int q = m > P / 2 ? P - m : m;
+    return q == 0 ? 1.f : P == 3 ? c3 : P == 5 ? c5[(q - 1) & 1] : c7[q - 1];
+}
+template <int P>
+__device__ __forceinline__ constexpr float odd_sin(int m) {
+    constexpr float s3 = 0.86602540378443864676f;
+    constexpr float s5[2] = {0.95105651629515357212f, 0.58778525229247312917f};
+    constexpr float s7[3] = {0.78183148246802980871f, 0.97492791218182360702f, 0.43388373911755812048f};
+    const int q = m > P / 2 ? P - m : m;
+    const float v = q == 0 ? 0.f : P == 3 ? s3 : P == 5 ? s5[(q - 1) & 1] : s7[q - 1];
+    return m > P / 2 ? -v : v;
+}
+
+// Odd prime P: the inputs n and P - n are folded into a sum and a difference, so each
+// output pair k, P - k takes P - 1 real-by-complex products.
+template <int P, typename V>
+__device__ __forceinline__ void dft_odd(V *v, bool inv) {
+    constexpr int H = P / 2;
+    V t[H], d[H];
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+        t[j] = vadd(v[1 + j], v[P - 1 - j]);
+        d[j] = vsub(v[1 + j], v[P - 1 - j]);
+    }
+    const V v0 = v[0];
+    V sum = v0;
+#pragma unroll
+    for (int j = 0; j < H; ++j) sum = vadd(sum, t[j]);
+    v[0] = sum;
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+        V m = vfma(odd_cos<P>(k % P), t[0], v0), n = vscale(odd_sin<P>(k % P), d[0]);
+#pragma unroll
+        for (int j = 1; j < H; ++j) {
+            m = vfma(odd_cos<P>(((j + 1) * k) % P), t[j], m);
+            n = vfma(odd_sin<P>(((j + 1) * k) % P), d[j], n);
+        }
+        n = vmul_mi(n, inv);
+        v[k] = vadd(m, n);
+        v[P - k] = vsub(m, n);
+    }
+}
+
 template <int R>
 __device__ __forceinline__ void dft_small(float2 *v, bool inv);
+template <int R>
+__device__ __forceinline__ void dft_v(float2 *v, bool inv) {
+    dft_small<R>(v, inv);
+}
+
+// R = A B with A, B coprime (the prime-factor map n = B a + A b mod R, k -> (k mod A,
+// k mod B)): an A x B transform without twiddles.
+template <int A, int B, typename V>
+__device__ __forceinline__ void dft_coprime(V *v, bool inv) {
+    constexpr int R = A * B;
+    V t[A][B];
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) t[a][b] = v[(B * a + A * b) % R];
+        dft_v<B>(t[a], inv);
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        V u[A];
+#pragma unroll
+        for (int a = 0; a < A; ++a) u[a] = t[a][b];
+        dft_v<A>(u, inv);
+#pragma unroll
+        for (int a = 0; a < A; ++a) t[a][b] = u[a];
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = t[k % A][k % B];
+}
+
+template <>
+__device__ __forceinline__ void dft_small<1>(float2 *, bool) {}
+template <>
+__device__ __forceinline__ void dft_small<3>(float2 *v, bool inv) {
+    dft_odd<3>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<5>(float2 *v, bool inv) {
+    dft_odd<5>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<7>(float2 *v, bool inv) {
+    dft_odd<7>(v, inv);
+}
 
 template <>
 __device__ __forceinline__ void dft_small<2>(float2 *v, bool) {
@@ -175,28 +284,62 @@ __device__ __forceinline__ void dft_small<16>(float2 *v, bool inv) {
     }
 }
 
+template <>
+__device__ __forceinline__ void dft_small<6>(float2 *v, bool inv) {
+    dft_coprime<2, 3>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<10>(float2 *v, bool inv) {
+    dft_coprime<2, 5>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<12>(float2 *v, bool inv) {
+    dft_coprime<4, 3>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<14>(float2 *v, bool inv) {
+    dft_coprime<2, 7>(v, inv);
+}
+
 // radix of the next power-of-two stage given the remaining length 2^m:
 // radix 16 where possible, never a lone radix-2 stage (2^5 -> 8 x 4, 2^9 -> 16 x 8 x 4)
 __host__ __device__ constexpr int pow2_radix(int rem) {
     return rem >= 16 && rem != 32 ? 16 : (rem >= 8 ? 8 : rem);
 }
 
-// ---- pruned two-level transforms (power-of-two lengths N = N1 * N2) ----
+// ---- two-level transforms, N = N1 * N2 with N1 even ----
 // With n = N2 n1 + n2 and k = k1 + N1 k2:
 //   X[k1 + N1 k2] = sum_n2 W_N2^{n2 k2} W_N^{n2 k1} sum_n1 x[N2 n1 + n2] W_N1^{n1 k1}.
-// Inputs vanish for n >= N/2 (n1 >= N1/2) on the forward side and only n < N/2 is kept
-// on the inverse side, so the outer N1-point passes run on half lines.  tw holds the N
-// twiddles e^{-2 pi i e / N}.
+// Along an open axis inputs vanish for n >= N/2 (n1 >= N1/2) on the forward side and only
+// n < N/2 is kept on the inverse side, so the outer N1-point passes run on half lines;
+// along a periodic axis (no padding) they run on full ones.  tw holds the N twiddles
+// e^{-2 pi i e / N}.
+//
+// Lengths: 2^a, 5/4 2^a, 3/2 2^a and 7/4 2^a from 16 to 512, so that padding 2n - 1 samples
+// up to the next one costs at most a quarter (11 % on average over log-uniform n) where a
+// power of two costs up to a factor of two per axis.  A 150 x 150 x 10 box takes 320 x 320
+// x 20 points instead of 512 x 512 x 32.
+__host__ __device__ constexpr bool two_level_length(int n) {
+    return n == 16 || n == 20 || n == 24 || n == 28 || n == 32 || n == 40 || n == 48 || n == 56 || n == 64 || n == 80 ||
+           n == 96 || n == 112 || n == 128 || n == 160 || n == 192 || n == 224 || n == 256 || n == 320 || n == 384 ||
+           n == 448 || n == 512;
+}
+// Outer length N1 of a pass whose inner pass holds one line of N2 = n / N1 values a thread:
+// both at most 16 (N1 counts half on open axes) up to n = 256.
+__host__ __device__ constexpr int split_line(int n) {
+    return n <= 28 ? 4 : n <= 64 ? 8 : n <= 256 ? 16 : n / 16;
+}
+// The same for a convolution pass, whose inner pass holds three lines: N2 <= 8 up to 256.
+__host__ __device__ constexpr int split_conv(int n) {
+    return n <= 28 ? 4 : n <= 64 ? 8 : n <= 128 ? 16 : n <= 256 ? n / 8 : 32;
+}
 
-// Half-input N1-point DFT of e[0..N1/2) (two N1/2-point DFTs: even and odd outputs),
-// times W_N^{n2 k1}, stored at line[sk(k1 * N2 + n2)].
+// N1-point DFT given as its even (e) and odd (o) halves -- inputs of the two N1/2-point
+// DFTs that give the even and odd outputs -- times W_N^{n2 k1}, at line[sk(k1 * N2 + n2)].
 template <int N1, int N2>
-__device__ __forceinline__ void half_dft_store(float2 (&e)[N1 / 2], int n2, float2 *line, const float2 *__restrict__ tw) {
+__device__ __forceinline__ void dft_halves_store(float2 (&e)[N1 / 2], float2 (&o)[N1 / 2], int n2, float2 *line,
+                                                 const float2 *__restrict__ tw) {
     constexpr int H1 = N1 / 2;
-    float2 o[H1];
-    o[0] = e[0];
-#pragma unroll
-    for (int n1 = 1; n1 < H1; ++n1) o[n1] = cmul(e[n1], __ldg(tw + n1 * N2));
     dft_small<H1>(e, false);
     dft_small<H1>(o, false);
 #pragma unroll
@@ -207,24 +350,62 @@ __device__ __forceinline__ void half_dft_store(float2 (&e)[N1 / 2], int n2, floa
     }
 }
 
-// Half-output inverse N1-point DFT over line[sk(k1 * N2 + n2)], k1 in [0, N1): returns
-// y[n1] for n1 < N1/2 in e (two N1/2-point inverses combined with W_N1^{-n1}).
+// Half-input N1-point DFT of e[0..N1/2).
 template <int N1, int N2>
-__device__ __forceinline__ void half_idft_load(float2 (&e)[N1 / 2], int n2, const float2 *line,
-                                               const float2 *__restrict__ tw) {
+__device__ __forceinline__ void half_dft_store(float2 (&e)[N1 / 2], int n2, float2 *line, const float2 *__restrict__ tw) {
     constexpr int H1 = N1 / 2;
     float2 o[H1];
+    o[0] = e[0];
+#pragma unroll
+    for (int n1 = 1; n1 < H1; ++n1) o[n1] = cmul(e[n1], __ldg(tw + n1 * N2));
+    dft_halves_store<N1, N2>(e, o, n2, line, tw);
+}
+
+// Full N1-point DFT of e[0..N1/2) and f[0..N1/2) = x[N1/2 + n1].
+template <int N1, int N2>
+__device__ __forceinline__ void full_dft_store(float2 (&e)[N1 / 2], float2 (&f)[N1 / 2], int n2, float2 *line,
+                                               const float2 *__restrict__ tw) {
+    constexpr int H1 = N1 / 2;
+#pragma unroll
+    for (int n1 = 0; n1 < H1; ++n1) {
+        const float2 d = csub(e[n1], f[n1]);
+        e[n1] = cadd(e[n1], f[n1]);
+        f[n1] = n1 ? cmul(d, __ldg(tw + n1 * N2)) : d;
+    }
+    dft_halves_store<N1, N2>(e, f, n2, line, tw);
+}
+
+// Inverse N1-point DFT over line[sk(k1 * N2 + n2)], k1 in [0, N1): y[n1] for n1 < N1/2 in e
+// (two N1/2-point inverses combined with W_N1^{-n1}); FULL: y[N1/2 + n1] in f.
+template <int N1, int N2, bool FULL>
+__device__ __forceinline__ void idft_load(float2 (&e)[N1 / 2], float2 (&f)[N1 / 2], int n2, const float2 *line,
+                                          const float2 *__restrict__ tw) {
+    constexpr int H1 = N1 / 2;
 #pragma unroll
     for (int u = 0; u < H1; ++u) {
         e[u] = line[sk(2 * u * N2 + n2)];
-        o[u] = line[sk((2 * u + 1) * N2 + n2)];
+        f[u] = line[sk((2 * u + 1) * N2 + n2)];
     }
     dft_small<H1>(e, true);
-    dft_small<H1>(o, true);
-    e[0] = cadd(e[0], o[0]);
+    dft_small<H1>(f, true);
 #pragma unroll
-    for (int n1 = 1; n1 < H1; ++n1) e[n1] = cadd(e[n1], cmul(o[n1], cconj(__ldg(tw + n1 * N2))));
+    for (int n1 = 0; n1 < H1; ++n1) {
+        const float2 o = n1 ? cmul(f[n1], cconj(__ldg(tw + n1 * N2))) : f[n1];
+        if (FULL) f[n1] = csub(e[n1], o);
+        e[n1] = cadd(e[n1], o);
+    }
 }
+template <int N1, int N2>
+__device__ __forceinline__ void half_idft_load(float2 (&e)[N1 / 2], int n2, const float2 *line,
+                                               const float2 *__restrict__ tw) {
+    float2 o[N1 / 2];
+    idft_load<N1, N2, false>(e, o, n2, line, tw);
+}
+
+// case labels of the two-level lengths: F(n) for each
+#define FM_LENGTHS_TO_256(F) \
+    F(16) F(20) F(24) F(28) F(32) F(40) F(48) F(56) F(64) F(80) F(96) F(112) F(128) F(160) F(192) F(224) F(256)
+#define FM_LENGTHS_LONG(F) F(320) F(384) F(448) F(512)
 
 // ---- runtime-length path ----
 
