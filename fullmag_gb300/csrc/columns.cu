@@ -1,5 +1,5 @@
 // columns.cu -- y transforms of the demag convolution, plus the deterministic final
-// reduction of the per-block statistics.
+// reduction of the per-block statistics of batched problems.
 //
 // Reference behaviour restated (paths in mzrptu/fullmag):
 //   multi-pass FP64 reductions                 native/backends/fdm/src/reductions_fp64.cu:30-84,354-393
@@ -239,13 +239,6 @@ __device__ __forceinline__ void finalize_body(const float2 *__restrict__ partial
     }
 }
 
-__global__ void __launch_bounds__(kFinThreads) finalize_stats_kernel(const float2 *__restrict__ partials, int nblocks,
-                                                                     double *__restrict__ out, int early) {
-    pdl_wait();
-    if (early) pdl_trigger();
-    finalize_body(partials, nblocks, out);
-}
-
 // One block per problem; statistics land in out[problem * kNumStats + s].
 __global__ void __launch_bounds__(kFinThreads) finalize_batched_kernel(const FinDesc *__restrict__ fd, double *__restrict__ out) {
     const FinDesc d = fd[blockIdx.x];
@@ -315,10 +308,6 @@ cudaError_t launch_y_inverse(const ColPass &p, cudaStream_t s) {
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s) {
     finalize_batched_kernel<<<nproblems, kFinThreads, 0, s>>>(fd, out);
     return cudaGetLastError();
-}
-
-cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early) {
-    return launch_pdl(finalize_stats_kernel, dim3(1), dim3(kFinThreads), 0, s, partials, nblocks, out, early);
 }
 
 namespace {

@@ -33,8 +33,8 @@
 namespace fm {
 
 static constexpr double kMu0 = 4.0 * M_PI * 1e-7;
-// device statistics slots: the kNumStats row-pass statistics, the step size of graph
-// replays, and the extra field pass's five sums (ExtraSums: Zeeman m.(H_ext + H_map), DMI,
+// statistics slots: the kNumStats row-pass statistics, one unused, and the extra field pass's
+// five sums (ExtraSums: Zeeman m.(H_ext + H_map), DMI,
 // uniaxial and cubic energy densities, region exchange pair sum)
 static constexpr int kStatSlots = kNumStats + 6;
 
@@ -365,8 +365,8 @@ struct Engine {
     float *kern = nullptr;
     uint8_t *mask = nullptr;
     float2 *partials = nullptr;  // [kNumStats][row blocks] float-float partial sums
-    double *dstats = nullptr;
-    double *hstats = nullptr;  // pinned
+    double *hstats = nullptr;  // pinned; kernels write it
+    unsigned *fin_count = nullptr;
     float2 *twid = nullptr;
     float2 *xpost = nullptr;
     FftPlan plan_x{}, plan_y{}, plan_z{};
@@ -679,6 +679,10 @@ struct Engine {
             rec_rows->push_back(p);
             return true;
         }
+        if (p.partials) {
+            p.fin_out = hstats;
+            p.fin_count = fin_count;
+        }
         launches += 1;
         kt_begin(KT_ROW);
         const cudaError_t rc = launch_row_pass(p, stream);
@@ -791,21 +795,13 @@ struct Engine {
         return run_row(p) && run_columns();
     }
 
+    // The row pass that collects statistics finalizes them itself, into the pinned hstats; the
+    // extra pass before it left per-CTA sums of its own.
     bool enqueue_stats() {
-        if (rec_rows) return true;  // the batched round finalizes all problems at once
+        if (rec_rows || !has_extra) return true;  // a batched round finalizes all problems at once
         launches += 1;
-        kt_begin(KT_FIN);
-        const cudaError_t rc = launch_finalize_stats(partials, row_blocks, dstats, stream, early_launch ? 1 : 0);
-        kt_end();
-        if (cuda_fail("finalize", rc)) return false;
-        if (has_extra) {  // the extra pass before this evaluation left its per-CTA sums
-            launches += 1;
-            if (cuda_fail("extra finalize",
-                          launch_extra_finalize(xpart, extra_field_blocks(g), dstats + kNumStats + 1, stream, early_launch ? 1 : 0)))
-                return false;
-        }
-        return !cuda_fail("stats copy",
-                          cudaMemcpyAsync(hstats, dstats, sizeof(double) * kStatSlots, cudaMemcpyDeviceToHost, stream));
+        return !cuda_fail("extra finalize", launch_extra_finalize(xpart, extra_field_blocks(g), hstats + kNumStats + 1, stream,
+                                                                  early_launch ? 1 : 0));
     }
 
     bool read_stats() {
@@ -861,7 +857,7 @@ struct Engine {
         p.m_in = S[cur];
         // a valid k1 stays: after DP45 / RK23 it is the first-same-as-last derivative, taken
         // inside the step (with that step's Oersted current and thermal counter)
-        p.k_out = k1_valid ? nullptr : K[0];
+        p.k_out = k1_valid ? nullptr : K[k1_slot()];
         p.partials = partials;
         if (write_fields) {
             p.h_ex_out = h_ex;
@@ -895,6 +891,10 @@ struct Engine {
         }
         p.dt = (float)dt;
         p.dt_dev = pass_dt_dev;
+        if (!m_in && pass_dt_host) {
+            p.dt_dev = pass_dt_host;
+            p.dt_copy = pass_dt_dev;
+        }
         p.x_out = X;
         return run_row(p) && run_columns();
     }
@@ -921,15 +921,12 @@ struct Engine {
     // One executable per state parity (the committed state alternates between
     // S[0] and S[1]); re-captured when dt changes.  With an interrupt poll
     // installed the step runs pass by pass instead, polling in between.
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    double gdt[2] = {0.0, 0.0};
-    uint64_t gkernels[2] = {0, 0};
     bool use_graphs = true;
 
     void drop_graphs() {
         for (int c = 0; c < 2; ++c) {
-            if (gexec[c]) cudaGraphExecDestroy(gexec[c]);
-            gexec[c] = nullptr;
+            gstep[c].drop();
+            ginner[c].drop();
             if (dexec[c]) cudaGraphExecDestroy(dexec[c]);
             dexec[c] = nullptr;
         }
@@ -962,12 +959,13 @@ struct Engine {
     }
 
     // Final evaluation at m (k1' -> K[0], statistics) fused with the next step's first stage.
-    bool final_prepare(float *m, double dt, bool sync) {
+    // stats false: an inner step of step_many, whose statistics nobody reads.
+    bool final_prepare(float *m, double dt, bool sync, bool stats = true) {
         RowPass p = row_base();
         p.x_in = X;
         p.m_in = m;
         p.k_out = K[0];
-        p.partials = partials;
+        p.partials = stats ? partials : nullptr;
         p.m0 = m;
         p.m_next = A[0];
         p.n_comb = 1;
@@ -975,13 +973,13 @@ struct Engine {
         p.comb_c[0] = (float)first_coef();
         p.dt = (float)dt;
         p.x_out = X;
-        return run_row(p) && run_columns() && (sync ? read_stats() : enqueue_stats());
+        return run_row(p) && run_columns() && (!stats || (sync ? read_stats() : enqueue_stats()));
     }
 
     // Enqueues a Heun or RK4 step from S[cur] into S[1-cur]; `poll_between` checks the
     // interrupt callback between passes (eager mode only).  with_first: run the first
     // pass (else X and A[0] already hold it); prepare: end with final_prepare.
-    int enqueue_fixed_step(double dt, bool poll_between, bool with_first = true, bool prepare = false) {
+    int enqueue_fixed_step(double dt, bool poll_between, bool with_first = true, bool prepare = false, bool stats = true) {
         const int nxt = 1 - cur;
         if (integrator == FULLMAG_FDM_INTEGRATOR_RK4) {
             const int self[1] = {-1};
@@ -1002,20 +1000,37 @@ struct Engine {
             const double c[2] = {0.5, 0.5};
             if (!stage(A[0], nullptr, 2, k, c, dt, S[nxt])) return -1;
         }
-        if (prepare) return final_prepare(S[nxt], dt, poll_between) ? 0 : -1;
+        if (prepare) return final_prepare(S[nxt], dt, poll_between, stats) ? 0 : -1;
         return final_eval(S[nxt], K[0], 0, nullptr, nullptr, dt, poll_between) ? 0 : -1;
     }
 
-    bool capture_step(double dt) {
-        if (gexec[cur]) {
-            cudaGraphExecDestroy(gexec[cur]);
-            gexec[cur] = nullptr;
+    // A captured run of fixed steps from state parity cur: one step with its statistics, or
+    // (inner) two without.
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        double dt = 0.0;
+        uint64_t kernels = 0;
+        void drop() {
+            if (exec) cudaGraphExecDestroy(exec);
+            exec = nullptr;
         }
+    };
+    StepGraph gstep[2], ginner[2];  // by state parity
+
+    bool ensure_step_graph(StepGraph &sg, double dt, bool inner) {
+        if (sg.exec && sg.dt == dt) return true;
+        sg.drop();
         const uint64_t l0 = launches;
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
         // the graph starts at the second pass: the first runs before it unless prepared
-        const int rc = enqueue_fixed_step(dt, false, false, true);
+        int rc = 0;
+        const int cur0 = cur;
+        for (int k = 0; k < (inner ? 2 : 1) && rc == 0; ++k) {
+            rc = enqueue_fixed_step(dt, false, false, true, !inner);
+            if (inner) cur = 1 - cur;
+        }
+        cur = cur0;
         const cudaError_t e = cudaStreamEndCapture(stream, &graph);
         launches = l0;
         if (rc != 0 || e != cudaSuccess || graph == nullptr) {
@@ -1024,15 +1039,67 @@ struct Engine {
         }
         size_t nnodes = 0;
         cudaGraphGetNodes(graph, nullptr, &nnodes);
-        const cudaError_t ie = cudaGraphInstantiate(&gexec[cur], graph, 0);
+        const cudaError_t ie = cudaGraphInstantiate(&sg.exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) {
-            gexec[cur] = nullptr;
+            sg.exec = nullptr;
             return false;
         }
-        gkernels[cur] = nnodes > 0 ? nnodes - 1 : 0;  // every node but the stats copy is a kernel
-        gdt[cur] = dt;
+        sg.kernels = nnodes;
+        sg.dt = dt;
         return true;
+    }
+    bool launch_steps(const StepGraph &sg) {
+        launches += sg.kernels;
+        return !cuda_fail("graph launch", cudaGraphLaunch(sg.exec, stream));
+    }
+
+    // n steps of a Heun or RK4 run in one call, of which only the last one's statistics are
+    // asked for: the others run without them, and nothing waits in between.  False in `done`:
+    // not run this way (interrupt polls, timing, terms the host sets per step, few steps).
+    int step_fixed_many(double dt, uint64_t n, bool &done) {
+        done = false;
+        const bool fixed = integrator == FULLMAG_FDM_INTEGRATOR_HEUN || integrator == FULLMAG_FDM_INTEGRATOR_RK4;
+        if (!fixed || n < 3 || poll || !use_graphs || ktime || has_thermal || (has_oersted && oe_kind != 0)) return 0;
+        interrupted = false;
+        if (!ensure_k1() || !set_oersted(time, time + dt)) return -1;
+        const bool ready = first_ready(dt);
+        // an odd number of inner steps starts with a whole one; the pairs keep the parity, and
+        // the last step follows them
+        const bool odd = ((n - 1) & 1) != 0;
+        const int c1 = odd ? 1 - cur : cur;
+        const int cur0 = cur;
+        bool ok = !odd || ensure_step_graph(gstep[cur], dt, false);
+        cur = c1;
+        ok = ok && ensure_step_graph(ginner[c1], dt, true) && ensure_step_graph(gstep[c1], dt, false);
+        cur = cur0;
+        if (!ok) {  // capture unavailable: clear the sticky state, the caller steps one by one
+            cudaGetLastError();
+            last_error.clear();
+            prep_ready = prep_ready && ready;
+            return 0;
+        }
+        done = true;
+        if (!ready && !first_stage(dt)) return -1;
+        auto advance = [&] {
+            cur = 1 - cur;
+            step_count += 1;
+            th_step += 1;
+            time += dt;
+        };
+        if (odd) {
+            if (!launch_steps(gstep[cur])) return -1;
+            advance();
+        }
+        for (uint64_t k = 0; k < (n - 1) / 2; ++k) {
+            if (!launch_steps(ginner[cur])) return -1;
+            advance();
+            advance();
+        }
+        if (!launch_steps(gstep[cur]) || cuda_fail("stream sync", cudaStreamSynchronize(stream))) return -1;
+        commit(dt, hstats);
+        mark_next(dt);
+        return 0;
     }
 
     int step_fixed(double dt) {
@@ -1044,7 +1111,7 @@ struct Engine {
         if (!set_oersted(time, time + dt) || !set_thermal(th_step, th_step + 1)) return -1;
         const bool ready = first_ready(dt);
         if (poll == nullptr && use_graphs && !ktime) {
-            if ((!gexec[cur] || gdt[cur] != dt) && !capture_step(dt)) {
+            if (!ensure_step_graph(gstep[cur], dt, false)) {
                 // capture unavailable: clear the sticky state and fall back to eager launches
                 cudaGetLastError();
                 use_graphs = false;
@@ -1052,8 +1119,7 @@ struct Engine {
             }
             if (use_graphs) {
                 if (!ready && !first_stage(dt)) return -1;
-                if (cuda_fail("graph launch", cudaGraphLaunch(gexec[cur], stream))) return -1;
-                launches += gkernels[cur];
+                if (!launch_steps(gstep[cur])) return -1;
                 if (cuda_fail("stream sync", cudaStreamSynchronize(stream))) return -1;
                 commit(dt, hstats);
                 mark_next(dt);
@@ -1089,14 +1155,14 @@ struct Engine {
     // ---- Dormand-Prince 5(4) with first-same-as-last ----
     // An attempt is seven passes from S[cur] into S[1-cur] ending with the error norm
     // and statistics at the proposed state.  With no interrupt poll it runs as one
-    // CUDA graph per state parity: dt comes from a device scalar (an H2D node copies
-    // the host value each replay) and the FSAL hand-over is a device copy K6 -> K0,
-    // so the captured pointers never change.
+    // CUDA graph per state parity: the first pass reads dt from the pinned host value and
+    // leaves it in a device scalar for the others, so the captured pointers never change.
     cudaGraphExec_t dexec[2] = {nullptr, nullptr};
     uint64_t dkernels[2] = {0, 0};
     double *dt_dev = nullptr;   // device scalar (arena)
     double *dt_host = nullptr;  // pinned
-    const double *pass_dt_dev = nullptr;  // set while capturing: passes read dt from dt_dev
+    double *pass_dt_dev = nullptr;        // set while capturing: passes read dt from dt_dev
+    const double *pass_dt_host = nullptr; // ... but the first, which reads it here and hands it on
     bool dp45_pending = false;
     double dp45_dt = 0.0;
 
@@ -1106,7 +1172,11 @@ struct Engine {
     bool adaptive() const {
         return integrator == FULLMAG_FDM_INTEGRATOR_DP45 || integrator == FULLMAG_FDM_INTEGRATOR_RK23;
     }
+    // First same as last: the last derivative of an accepted attempt is k1 of the next one, so
+    // K[0] and the last buffer change roles with the state parity instead of being copied.
     int fsal_index() const { return integrator == FULLMAG_FDM_INTEGRATOR_RK23 ? 3 : 6; }
+    int k1_slot() const { return adaptive() && cur ? fsal_index() : 0; }
+    int last_slot() const { return cur ? 0 : fsal_index(); }
     double ctrl_exp() const { return integrator == FULLMAG_FDM_INTEGRATOR_RK23 ? 1.0 / 3.0 : 0.2; }
 
     // Bogacki-Shampine 3(2) with FSAL (native/backends/fdm/src/llg_rk23_fp32.cu:150-265):
@@ -1118,14 +1188,15 @@ struct Engine {
         static const double b[3] = {2.0 / 9.0, 1.0 / 3.0, 4.0 / 9.0};
         static const double e[4] = {-5.0 / 72.0, 1.0 / 12.0, 1.0 / 9.0, -1.0 / 8.0};
         const int nxt = 1 - cur;
-        const int k1[1] = {0}, self[1] = {-1}, kb[3] = {0, 1, -1}, ke[4] = {0, 1, 2, -1};
+        const int f = k1_slot();
+        const int k1[1] = {f}, self[1] = {-1}, kb[3] = {f, 1, -1}, ke[4] = {f, 1, 2, -1};
         if (!stage(nullptr, nullptr, 1, k1, a2, dt, A[0])) return -1;
         if (poll_between && poll_hit()) return 1;
         if (!stage(A[0], K[1], 1, self, a3, dt, A[1])) return -1;
         if (poll_between && poll_hit()) return 1;
         if (!stage(A[1], K[2], 3, kb, b, dt, S[nxt])) return -1;
         if (poll_between && poll_hit()) return 1;
-        return final_eval(S[nxt], K[3], 4, ke, e, dt, false) ? 0 : -1;
+        return final_eval(S[nxt], K[last_slot()], 4, ke, e, dt, false) ? 0 : -1;
     }
 
     int enqueue_dp45(double dt, bool poll_between) {
@@ -1139,8 +1210,9 @@ struct Engine {
         static const double e[6] = {71.0 / 57600.0, -71.0 / 16695.0, 71.0 / 1920.0, -17253.0 / 339200.0, 22.0 / 525.0,
                                     -1.0 / 40.0};
         const int nxt = 1 - cur;
-        const int k1[1] = {0}, k2[2] = {0, -1}, k3[3] = {0, 1, -1}, k4[4] = {0, 1, 2, -1}, k5[5] = {0, 1, 2, 3, -1};
-        const int kb[5] = {0, 2, 3, 4, -1}, ke[6] = {0, 2, 3, 4, 5, -1};
+        const int f = k1_slot();
+        const int k1[1] = {f}, k2[2] = {f, -1}, k3[3] = {f, 1, -1}, k4[4] = {f, 1, 2, -1}, k5[5] = {f, 1, 2, 3, -1};
+        const int kb[5] = {f, 2, 3, 4, -1}, ke[6] = {f, 2, 3, 4, 5, -1};
         if (!stage(nullptr, nullptr, 1, k1, a21, dt, A[0])) return -1;
         if (poll_between && poll_hit()) return 1;
         if (!stage(A[0], K[1], 2, k2, a3, dt, A[1])) return -1;
@@ -1153,7 +1225,7 @@ struct Engine {
         if (poll_between && poll_hit()) return 1;
         if (!stage(A[0], K[5], 5, kb, b, dt, S[nxt])) return -1;
         if (poll_between && poll_hit()) return 1;
-        return final_eval(S[nxt], K[6], 6, ke, e, dt, false) ? 0 : -1;
+        return final_eval(S[nxt], K[last_slot()], 6, ke, e, dt, false) ? 0 : -1;
     }
 
     bool capture_dp45() {
@@ -1164,10 +1236,11 @@ struct Engine {
         const uint64_t l0 = launches;
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
-        bool ok = cudaMemcpyAsync(dt_dev, dt_host, sizeof(double), cudaMemcpyHostToDevice, stream) == cudaSuccess;
         pass_dt_dev = dt_dev;
-        if (ok) ok = enqueue_dp45(0.0, false) == 0;
+        pass_dt_host = dt_host;
+        const bool ok = enqueue_dp45(0.0, false) == 0;
         pass_dt_dev = nullptr;
+        pass_dt_host = nullptr;
         const cudaError_t e = cudaStreamEndCapture(stream, &graph);
         launches = l0;
         if (!ok || e != cudaSuccess || graph == nullptr) {
@@ -1182,7 +1255,7 @@ struct Engine {
             dexec[cur] = nullptr;
             return false;
         }
-        dkernels[cur] = nnodes > 2 ? nnodes - 2 : 0;  // all but the dt and stats copies
+        dkernels[cur] = nnodes;
         return true;
     }
 
@@ -1228,10 +1301,6 @@ struct Engine {
         if (err <= max_error || dt <= dt_min) {
             double dt_next = dt_max;
             if (err > 0.0) dt_next = std::min(std::max(headroom * dt * pow(max_error / err, ctrl_exp()), dt_min), dt_max);
-            // first-same-as-last: the last derivative (at the accepted state) is the next step's k1
-            if (cuda_fail("fsal copy", cudaMemcpyAsync(K[0], K[fsal_index()], sizeof(float) * 3 * (size_t)g.n,
-                                                       cudaMemcpyDeviceToDevice, stream)))
-                return -1;
             commit(dt, hstats);
             cur_stats.suggested_next_dt = dt_next;
             next_dt = dt_next;
@@ -1251,7 +1320,7 @@ struct Engine {
         thermal_dt_for(dt);
         if (!ensure_k1()) return -1;
         if (!set_oersted(time, time + dt) || !set_thermal(th_step, th_step + 1)) return -1;
-        if (use_graphs && (!gexec[cur] || gdt[cur] != dt) && !capture_step(dt)) {
+        if (use_graphs && !ensure_step_graph(gstep[cur], dt, false)) {
             cudaGetLastError();
             use_graphs = false;
             last_error.clear();
@@ -1259,8 +1328,7 @@ struct Engine {
         const bool ready = first_ready(dt);
         if (use_graphs) {
             if (!ready && !first_stage(dt)) return -1;
-            if (cuda_fail("graph launch", cudaGraphLaunch(gexec[cur], stream))) return -1;
-            launches += gkernels[cur];
+            if (!launch_steps(gstep[cur])) return -1;
         } else if (enqueue_fixed_step(dt, false, !ready, true) != 0) {
             return -1;
         }
@@ -1561,7 +1629,7 @@ struct Engine {
 
     // Records the seven row passes and six column passes of one attempt, with dt read
     // from dt_ptr.  False when a pass cannot run batched (large 3-D grids).
-    bool record_attempt(const double *dt_ptr, std::vector<RowPass> &rows, std::vector<int> &cols) {
+    bool record_attempt(double *dt_ptr, std::vector<RowPass> &rows, std::vector<int> &cols) {
         rows.clear();
         cols.clear();
         if (has_extra) return false;  // the extra field pass is not part of the batched rounds
@@ -1598,7 +1666,7 @@ struct Engine {
             double next = dt;
             const int ok = finish_dp45_attempt(next);
             if (ok < 0) return -1;
-            if (ok == 1) return cuda_fail("stream sync", cudaStreamSynchronize(stream)) ? -1 : 0;
+            if (ok == 1) return 0;
             dt = next;
         }
     }
@@ -2217,7 +2285,7 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     take(xlen); take(ylen); take(klen);                     // spectra + kernel
     take(has_mask ? (size_t)g.n : 0);                       // mask
     take(sizeof(float2) * kNumStats * (size_t)max_row_blocks);
-    take(sizeof(double) * kStatSlots);
+    take(2 * sizeof(double));                               // dt of graph replays, finalize counter
     take(sizeof(float2) * tw.size());
     arena_bytes = off;
     if (cuda_fail("cudaMalloc(arena)", cudaMalloc((void **)&arena, arena_bytes))) return false;
@@ -2240,9 +2308,11 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     mask = has_mask ? (uint8_t *)(arena + o[q]) : nullptr;
     q++;
     partials = (float2 *)(arena + o[q++]);
-    dstats = (double *)(arena + o[q++]);
+    dt_dev = (double *)(arena + o[q]);
+    fin_count = (unsigned *)(arena + o[q++] + sizeof(double));
     twid = (float2 *)(arena + o[q++]);
     if (cuda_fail("cudaMallocHost(stats)", cudaMallocHost((void **)&hstats, sizeof(double) * kStatSlots))) return false;
+    memset(hstats, 0, sizeof(double) * kStatSlots);
     if (has_extra &&
         (cuda_fail("cudaMalloc(extra field)", cudaMalloc((void **)&hextra, sizeof(float) * 3 * (size_t)g.n)) ||
          cuda_fail("cudaMalloc(extra sums)", cudaMalloc((void **)&xpart, sizeof(ExtraSums) * (size_t)extra_field_blocks(g)))))
@@ -2307,7 +2377,6 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
             return false;
     }
     if (cuda_fail("cudaMallocHost(dt)", cudaMallocHost((void **)&dt_host, sizeof(double)))) return false;
-    dt_dev = dstats + kNumStats;  // slot kNumStats holds dt (kStatSlots)
 
     if (cuda_fail("cudaMemcpy(twiddles)", cudaMemcpyAsync(twid, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice, stream)))
         return false;
@@ -2761,6 +2830,18 @@ int fullmag_fdm_backend_step_many(fullmag_fdm_backend *handle, double dt_seconds
     if (!e->f64 && e->adaptive()) {
         e->last_error = "step_many supports fixed-step integrators only";
         return FULLMAG_FDM_ERR_INVALID;
+    }
+    if (!e->f64 && n_steps > 0 && dt_seconds > 0.0 && std::isfinite(dt_seconds)) {
+        const auto t0 = std::chrono::steady_clock::now();
+        bool done = false;
+        if (e->step_fixed_many(dt_seconds, n_steps, done) < 0) return FULLMAG_FDM_ERR_CUDA;
+        if (done) {
+            const auto t1 = std::chrono::steady_clock::now();
+            *out_stats = e->cur_stats;
+            out_stats->wall_time_ns =
+                (uint64_t)std::chrono::duration_cast<std::chrono::nanoseconds>(t1 - t0).count() / n_steps;
+            return FULLMAG_FDM_OK;
+        }
     }
     for (uint64_t s = 0; s < n_steps; ++s) {
         const int rc = fullmag_fdm_backend_step(handle, dt_seconds, out_stats);

@@ -120,6 +120,8 @@ struct RowPass {
     float *k_out;            // NULL: keep the right-hand side in registers only
     // (3)
     float2 *partials;        // NULL: no statistics; else [kNumStats][gridDim.x] (hi, lo) pairs
+    double *fin_out;         // with partials: the nine sums / maxima of the whole grid go here (NULL: they do not)
+    unsigned *fin_count;     // CTAs that have written their partials; 0 between launches
     int n_err;               // DP45 error terms (0: none); NULL pointer = current k
     const float *err_k[kMaxTerms];
     double err_c[kMaxTerms];
@@ -131,7 +133,8 @@ struct RowPass {
     const float *comb_k[kMaxTerms];  // NULL entry = current k
     float comb_c[kMaxTerms];
     float dt;
-    const double *dt_dev;    // non-NULL: dt (and err_dt) read from device memory (graph replays)
+    const double *dt_dev;    // non-NULL: dt (and err_dt) read through this pointer (graph replays)
+    double *dt_copy;         // non-NULL: CTA 0 leaves the dt it read there for the passes that follow
     // (5)
     float2 *x_out;           // NULL: no forward transform
     const float *m_fwd;      // forward-transform source when m0 == NULL
@@ -295,7 +298,6 @@ int row_pass_length(const Grid &g, bool demag);  // x half length of the row-pas
 int row_pass_class(const Grid &g, bool demag);   // its class: 0 general, 1 up to 64, 2 up to 256, 3 longer
 cudaError_t launch_col_batched(const ColPass *ps, const int2 *work, int nwork, int kind, size_t smem, cudaStream_t s);
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s);
-cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early = 0);
 int row_pass_blocks(const RowPass &p);
 // Kernel of the batched column pass for a grid: 3 k + c with k = 0 thin film two-level, 1 fused
 // y+z two-level, 2 its longer z lengths and c the class of py (0 up to 64, 1 up to 256, 2
