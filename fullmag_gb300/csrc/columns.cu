@@ -20,12 +20,12 @@ __global__ void __launch_bounds__(kThreads) y_forward_kernel(const ColPass p) {
     const int ls = skewed_len(g.py);
     float2 *a = reinterpret_cast<float2 *>(smem);
     float2 *b = a + tx * ls;
-    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.ny * g.nkx;
+    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.ny * g.xs;
     batched_copy<8>(
         g.ny * tx,
         [&](int idx) {
             const int y = p.fd_tx.div(idx), col = idx - y * tx;
-            return col < ncol ? src[(size_t)y * g.nkx + kx0 + col] : make_float2(0.f, 0.f);
+            return col < ncol ? src[(size_t)y * g.xs + kx0 + col] : make_float2(0.f, 0.f);
         },
         [&](int idx, float2 v) {
             const int y = p.fd_tx.div(idx), col = idx - y * tx;
@@ -35,10 +35,10 @@ __global__ void __launch_bounds__(kThreads) y_forward_kernel(const ColPass p) {
         for (int y = g.ny + (threadIdx.x & 31); y < g.py; y += 32) a[line * ls + sk(y)] = make_float2(0.f, 0.f);
     __syncthreads();
     float2 *r = fft_lines(a, b, tx, ls, p.plan, false);
-    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.py * g.nkx;
+    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.py * g.xs;
     for (int idx = threadIdx.x; idx < g.py * tx; idx += blockDim.x) {
         const int y = p.fd_tx.div(idx), col = idx - y * tx;
-        if (col < ncol) dst[(size_t)y * g.nkx + kx0 + col] = r[col * ls + sk(y)];
+        if (col < ncol) dst[(size_t)y * g.xs + kx0 + col] = r[col * ls + sk(y)];
     }
 }
 
@@ -53,12 +53,12 @@ __global__ void __launch_bounds__(kThreads) y_inverse_kernel(const ColPass p) {
     const int ls = skewed_len(g.py);
     float2 *a = reinterpret_cast<float2 *>(smem);
     float2 *b = a + tx * ls;
-    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.py * g.nkx;
+    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.py * g.xs;
     batched_copy<8>(
         g.py * tx,
         [&](int idx) {
             const int y = p.fd_tx.div(idx), col = idx - y * tx;
-            return col < ncol ? src[(size_t)y * g.nkx + kx0 + col] : make_float2(0.f, 0.f);
+            return col < ncol ? src[(size_t)y * g.xs + kx0 + col] : make_float2(0.f, 0.f);
         },
         [&](int idx, float2 v) {
             const int y = p.fd_tx.div(idx), col = idx - y * tx;
@@ -66,10 +66,10 @@ __global__ void __launch_bounds__(kThreads) y_inverse_kernel(const ColPass p) {
         });
     __syncthreads();
     float2 *r = fft_lines(a, b, tx, ls, p.plan, true);
-    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.ny * g.nkx;
+    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.ny * g.xs;
     for (int idx = threadIdx.x; idx < g.ny * tx; idx += blockDim.x) {
         const int y = p.fd_tx.div(idx), col = idx - y * tx;
-        if (col < ncol) dst[(size_t)y * g.nkx + kx0 + col] = r[col * ls + sk(y)];
+        if (col < ncol) dst[(size_t)y * g.xs + kx0 + col] = r[col * ls + sk(y)];
     }
 }
 
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_forward_fused_kernel(const
     const int tx = p.tx, kx0 = blockIdx.x * tx, ncol = min(tx, g.nkx - kx0);
     const int z = blockIdx.y, c = blockIdx.z;
     const float2 *__restrict__ tw = p.plan.tw;
-    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.ny * g.nkx + kx0;
+    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.ny * g.xs + kx0;
     for (int it = threadIdx.x; it < N2 * ncol; it += blockDim.x) {
         int n2, col;
         tile_item(p, ncol, it, n2, col);
@@ -101,19 +101,19 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_forward_fused_kernel(const
 #pragma unroll
         for (int n1 = 0; n1 < H1; ++n1) {
             const int y = N2 * n1 + n2;
-            e[n1] = y < g.ny ? src[(size_t)y * g.nkx + col] : make_float2(0.f, 0.f);
+            e[n1] = y < g.ny ? src[(size_t)y * g.xs + col] : make_float2(0.f, 0.f);
         }
         if constexpr (FULL) {
             float2 f[H1];
 #pragma unroll
-            for (int n1 = 0; n1 < H1; ++n1) f[n1] = src[(size_t)(N2 * (n1 + H1) + n2) * g.nkx + col];
+            for (int n1 = 0; n1 < H1; ++n1) f[n1] = src[(size_t)(N2 * (n1 + H1) + n2) * g.xs + col];
             full_dft_store<N1, N2>(e, f, n2, buf + col * ls, tw);
         } else {
             half_dft_store<N1, N2>(e, n2, buf + col * ls, tw);
         }
     }
     __syncthreads();
-    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.py * g.nkx + kx0;
+    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.py * g.xs + kx0;
     for (int it = threadIdx.x; it < N1 * ncol; it += blockDim.x) {
         int k1, col;
         tile_item(p, ncol, it, k1, col);
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_forward_fused_kernel(const
         for (int n2 = 0; n2 < N2; ++n2) v[n2] = line[sk(k1 * N2 + n2)];
         dft_small<N2>(v, false);
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) dst[(size_t)(k1 + N1 * k2) * g.nkx + col] = v[k2];
+        for (int k2 = 0; k2 < N2; ++k2) dst[(size_t)(k1 + N1 * k2) * g.xs + col] = v[k2];
     }
 }
 
@@ -141,13 +141,13 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_inverse_fused_kernel(const
     const int tx = p.tx, kx0 = blockIdx.x * tx, ncol = min(tx, g.nkx - kx0);
     const int z = blockIdx.y, c = blockIdx.z;
     const float2 *__restrict__ tw = p.plan.tw;
-    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.py * g.nkx + kx0;
+    const float2 *src = p.in + ((size_t)c * g.nz + z) * g.py * g.xs + kx0;
     for (int it = threadIdx.x; it < N1 * ncol; it += blockDim.x) {
         int k1, col;
         tile_item(p, ncol, it, k1, col);
         float2 v[N2];
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) v[k2] = src[(size_t)(k1 + N1 * k2) * g.nkx + col];
+        for (int k2 = 0; k2 < N2; ++k2) v[k2] = src[(size_t)(k1 + N1 * k2) * g.xs + col];
         dft_small<N2>(v, true);
         float2 *line = buf + col * ls;
 #pragma unroll
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_inverse_fused_kernel(const
             line[sk(k1 * N2 + n2)] = (n2 && k1) ? cmul(v[n2], cconj(__ldg(tw + n2 * k1))) : v[n2];
     }
     __syncthreads();
-    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.ny * g.nkx + kx0;
+    float2 *dst = p.out + ((size_t)c * g.nz + z) * g.ny * g.xs + kx0;
     for (int it = threadIdx.x; it < N2 * ncol; it += blockDim.x) {
         int n2, col;
         tile_item(p, ncol, it, n2, col);
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(y_threads(N1), 2) y_inverse_fused_kernel(const
 #pragma unroll
         for (int n1 = 0; n1 < H1; ++n1) {
             const int y = N2 * n1 + n2;
-            if (y < g.ny) dst[(size_t)y * g.nkx + col] = e[n1];
-            if (FULL) dst[(size_t)(y + N2 * H1) * g.nkx + col] = f[n1];
+            if (y < g.ny) dst[(size_t)y * g.xs + col] = e[n1];
+            if (FULL) dst[(size_t)(y + N2 * H1) * g.xs + col] = f[n1];
         }
     }
 }

@@ -63,7 +63,7 @@ __device__ __forceinline__ void yz_forward(const ColPass &p, int kx0, int ncol, 
     constexpr int ls = skewed_len(N);
     const Grid &g = p.g;
     const int tx = p.tx, nlive = 3 * g.nz * ncol;
-    const size_t zstride = (size_t)g.ny * g.nkx;
+    const size_t zstride = (size_t)g.ny * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;
     for (int it = threadIdx.x; it < nlive * N2; it += blockDim.x) {
         int rest, col;
@@ -74,7 +74,7 @@ __device__ __forceinline__ void yz_forward(const ColPass &p, int kx0, int ncol, 
 #pragma unroll
         for (int y1 = 0; y1 < H1; ++y1) {
             const int y = N2 * y1 + n2;
-            e[y1] = y < g.ny ? src[(size_t)y * g.nkx] : make_float2(0.f, 0.f);
+            e[y1] = y < g.ny ? src[(size_t)y * g.xs] : make_float2(0.f, 0.f);
         }
         half_dft_store<N1, N2>(e, n2, A + (cz * tx + col) * ls, tw);
     }
@@ -100,7 +100,7 @@ __device__ __forceinline__ void yz_inverse(const ColPass &p, int kx0, int ncol, 
     constexpr int ls = skewed_len(N);
     const Grid &g = p.g;
     const int tx = p.tx, nlive = 3 * g.nz * ncol;
-    const size_t zstride = (size_t)g.ny * g.nkx;
+    const size_t zstride = (size_t)g.ny * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;
     __syncthreads();
     for (int it = threadIdx.x; it < nlive * N1; it += blockDim.x) {
@@ -127,7 +127,7 @@ __device__ __forceinline__ void yz_inverse(const ColPass &p, int kx0, int ncol, 
 #pragma unroll
         for (int y1 = 0; y1 < H1; ++y1) {
             const int y = N2 * y1 + n2;
-            if (y < g.ny) dst[(size_t)y * g.nkx] = e[y1];
+            if (y < g.ny) dst[(size_t)y * g.xs] = e[y1];
         }
     }
 }
@@ -186,14 +186,14 @@ __device__ __forceinline__ void yz_convolve_general_body(const ColPass &p, const
     const int half_buf = max(nly * lsy, nlz * lsz);
     float2 *P = reinterpret_cast<float2 *>(smem);
     float2 *Q = P + half_buf;
-    const size_t cstride = (size_t)g.nz * g.ny * g.nkx;
+    const size_t cstride = (size_t)g.nz * g.ny * g.xs;
     batched_copy<8>(
         3 * g.nz * g.ny * tx,
         [&](int idx) {
             const int r = p.fd_tx.div(idx), col = idx - r * tx;
             const int r2 = g.fd_ny.div(r), y = r - r2 * g.ny;
             const int c = g.fd_nz.div(r2), z = r2 - c * g.nz;
-            return col < ncol ? p.in[c * cstride + ((size_t)z * g.ny + y) * g.nkx + kx0 + col] : make_float2(0.f, 0.f);
+            return col < ncol ? p.in[c * cstride + ((size_t)z * g.ny + y) * g.xs + kx0 + col] : make_float2(0.f, 0.f);
         },
         [&](int idx, float2 v) {
             const int r = p.fd_tx.div(idx), col = idx - r * tx;
@@ -250,7 +250,7 @@ __device__ __forceinline__ void yz_convolve_general_body(const ColPass &p, const
         const int r2 = g.fd_ny.div(r), y = r - r2 * g.ny;
         const int c = g.fd_nz.div(r2), z = r2 - c * g.nz;
         if (col < ncol)
-            p.out[c * cstride + ((size_t)z * g.ny + y) * g.nkx + kx0 + col] = R4[((c * tx + col) * g.nz + z) * lsy + sk(y)];
+            p.out[c * cstride + ((size_t)z * g.ny + y) * g.xs + kx0 + col] = R4[((c * tx + col) * g.nz + z) * lsy + sk(y)];
     }
 }
 
@@ -265,7 +265,7 @@ __device__ __forceinline__ void y_convolve_2d_fused(const ColPass &p, const int 
     float2 *buf = reinterpret_cast<float2 *>(smem);  // line (c, col) at (c*tx + col)*ls
     const Grid &g = p.g;
     const int tx = p.tx, kx0 = tile * tx, ncol = min(tx, g.nkx - kx0);
-    const size_t cstride = (size_t)g.ny * g.nkx;
+    const size_t cstride = (size_t)g.ny * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;
     const int n13 = 3 * N2 * ncol;
     for (int it = threadIdx.x; it < n13; it += blockDim.x) {
@@ -277,19 +277,19 @@ __device__ __forceinline__ void y_convolve_2d_fused(const ColPass &p, const int 
 #pragma unroll
         for (int n1 = 0; n1 < H1; ++n1) {
             const int y = N2 * n1 + n2;
-            e[n1] = FULL || y < g.ny ? src[(size_t)y * g.nkx] : make_float2(0.f, 0.f);
+            e[n1] = FULL || y < g.ny ? src[(size_t)y * g.xs] : make_float2(0.f, 0.f);
         }
         if constexpr (FULL) {
             float2 f[H1];
 #pragma unroll
-            for (int n1 = 0; n1 < H1; ++n1) f[n1] = src[(size_t)(N2 * (n1 + H1) + n2) * g.nkx];
+            for (int n1 = 0; n1 < H1; ++n1) f[n1] = src[(size_t)(N2 * (n1 + H1) + n2) * g.xs];
             full_dft_store<N1, N2>(e, f, n2, buf + (c * tx + col) * ls, tw);
         } else {
             half_dft_store<N1, N2>(e, n2, buf + (c * tx + col) * ls, tw);
         }
     }
     __syncthreads();
-    const size_t kc = (size_t)(PER ? g.py : g.nky) * g.nkx;
+    const size_t kc = (size_t)(PER ? g.py : g.nky) * g.ks;
     for (int it = threadIdx.x; it < N1 * ncol; it += blockDim.x) {
         int k1, col;
         tile_item(p, ncol, it, k1, col);
@@ -305,13 +305,13 @@ __device__ __forceinline__ void y_convolve_2d_fused(const ColPass &p, const int 
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
             if constexpr (PER) {  // complex kernel K[c][ky][kx]
-                multiply_periodic(reinterpret_cast<const float2 *>(p.kern) + (size_t)(k1 + N1 * k2) * g.nkx + kx, kc, true,
+                multiply_periodic(reinterpret_cast<const float2 *>(p.kern) + (size_t)(k1 + N1 * k2) * g.ks + kx, kc, true,
                                   &m[0][k2], &m[1][k2], &m[2][k2]);
             } else {
                 int kym;
                 float sy;
                 kernel_mirror(k1 + N1 * k2, N, kym, sy);
-                const float *K = p.kern + (size_t)kym * g.nkx + kx;
+                const float *K = p.kern + (size_t)kym * g.ks + kx;
                 const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc), kxy = sy * __ldg(K + 3 * kc);
                 const float2 mx = m[0][k2], my = m[1][k2], mz = m[2][k2];
                 m[0][k2] = make_float2(-(kxx * mx.x + kxy * my.x), -(kxx * mx.y + kxy * my.y));
@@ -339,8 +339,8 @@ __device__ __forceinline__ void y_convolve_2d_fused(const ColPass &p, const int 
 #pragma unroll
         for (int n1 = 0; n1 < H1; ++n1) {
             const int y = N2 * n1 + n2;
-            if (FULL || y < g.ny) dst[(size_t)y * g.nkx] = e[n1];
-            if (FULL) dst[(size_t)(y + N2 * H1) * g.nkx] = f[n1];
+            if (FULL || y < g.ny) dst[(size_t)y * g.xs] = e[n1];
+            if (FULL) dst[(size_t)(y + N2 * H1) * g.xs] = f[n1];
         }
     }
 }
@@ -358,13 +358,13 @@ __device__ __forceinline__ void y_convolve_2d_general_body(const ColPass &p, con
     const int nl = 3 * tx;
     float2 *a = reinterpret_cast<float2 *>(smem);
     float2 *b = a + nl * ls;
-    const size_t cstride = (size_t)g.ny * g.nkx;
+    const size_t cstride = (size_t)g.ny * g.xs;
     batched_copy<8>(
         3 * g.ny * tx,
         [&](int idx) {
             const int r1 = p.fd_tx.div(idx), col = idx - r1 * tx;
             const int c = g.fd_ny.div(r1), y = r1 - c * g.ny;
-            return col < ncol ? p.in[c * cstride + (size_t)y * g.nkx + kx0 + col] : make_float2(0.f, 0.f);
+            return col < ncol ? p.in[c * cstride + (size_t)y * g.xs + kx0 + col] : make_float2(0.f, 0.f);
         },
         [&](int idx, float2 v) {
             const int r1 = p.fd_tx.div(idx), col = idx - r1 * tx;
@@ -377,23 +377,23 @@ __device__ __forceinline__ void y_convolve_2d_general_body(const ColPass &p, con
     float2 *r = fft_lines(a, b, nl, ls, p.plan, false);
     float2 *o = (r == a) ? b : a;
     if (g.per) {  // complex kernel K[c][ky][kx]
-        const size_t kcp = (size_t)g.py * g.nkx;
+        const size_t kcp = (size_t)g.py * g.ks;
         for (int idx = threadIdx.x; idx < g.py * tx; idx += blockDim.x) {
             const int ky = p.fd_tx.div(idx), col = idx - ky * tx;
             const int kx = min(kx0 + col, g.nkx - 1);
-            const float2 *K = reinterpret_cast<const float2 *>(p.kern) + (size_t)ky * g.nkx + kx;
+            const float2 *K = reinterpret_cast<const float2 *>(p.kern) + (size_t)ky * g.ks + kx;
             multiply_periodic(K, kcp, true, r + (0 * tx + col) * ls + sk(ky), r + (1 * tx + col) * ls + sk(ky),
                               r + (2 * tx + col) * ls + sk(ky));
         }
     }
-    const size_t kc = (size_t)g.nky * g.nkx;
+    const size_t kc = (size_t)g.nky * g.ks;
     for (int idx = threadIdx.x; idx < (g.per ? 0 : g.py * tx); idx += blockDim.x) {
         const int ky = p.fd_tx.div(idx), col = idx - ky * tx;
         const int kx = min(kx0 + col, g.nkx - 1);
         int kym;
         float sy;
         kernel_mirror(ky, g.py, kym, sy);
-        const float *K = p.kern + (size_t)kym * g.nkx + kx;
+        const float *K = p.kern + (size_t)kym * g.ks + kx;
         const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc), kxy = sy * __ldg(K + 3 * kc);
         float2 *lx = r + (0 * tx + col) * ls + sk(ky);
         float2 *ly = r + (1 * tx + col) * ls + sk(ky);
@@ -408,7 +408,7 @@ __device__ __forceinline__ void y_convolve_2d_general_body(const ColPass &p, con
     for (int idx = threadIdx.x; idx < 3 * g.ny * tx; idx += blockDim.x) {
         const int r1 = p.fd_tx.div(idx), col = idx - r1 * tx;
         const int c = g.fd_ny.div(r1), y = r1 - c * g.ny;
-        if (col < ncol) p.out[c * cstride + (size_t)y * g.nkx + kx0 + col] = q[(c * tx + col) * ls + sk(y)];
+        if (col < ncol) p.out[c * cstride + (size_t)y * g.xs + kx0 + col] = q[(c * tx + col) * ls + sk(y)];
     }
 }
 

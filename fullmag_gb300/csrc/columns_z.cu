@@ -22,8 +22,8 @@ __global__ void __launch_bounds__(kThreads) z_convolve_kernel(const ColPass p) {
     const int nl = np * 3 * tx;  // line (q, c, col) at ((q*3 + c)*tx + col)
     float2 *a = reinterpret_cast<float2 *>(smem);
     float2 *b = a + (size_t)2 * 3 * tx * ls;
-    const size_t cstride = (size_t)g.nz * g.py * g.nkx;  // component stride of Y
-    const size_t zstride = (size_t)g.py * g.nkx;
+    const size_t cstride = (size_t)g.nz * g.py * g.xs;  // component stride of Y
+    const size_t zstride = (size_t)g.py * g.xs;
     batched_copy<8>(
         np * 3 * g.nz * tx,
         [&](int idx) {
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kThreads) z_convolve_kernel(const ColPass p) {
             const int r2 = g.fd_nz.div(r1), z = r1 - r2 * g.nz;
             const int q = r2 / 3, c = r2 - 3 * q;
             const int ky = q ? kyb : kya;
-            return col < ncol ? p.in[c * cstride + z * zstride + (size_t)ky * g.nkx + kx0 + col] : make_float2(0.f, 0.f);
+            return col < ncol ? p.in[c * cstride + z * zstride + (size_t)ky * g.xs + kx0 + col] : make_float2(0.f, 0.f);
         },
         [&](int idx, float2 v) {
             const int r1 = p.fd_tx.div(idx), col = idx - r1 * tx;
@@ -45,24 +45,24 @@ __global__ void __launch_bounds__(kThreads) z_convolve_kernel(const ColPass p) {
     float2 *r = fft_lines(a, b, nl, ls, p.plan, false);
     float2 *o = (r == a) ? b : a;
     if (g.per) {  // complex kernel K[c][kz][ky][kx]
-        const size_t kcp = (size_t)g.pz * g.py * g.nkx;
+        const size_t kcp = (size_t)g.pz * g.py * g.ks;
         for (int idx = threadIdx.x; idx < np * g.pz * tx; idx += blockDim.x) {
             const int r1 = p.fd_tx.div(idx), col = idx - r1 * tx;
             const int q = r1 >= g.pz ? 1 : 0, kz = r1 - q * g.pz;
             const int kx = min(kx0 + col, g.nkx - 1), ky = q ? kyb : kya;
-            const float2 *K = reinterpret_cast<const float2 *>(p.kern) + ((size_t)kz * g.py + ky) * g.nkx + kx;
+            const float2 *K = reinterpret_cast<const float2 *>(p.kern) + ((size_t)kz * g.py + ky) * g.ks + kx;
             multiply_periodic(K, kcp, false, r + ((q * 3 + 0) * tx + col) * ls + sk(kz), r + ((q * 3 + 1) * tx + col) * ls + sk(kz),
                               r + ((q * 3 + 2) * tx + col) * ls + sk(kz));
         }
     }
-    const size_t kc = (size_t)g.nkz * g.nky * g.nkx;
+    const size_t kc = (size_t)g.nkz * g.nky * g.ks;
     for (int idx = threadIdx.x; idx < (g.per ? 0 : g.pz * tx); idx += blockDim.x) {
         const int kz = p.fd_tx.div(idx), col = idx - kz * tx;
         const int kx = min(kx0 + col, g.nkx - 1);
         int kzm;
         float sz;
         kernel_mirror(kz, g.pz, kzm, sz);
-        const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.nkx + kx;
+        const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.ks + kx;
         const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc);
         const float kxy0 = __ldg(K + 3 * kc), kxz = sz * __ldg(K + 4 * kc), kyz0 = sz * __ldg(K + 5 * kc);
         for (int q = 0; q < np; ++q) {
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kThreads) z_convolve_kernel(const ColPass p) {
         const int q = r2 / 3, c = r2 - 3 * q;
         const int ky = q ? kyb : kya;
         if (col < ncol)
-            p.out[c * cstride + z * zstride + (size_t)ky * g.nkx + kx0 + col] = qb[((q * 3 + c) * tx + col) * ls + sk(z)];
+            p.out[c * cstride + z * zstride + (size_t)ky * g.xs + kx0 + col] = qb[((q * 3 + c) * tx + col) * ls + sk(z)];
     }
 }
 
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
     int kyb;
     const int np = ky_pair(kya, g.py, kyb);
     const int nz = g.nz;
-    const size_t cstride = (size_t)nz * g.py * g.nkx;  // component stride of Y
-    const size_t zstride = (size_t)g.py * g.nkx;
+    const size_t cstride = (size_t)nz * g.py * g.xs;  // component stride of Y
+    const size_t zstride = (size_t)g.py * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;        // e^{-2 pi i e / N}
 
     // phase 1: item (r2, z2, col), col fastest
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
         const int z2 = rz % N2, r2 = rz / N2;
         const int q = r2 >= 3, c = r2 - 3 * q;
         const int ky = q ? kyb : kya;
-        const float2 *src = p.in + c * cstride + (size_t)ky * g.nkx + kx0 + col;
+        const float2 *src = p.in + c * cstride + (size_t)ky * g.xs + kx0 + col;
         float2 e[H1];
 #pragma unroll
         for (int z1 = 0; z1 < H1; ++z1) {
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
     __syncthreads();
 
     // phase 2: item (q, k1, col), col fastest; all three components of one frequency column
-    const size_t kc = (size_t)g.nkz * g.nky * g.nkx;
+    const size_t kc = (size_t)g.nkz * g.nky * g.ks;
     const int n2 = np * N1 * ncol;
     for (int it = threadIdx.x; it < n2; it += blockDim.x) {
         int qk, col;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
             int kzm;
             float sz;
             kernel_mirror(k1 + N1 * k2, N, kzm, sz);
-            const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.nkx + kx;
+            const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.ks + kx;
             const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc);
             const float kxy = sy * __ldg(K + 3 * kc), kxz = sz * __ldg(K + 4 * kc), kyz = sy * sz * __ldg(K + 5 * kc);
             const float2 mx = m[0][k2], my = m[1][k2], mz = m[2][k2];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
         const int ky = q ? kyb : kya;
         float2 e[H1];
         half_idft_load<N1, N2>(e, z2, buf + (r2 * tx + col) * ls, tw);
-        float2 *dst = p.out + c * cstride + (size_t)ky * g.nkx + kx0 + col;
+        float2 *dst = p.out + c * cstride + (size_t)ky * g.xs + kx0 + col;
 #pragma unroll
         for (int z1 = 0; z1 < H1; ++z1) {
             const int z = N2 * z1 + z2;
@@ -220,8 +220,8 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
     const int np = ky_pair(kya, g.py, kyb);
     const int kyB = np == 2 ? kyb : kya;
     const int nz = g.nz;
-    const size_t cstride = (size_t)nz * g.py * g.nkx;  // component stride of Y
-    const size_t zstride = (size_t)g.py * g.nkx;
+    const size_t cstride = (size_t)nz * g.py * g.xs;  // component stride of Y
+    const size_t zstride = (size_t)g.py * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;        // e^{-2 pi i e / N}
 
     // phase 1: item (c, z2, col), col fastest
@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
         const int col = it & (TX - 1), cz = it >> 3;
         if (col >= ncol) continue;
         const int z2 = cz % N2, c = cz / N2;
-        const float2 *srcA = p.in + c * cstride + (size_t)kya * g.nkx + kx0 + col;
-        const float2 *srcB = p.in + c * cstride + (size_t)kyB * g.nkx + kx0 + col;
+        const float2 *srcA = p.in + c * cstride + (size_t)kya * g.xs + kx0 + col;
+        const float2 *srcB = p.in + c * cstride + (size_t)kyB * g.xs + kx0 + col;
         cp2 e[H1];
 #pragma unroll
         for (int z1 = 0; z1 < H1; ++z1) {
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
     __syncthreads();
 
     // phase 2: item (k1, col); inner DFTs, the tensor multiply, inverse inner DFTs
-    const size_t kc = (size_t)g.nkz * g.nky * g.nkx;
+    const size_t kc = (size_t)g.nkz * g.nky * g.ks;
     for (int it = threadIdx.x; it < N1 * TX; it += blockDim.x) {
         const int col = it & (TX - 1), k1 = it >> 3;
         if (col >= ncol) continue;
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
             int kzm;
             float sz;
             kernel_mirror(k1 + N1 * k2, N, kzm, sz);
-            const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.nkx + kx;
+            const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.ks + kx;
             const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc);
             const float kxy = __ldg(K + 3 * kc), kxz = sz * __ldg(K + 4 * kc), kyz = sz * __ldg(K + 5 * kc);
             // H = -N M; lane B (py - ky) flips the odd-in-y components xy and yz
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
         const int z2 = cz % N2, c = cz / N2;
         cp2 e[H1];
         phalf_idft_load<N1, N2>(e, z2, buf + (c * TX + col) * ls, tw);
-        float2 *dstA = p.out + c * cstride + (size_t)kya * g.nkx + kx0 + col;
-        float2 *dstB = p.out + c * cstride + (size_t)kyb * g.nkx + kx0 + col;
+        float2 *dstA = p.out + c * cstride + (size_t)kya * g.xs + kx0 + col;
+        float2 *dstB = p.out + c * cstride + (size_t)kyb * g.xs + kx0 + col;
 #pragma unroll
         for (int z1 = 0; z1 < H1; ++z1) {
             const int z = N2 * z1 + z2;
@@ -306,38 +306,41 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
 }
 
 // pz <= 24: one thread per (kx, ky) holds the three components' z columns in registers, so
-// the pass is one read and one write of Y with no shared memory and no barrier; the (ky, kx)
-// plane is contiguous, so every access coalesces whatever nkx is.  3 nz independent loads a
-// thread keep enough bytes in flight at two to four CTAs of 128 threads per SM.
+// the pass is one read and one write of Y with no shared memory and no barrier.  3 nz
+// independent loads a thread keep enough bytes in flight at two to four CTAs of 128 threads
+// per SM.
 template <int PZ, bool PER>
 __global__ void __launch_bounds__(128, PZ <= 8 ? 4 : PZ <= 14 ? 3 : 2) z_convolve_register_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     constexpr int H = PZ / 2;
     const Grid &g = p.g;
-    const int plane = g.py * g.nkx, idx = blockIdx.x * 128 + threadIdx.x;
-    if (idx >= plane) return;
+    const int idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= g.py * g.nkx) return;
     const int ky = g.fd_nkx.div(idx), kx = idx - ky * g.nkx, nz = g.nz;
+    const size_t plane = (size_t)g.py * g.xs, at = (size_t)ky * g.xs + kx;
     float2 v[3][H];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int z = 0; z < H; ++z) v[c][z] = z < nz ? p.in[(size_t)(c * nz + z) * plane + idx] : make_float2(0.f, 0.f);
+        for (int z = 0; z < H; ++z) v[c][z] = z < nz ? p.in[(size_t)(c * nz + z) * plane + at] : make_float2(0.f, 0.f);
     if constexpr (PER) {
-        z_column_convolve<PZ, true>(v, reinterpret_cast<const float *>(reinterpret_cast<const float2 *>(p.kern) + idx),
-                                    (size_t)plane, (size_t)PZ * plane, 1.f, p.plan.tw);
+        const size_t kp = (size_t)g.py * g.ks;
+        z_column_convolve<PZ, true>(
+            v, reinterpret_cast<const float *>(reinterpret_cast<const float2 *>(p.kern) + (size_t)ky * g.ks + kx), kp,
+            PZ * kp, 1.f, p.plan.tw);
     } else {
         int kym;
         float sy;
         kernel_mirror(ky, g.py, kym, sy);
-        z_column_convolve<PZ, false>(v, p.kern + (size_t)kym * g.nkx + kx, (size_t)g.nky * g.nkx,
-                                     (size_t)g.nkz * g.nky * g.nkx, sy, p.plan.tw);
+        z_column_convolve<PZ, false>(v, p.kern + (size_t)kym * g.ks + kx, (size_t)g.nky * g.ks,
+                                     (size_t)g.nkz * g.nky * g.ks, sy, p.plan.tw);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int z = 0; z < H; ++z)
-            if (z < nz) p.out[(size_t)(c * nz + z) * plane + idx] = v[c][z];
+            if (z < nz) p.out[(size_t)(c * nz + z) * plane + at] = v[c][z];
 }
 
 }  // namespace

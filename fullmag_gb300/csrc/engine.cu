@@ -2043,6 +2043,7 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     if (g.px < 2) g.px = 2;
     g.half = g.px / 2;
     g.nkx = g.half + 1;
+    g.xs = x_pitch(g.nkx);
     g.nky = g.py / 2 + 1;
     g.nkz = g.pz / 2 + 1;
     grid_dividers(g);
@@ -2267,11 +2268,12 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
         }
     }
     const size_t vec = sizeof(float) * 3 * (size_t)g.n;
-    const size_t xlen = demag ? sizeof(float2) * 3 * (size_t)g.nz * g.ny * g.nkx : 0;
-    const size_t ylen = (demag && !thin && !use_yz) ? sizeof(float2) * 3 * (size_t)g.nz * g.py * g.nkx : 0;
+    const size_t xlen = demag ? sizeof(float2) * 3 * (size_t)g.nz * g.ny * g.xs : 0;
+    const size_t ylen = (demag && !thin && !use_yz) ? sizeof(float2) * 3 * (size_t)g.nz * g.py * g.xs : 0;
+    g.ks = g.per || use_yz ? g.nkx : g.xs;
     const size_t klen = !demag ? 0
-                        : g.per ? sizeof(float2) * (thin ? 4 : 6) * (size_t)g.pz * g.py * g.nkx
-                                : sizeof(float) * (thin ? 4 : 6) * (size_t)g.nkz * g.nky * g.nkx;
+                        : g.per ? sizeof(float2) * (thin ? 4 : 6) * (size_t)g.pz * g.py * g.ks
+                                : sizeof(float) * (thin ? 4 : 6) * (size_t)g.nkz * g.nky * g.ks;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     size_t off = 0;
     std::vector<size_t> o;
@@ -2614,14 +2616,14 @@ bool Engine::upload_spectra(const fullmag_fdm_plan_desc *plan, bool thin) {
     const int ncomp = thin ? 4 : 6;
     const double P = (double)g.px * g.py * (thin ? 1 : g.pz);
     const double scale = ms / P;
-    const size_t per = (size_t)g.nkz * g.nky * g.nkx;
+    const size_t per = (size_t)g.nkz * g.nky * g.ks;
     std::vector<float> h((size_t)ncomp * per);
     for (int c = 0; c < ncomp; ++c)
         for (int kz = 0; kz < g.nkz; ++kz)
             for (int ky = 0; ky < g.nky; ++ky)
                 for (int kx = 0; kx < g.nkx; ++kx) {
                     const size_t s = (size_t)kx + (size_t)g.px * (ky + (size_t)g.py * kz);
-                    h[(size_t)c * per + ((size_t)kz * g.nky + ky) * g.nkx + kx] = (float)(src[c][2 * s] * scale);
+                    h[(size_t)c * per + ((size_t)kz * g.nky + ky) * g.ks + kx] = (float)(src[c][2 * s] * scale);
                 }
     if (cuda_fail("cudaMemcpy(kernel)", cudaMemcpyAsync(kern, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, stream)))
         return false;

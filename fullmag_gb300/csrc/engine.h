@@ -3,7 +3,7 @@
 // Layout in HBM (one allocation per buffer class, all 256-byte aligned):
 //   vector fields : SoA float, component c of cell i at base[c*n + i],
 //                   cell i = x + nx*(y + ny*z)
-//   X spectrum    : x-transformed half spectrum, float2 X[c][z][y][kx],
+//   X spectrum    : x-transformed half spectrum, float2 X[c][z][y][kx], rows at pitch xs,
 //                   kx in [0, px/2], rows only for y < ny, z < nz (zero rows pruned)
 //   Y spectrum    : (3-D only) y-transformed, float2 Y[c][z][ky][kx], ky in [0, py)
 //   demag kernel  : with a periodic axis complex and full, pre-scaled by Ms/P:
@@ -75,12 +75,18 @@ struct Material {
     float ku1f, ku2f, kc1f, kc2f, kc3f;
 };
 
+// Rows of the spectra start on 128-byte boundaries (32-byte on short rows), so that the column
+// passes' tiles of 8 or 16 kx take whole sectors; nkx itself is odd.
+__host__ __device__ constexpr int x_pitch(int nkx) { return nkx >= 128 ? (nkx + 15) & ~15 : (nkx + 3) & ~3; }
+
 struct Grid {
     int nx, ny, nz;
     long long n;
     int px, py, pz;  // padded extents (pz == 1 on the thin-film path)
     int nkx;         // px/2 + 1
     int half;        // px/2
+    int xs;          // kx pitch of the spectra (x_pitch(nkx))
+    int ks;          // kx pitch of the demag kernel: xs for the open kernel read kx-fastest, else nkx
     int nky, nkz;    // py/2+1, pz/2+1 (kernel octant extents)
     int thin;        // 1: 2-D transform (nz == 1, pz == 1)
     int per;         // periodic axes (bit 0 x, 1 y, 2 z): wrap-around stencils, unpadded transforms

@@ -180,12 +180,13 @@ __global__ void axis_transform_kernel(const double *__restrict__ in, double *__r
 
 template <typename T>
 __global__ void to_float_kernel(const double *__restrict__ in, T *__restrict__ out, long long per, int ncomp,
-                                double scale, unsigned neg_mask) {
+                                double scale, unsigned neg_mask, int nkx, int pitch) {
     const long long total = per * ncomp;
     for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total; id += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(id / per);
         const double s = ((neg_mask >> c) & 1u) ? -scale : scale;
-        out[id] = (T)(in[id] * s);
+        const long long row = id / nkx;
+        out[row * pitch + (id - row * nkx)] = (T)(in[id] * s);
     }
 }
 
@@ -208,6 +209,7 @@ static bool newell_build(const Grid &g, double dx, double dy, double dz, double 
     const long long tl = (long long)sx * sy * sz;
     const long long n = (long long)nx * ny * nz;
     const int ncomp = g.thin ? 4 : 6;
+    const int pitch = g.ks ? g.ks : g.nkx;  // of the FP32 kernel's kx rows
     // parity bits per component (xx yy zz xy xz yz)
     const unsigned oddx = (1u << 3) | (1u << 4), oddy = (1u << 3) | (1u << 5), oddz = (1u << 4) | (1u << 5);
     const unsigned neg = (1u << 3) | (1u << 4) | (1u << 5);
@@ -245,16 +247,16 @@ static bool newell_build(const Grid &g, double dx, double dy, double dz, double 
             const long long per = (long long)g.nky * g.nkx;
             const double scale = ms / ((double)g.px * g.py);
             // components 0..3 of Bb are contiguous blocks of nz*nky*nkx = per (nz == 1)
-            if (kern64) to_float_kernel<<<grid_for(per * 4), 256, 0, s>>>(Bb, kern64, per, 4, scale, 1u << 3);
-            else to_float_kernel<<<grid_for(per * 4), 256, 0, s>>>(Bb, kern, per, 4, scale, 1u << 3);
+            if (kern64) to_float_kernel<<<grid_for(per * 4), 256, 0, s>>>(Bb, kern64, per, 4, scale, 1u << 3, g.nkx, g.nkx);
+            else to_float_kernel<<<grid_for(per * 4), 256, 0, s>>>(Bb, kern, per, 4, scale, 1u << 3, g.nkx, pitch);
         } else {
             // z: [c][k][(ky,kx)] -> [c][kz][(ky,kx)]
             axis_transform_kernel<<<grid_for(sizeC), 256, 0, s>>>(Bb, Cb, 6, 1, nz, g.nkz, g.nky * g.nkx, g.pz, dtw + off[2],
                                                                   oddz);
             const long long per = (long long)g.nkz * g.nky * g.nkx;
             const double scale = ms / ((double)g.px * g.py * g.pz);
-            if (kern64) to_float_kernel<<<grid_for(per * 6), 256, 0, s>>>(Cb, kern64, per, 6, scale, neg);
-            else to_float_kernel<<<grid_for(per * 6), 256, 0, s>>>(Cb, kern, per, 6, scale, neg);
+            if (kern64) to_float_kernel<<<grid_for(per * 6), 256, 0, s>>>(Cb, kern64, per, 6, scale, neg, g.nkx, g.nkx);
+            else to_float_kernel<<<grid_for(per * 6), 256, 0, s>>>(Cb, kern, per, 6, scale, neg, g.nkx, pitch);
         }
         ok = ck(cudaGetLastError(), "newell kernels", err) && ck(cudaStreamSynchronize(s), "newell sync", err);
     }
