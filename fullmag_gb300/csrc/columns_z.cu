@@ -198,6 +198,12 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
     }
 }
 
+__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The pruned two-level z convolution on y-frequency pairs in packed FP32x2 form: lane A
 // is ky, lane B is py - ky (the two share every twiddle and, up to the sign of the
 // odd-in-y components xy and yz, every kernel value).  Tiles of 8 kx columns; phase 1
@@ -206,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, (N1 * N2 <= 128) ? 3 : 1) z_convolve
 // buffer is the size of the unpaired kernel's.  For ky = 0 and ky = py/2 (no partner)
 // lane B repeats lane A and is not stored.
 template <int N1, int N2>
-__global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_kernel(const ColPass p) {
+__global__ void __launch_bounds__(3 * N2 * 8, N2 >= 7 ? 2 : 3) z_convolve_pair_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     constexpr int N = N1 * N2, H1 = N1 / 2, TX = 8;
@@ -224,6 +230,16 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
     const size_t zstride = (size_t)g.py * g.xs;
     const float2 *__restrict__ tw = p.plan.tw;        // e^{-2 pi i e / N}
 
+    // the tile's kernel values [6][N/2 + 1][8], in flight during phase 1 (rows are 16-byte aligned)
+    const size_t kc = (size_t)g.nkz * g.nky * g.ks;
+    constexpr int NKZ = N / 2 + 1;
+    float *kt = reinterpret_cast<float *>(buf + 3 * TX * ls);
+    for (int r = threadIdx.x; r < 2 * 6 * NKZ; r += blockDim.x) {
+        const int h = r & 1, ck = r >> 1, c = ck / NKZ, kz = ck - c * NKZ;
+        if (kx0 + 4 * h < g.ks)
+            cp_async16(kt + 4 * r, p.kern + c * kc + ((size_t)kz * g.nky + kya) * g.ks + kx0 + 4 * h);
+    }
+
     // phase 1: item (c, z2, col), col fastest
     for (int it = threadIdx.x; it < 3 * N2 * TX; it += blockDim.x) {
         const int col = it & (TX - 1), cz = it >> 3;
@@ -239,10 +255,10 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
         }
         phalf_dft_store<N1, N2>(e, z2, buf + (c * TX + col) * ls, tw);
     }
+    cp_async_wait();
     __syncthreads();
 
     // phase 2: item (k1, col); inner DFTs, the tensor multiply, inverse inner DFTs
-    const size_t kc = (size_t)g.nkz * g.nky * g.ks;
     for (int it = threadIdx.x; it < N1 * TX; it += blockDim.x) {
         const int col = it & (TX - 1), k1 = it >> 3;
         if (col >= ncol) continue;
@@ -254,15 +270,14 @@ __global__ void __launch_bounds__(3 * N2 * 8, N2 == 8 ? 2 : 3) z_convolve_pair_k
             for (int z2 = 0; z2 < N2; ++z2) m[c][z2] = pload(line[sk(k1 * N2 + z2)]);
             pdft<N2>(m[c], false);
         }
-        const int kx = kx0 + col;
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
             int kzm;
             float sz;
             kernel_mirror(k1 + N1 * k2, N, kzm, sz);
-            const float *K = p.kern + ((size_t)kzm * g.nky + kya) * g.ks + kx;
-            const float kxx = __ldg(K), kyy = __ldg(K + kc), kzz = __ldg(K + 2 * kc);
-            const float kxy = __ldg(K + 3 * kc), kxz = sz * __ldg(K + 4 * kc), kyz = sz * __ldg(K + 5 * kc);
+            const float *K = kt + kzm * TX + col;
+            const float kxx = K[0], kyy = K[NKZ * TX], kzz = K[2 * NKZ * TX];
+            const float kxy = K[3 * NKZ * TX], kxz = sz * K[4 * NKZ * TX], kyz = sz * K[5 * NKZ * TX];
             // H = -N M; lane B (py - ky) flips the odd-in-y components xy and yz
             const float2 Nxx = pb(-kxx), Nyy = pb(-kyy), Nzz = pb(-kzz), Nxz = pb(-kxz);
             const float2 Nxy = make_float2(-kxy, kxy), Nyz = make_float2(-kyz, kyz);
@@ -367,7 +382,7 @@ namespace {
 template <int N1, int N2>
 cudaError_t launch_z_pair(const ColPass &p, cudaStream_t s) {
     const void *fn = (const void *)z_convolve_pair_kernel<N1, N2>;
-    const size_t sm = sizeof(float4) * (size_t)3 * 8 * skewed_len(N1 * N2);
+    const size_t sm = sizeof(float4) * (size_t)3 * 8 * skewed_len(N1 * N2) + sizeof(float) * 6 * (N1 * N2 / 2 + 1) * 8;
     cudaError_t e = ensure_smem(fn, sm);
     if (e != cudaSuccess) return e;
     return launch_pdl(z_convolve_pair_kernel<N1, N2>, dim3(tiles(p), p.g.nky), dim3(3 * N2 * 8), sm, s, p);
