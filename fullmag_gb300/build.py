@@ -17,7 +17,7 @@ SRC = PKG / "csrc"
 OUT = PKG / "_build"
 LIB = OUT / "libfullmag_fdm.so"
 SOURCES = ["row_pass.cu", "row_pass_batched.cu", "columns.cu", "columns_z.cu", "columns_conv.cu", "columns_batched.cu", "engine.cu",
-           "newell.cu", "adjoint.cu", "noalloc.cu", "extra_field.cu", "fp64.cu"]
+           "newell.cu", "noalloc.cu", "extra_field.cu", "fp64.cu"]
 # kernels per transform length, compiled in groups (FM_GROUP) so that they build in parallel
 GROUPED = ["row_pass_lengths.cu", "columns_lengths.cu"]
 GROUPS = range(7)

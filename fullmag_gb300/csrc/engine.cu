@@ -1350,13 +1350,13 @@ struct Engine {
     // every C steps (C ~ sqrt(n)).  adjoint_backward walks the segments backwards:
     // it recomputes a segment from its checkpoint while storing every stage input
     // y0..y3, effective field H0..H3 and k1..k4, then applies the transposed step in
-    // reverse (equations in adjoint.cu): per stage one row pass computes the local VJP
+    // reverse (equations in row_pass.cuh): per stage one row pass computes the local VJP
     // and forward-transforms lambda_H, the column passes convolve it, and a second row
     // pass adds H_lin(lambda_H) and pushes the result through the stage normalisation.
     // d loss / d field map accumulates in float-float.
     float *adj_ckpt = nullptr;  // [n_ckpt][3n]
     float *adj_seg = nullptr;   // [C][12][3n]: y0 y1 y2 y3 H0 H1 H2 H3 k1 k2 k3 k4
-    float *adj_work = nullptr;  // [12][3n]: lam_next lam_y0 lk1 lk2 lk3 lk4 lam_h[0] lam_m lam_h[1] g_hi g_lo spare
+    float *adj_work = nullptr;  // [10][3n]: lam_y0 lk1 lk2 lk3 lam_h[0] lam_m lam_h[1] g_hi g_lo spare
     uint64_t adj_nsteps = 0;
     uint32_t adj_C = 0;
     size_t adj_nck = 0;
@@ -1470,17 +1470,17 @@ struct Engine {
         const long long n = g.n;
         if (!adj_seg && cuda_fail("cudaMalloc(adjoint segment)", cudaMalloc((void **)&adj_seg, sizeof(float) * v3 * 12 * adj_C)))
             return FULLMAG_FDM_ERR_CUDA;
-        if (!adj_work && cuda_fail("cudaMalloc(adjoint work)", cudaMalloc((void **)&adj_work, sizeof(float) * v3 * 12)))
+        if (!adj_work && cuda_fail("cudaMalloc(adjoint work)", cudaMalloc((void **)&adj_work, sizeof(float) * v3 * 10)))
             return FULLMAG_FDM_ERR_CUDA;
-        float *W[12];
-        for (int i = 0; i < 12; ++i) W[i] = adj_work + i * v3;
-        float *lam_next = W[0], *lam_y0 = W[1], *lk[5] = {nullptr, W[2], W[3], W[4], W[5]};
-        float *lam_hb[2] = {W[6], W[8]}, *lam_m = W[7], *g_hi = W[9], *g_lo = W[10], *spare = W[11];
+        float *W[10];
+        for (int i = 0; i < 10; ++i) W[i] = adj_work + i * v3;
+        float *lam_y0 = W[0], *lk[4] = {nullptr, W[1], W[2], W[3]};
+        float *lam_hb[2] = {W[4], W[6]}, *lam_m = W[5], *g_hi = W[7], *g_lo = W[8], *spare = W[9];
         if (!ensure_staging()) return FULLMAG_FDM_ERR_CUDA;
         if (cuda_fail("cudaMemcpy(lambda)", cudaMemcpyAsync(staging, lam_T, sizeof(double) * v3, cudaMemcpyHostToDevice, stream)))
             return FULLMAG_FDM_ERR_CUDA;
         aos_to_soa_kernel<<<std::min<long long>((n + 255) / 256, 4096), 256, 0, stream>>>((const double *)staging, nullptr,
-                                                                                          lam_next, mask, n);
+                                                                                          lam_y0, mask, n);
         if (cuda_fail("zero", cudaMemsetAsync(g_hi, 0, sizeof(float) * v3 * 2, stream))) return FULLMAG_FDM_ERR_CUDA;
         const double h = adj_h;
         const float hf = (float)h;
@@ -1498,16 +1498,16 @@ struct Engine {
                 for (int f = 0; f < 12; ++f) out[f] = slot(t, f);
                 ok = adj_step(slot(t, 0), out, t + 1 < len ? slot(t + 1, 0) : spare, h);
             }
-            for (long long t = (long long)len - 1; t >= 0 && ok; --t) {
-                AdjFinal af{n, lam_next, slot(t, 0), slot(t, 8), slot(t, 9), slot(t, 10), slot(t, 11), hf,
-                            lam_y0, lk[1], lk[2], lk[3], lk[4]};
-                ok = !cuda_fail("adjoint final", launch_adj_final(af, stream));
-                // Five row passes per step, like a forward step: the local VJP of stage s - 1
-                // (bit 1) shares a pass with the stage-s update after H_lin (bit 2), because the
-                // cotangent of k_s it needs is complete at each cell once bit 2 has run there.
-                // lambda_H alternates between two buffers (the stencil reads its neighbours).
-                int lh = 0;
-                for (int s = 4; s >= 0 && ok; --s) {
+            // Four row passes per step, as in a forward step.  The local VJP of stage s - 1
+            // (bit 1) shares a pass with the stage-s update after H_lin (bit 2), because the
+            // cotangent of k_s it needs is complete at each cell once bit 2 has run there; the
+            // last normalisation of a step (bit 4) likewise sits between the stage-0 update of
+            // the step after it and the VJP of its own stage 3.  Only where a segment begins
+            // does the stage-0 update run alone, before the recomputation overwrites X.
+            // lambda_H alternates between two buffers (the stencil reads its neighbours).
+            int lh = 0;
+            for (long long t = (long long)len - 1; t >= -1 && ok; --t) {
+                for (int s = 4; s >= (t < 0 ? 4 : 1) && ok; --s) {
                     RowPass b = row_base();
                     b.mat.has_ext = 0;
                     b.mat.has_uni = 0;
@@ -1515,41 +1515,56 @@ struct Engine {
                     b.hmap = nullptr;
                     b.adj_uni = mat.has_uni;
                     b.adj_mode = 0;
-                    if (s <= 3) {  // bit 2: update of stage s from H_lin(lambda_H of stage s)
+                    b.adj_lam_m = lam_m;
+                    b.adj_lam_y0 = lam_y0;
+                    // bit 2: update of stage s of step t (stage 0 of step t + 1 for s = 4) from H_lin
+                    // of its lambda_H
+                    const long long tu = s == 4 ? t + 1 : t;
+                    const int su = s == 4 ? 0 : s;
+                    if (tu < (long long)len) {
                         b.adj_mode |= 2;
                         b.x_in = X;
                         b.m_in = lam_hb[lh];
-                        b.adj_lam_m = lam_m;
-                        b.adj_y0 = slot(t, 0);
-                        b.adj_k = s >= 1 ? slot(t, 8 + s - 1) : nullptr;
-                        b.adj_ch = cs[s] * hf;
-                        b.adj_lam_y0 = lam_y0;
-                        b.adj_lam_k = s >= 1 ? lk[s] : nullptr;
+                        b.adj_y0 = slot(tu, 0);
+                        b.adj_k = su >= 1 ? slot(tu, 8 + su - 1) : nullptr;
+                        b.adj_ch = cs[su] * hf;
+                        b.adj_lam_k = su >= 1 ? lk[su] : nullptr;
                     }
-                    if (s >= 1) {  // bit 1: local VJP of stage s - 1, forward x-transform of its lambda_H
+                    if (t >= 0) {
+                        if (s == 4) {  // bit 4: the last normalisation of step t
+                            b.adj_mode |= 4;
+                            b.adj_fy0 = slot(t, 0);
+                            b.adj_fk1 = slot(t, 8);
+                            b.adj_fk2 = slot(t, 9);
+                            b.adj_fk3 = slot(t, 10);
+                            b.adj_fk4 = slot(t, 11);
+                            b.adj_h6 = hf / 6.0f;
+                            b.adj_lk1 = lk[1];
+                            b.adj_lk2 = lk[2];
+                            b.adj_lk3 = lk[3];
+                        }
+                        // bit 1: local VJP of stage s - 1, forward x-transform of its lambda_H
                         b.adj_mode |= 1;
                         b.adj_m = slot(t, s - 1);
                         b.adj_H = slot(t, 4 + s - 1);
-                        b.adj_w = lk[s];
+                        b.adj_w = s < 4 ? lk[s] : nullptr;
                         b.adj_lam_h = lam_hb[1 - lh];
-                        b.adj_lam_m = lam_m;
                         b.adj_g_hi = g_hi;
                         b.adj_g_lo = g_lo;
                         b.x_out = X;
                     }
-                    ok = run_row_adj(b) && (s == 0 || run_columns());
+                    ok = run_row_adj(b) && (t < 0 || run_columns());
                     lh = 1 - lh;
                 }
-                std::swap(lam_next, lam_y0);
             }
         }
         if (!ok) return FULLMAG_FDM_ERR_CUDA;
-        // gradient: g_hi + g_lo (per A/m of the map), lambda_0 = lam_next
+        // gradient: g_hi + g_lo (per A/m of the map), lambda_0 = lam_y0
         std::vector<float> hi(v3), lo(v3), l0(v3);
         if (cuda_fail("cudaMemcpy(grad)", cudaMemcpyAsync(hi.data(), g_hi, sizeof(float) * v3, cudaMemcpyDeviceToHost, stream)) ||
             cuda_fail("cudaMemcpy(grad)", cudaMemcpyAsync(lo.data(), g_lo, sizeof(float) * v3, cudaMemcpyDeviceToHost, stream)) ||
             cuda_fail("cudaMemcpy(lambda0)",
-                      cudaMemcpyAsync(l0.data(), lam_next, sizeof(float) * v3, cudaMemcpyDeviceToHost, stream)) ||
+                      cudaMemcpyAsync(l0.data(), lam_y0, sizeof(float) * v3, cudaMemcpyDeviceToHost, stream)) ||
             cuda_fail("adjoint sync", cudaStreamSynchronize(stream)))
             return FULLMAG_FDM_ERR_CUDA;
         for (long long i = 0; i < n; ++i)

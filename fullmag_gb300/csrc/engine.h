@@ -150,11 +150,14 @@ struct RowPass {
     float *h_ex_out, *h_d_out, *h_eff_out;  // NULL: not written
     int rows;                // rows per CTA
     int early;               // let the next kernel launch early (pdl_trigger)
-    // adjoint passes (launch_row_pass_adj only; see adjoint.cu for the equations); adj_mode
-    // is a bit set, bit 2 runs before bit 1 at each cell:
+    // adjoint passes (launch_row_pass_adj only; equations in row_pass.cuh); adj_mode
+    // is a bit set, bit 2 runs before bit 4 and bit 4 before bit 1 at each cell:
     //   bit 2, after H_lin(lambda_H) (m_in = lambda_H, local terms off): lambda_y = adj_lam_m
     //          + H_lin; through y_s = N(y0 + ch k) into adj_lam_y0 and adj_lam_k (adj_k NULL:
     //          stage 0, lambda_y added to adj_lam_y0)
+    //   bit 4, after bit 2 (or alone): the last normalisation of the step before,
+    //          m' = N(adj_fy0 + h/6 (k1 + 2 k2 + 2 k3 + k4)), with the cotangent in adj_lam_y0: into
+    //          adj_lam_y0 and adj_lk1..3; the cotangent of k4 is the w of bit 1
     //   bit 1, local VJP of k = f(m, H) with cotangent w (adj_uni: uniaxial Jacobian term):
     //          lambda_H -> adj_lam_h and the forward x-transform, lambda_m -> adj_lam_m
     //          (in place after bit 2 read it), lambda_H added to (adj_g_hi, adj_g_lo)
@@ -165,6 +168,9 @@ struct RowPass {
     const float *adj_y0, *adj_k;
     float adj_ch;
     float *adj_lam_y0, *adj_lam_k;
+    const float *adj_fy0, *adj_fk1, *adj_fk2, *adj_fk3, *adj_fk4;
+    float adj_h6;            // h / 6
+    float *adj_lk1, *adj_lk2, *adj_lk3;
 };
 
 struct ColPass {
@@ -279,16 +285,6 @@ int extra_field_blocks(const Grid &g);
 cudaError_t launch_extra_field(const ExtraField &p, cudaStream_t s);
 // sums the per-CTA partials into out[0..4] (fixed order)
 cudaError_t launch_extra_finalize(const ExtraSums *partials, int nblocks, double *out, cudaStream_t s, int early = 0);
-
-// Adjoint (reverse-mode RK4): the final-combination pass (adjoint.cu); all fields SoA.
-// The local VJP and the stage update are the row pass's adjoint modes.
-struct AdjFinal {
-    long long n;
-    const float *lam_next, *y0, *k1, *k2, *k3, *k4;
-    float h;
-    float *lam_y0, *lk1, *lk2, *lk3, *lk4;
-};
-cudaError_t launch_adj_final(const AdjFinal &a, cudaStream_t s);
 
 // Batched launches: one grid covering many problems through a (problem, block) table.
 struct FinDesc {

@@ -60,8 +60,7 @@ cudaError_t launch_row_pass_adj(const RowPass &p, cudaStream_t s) {
     const RowKernel fn = row_kernels_for(row_pass_length(p.g, p.x_in || p.x_out)).adj;
     cudaError_t e = ensure_smem((const void *)fn, sm);
     if (e != cudaSuccess) return e;
-    fn<<<row_pass_blocks(p), kThreads, sm, s>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(fn, dim3(row_pass_blocks(p)), dim3(kThreads), sm, s, p);
 }
 
 }  // namespace fm

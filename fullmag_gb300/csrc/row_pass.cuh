@@ -230,7 +230,19 @@ __device__ __forceinline__ void row_forward_x_select(const RowPass &p, int rows,
 #undef FM_CASE
 }
 
-// Adjoint helpers (the element-wise equations of adjoint.cu, inlined into the row pass)
+// ---- the reverse-mode (adjoint) RK4 step, compiled into the ADJ instances ----
+// Forward step (the fixed-step RK4 of crates/fullmag-engine/src/fdm_integrators.rs:155-262
+// with the per-stage normalisation N(v) = v/|v|):
+//   k1 = f(y0), y1 = N(y0 + h/2 k1), k2 = f(y1), y2 = N(y0 + h/2 k2), k3 = f(y2),
+//   y3 = N(y0 + h k3), k4 = f(y3), m' = N(y0 + h/6 (k1 + 2k2 + 2k3 + k4)),
+//   f(m) = -gbar [p + alpha m x p], p = m x H, H = H_lin(m) + H_anis(m) + H_map + H_ext.
+// Reverse mode, given the cotangent w of k = f(m) at (m, H):
+//   q = prec w + alpha (w x m)
+//   lambda_m  = -gbar [H x q + alpha p x w] + (dH_anis/dm)^T lambda_H + H_lin(lambda_H)
+//   lambda_H  = -gbar (q x m)          (also the gradient with respect to the field map)
+// and through a normalisation u = N(v):  lambda_v = (lambda_u - (u . lambda_u) u) / |v|.
+// H_lin (exchange stencil + Newell convolution) is symmetric, so its transpose is
+// applied by the forward field passes themselves.
 struct A3 {
     float x, y, z;
 };
@@ -777,7 +789,32 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
         if (adj_local) {
             if constexpr (ADJ) {
                 // local VJP of k = -gbar [prec m x H + alpha m x (m x H)] with cotangent w
-                const A3 m = a3_ld(p.adj_m, n, i), H = a3_ld(p.adj_H, n, i), w = a3_ld(p.adj_w, n, i);
+                const A3 m = a3_ld(p.adj_m, n, i), H = a3_ld(p.adj_H, n, i);
+                A3 w;
+                if (p.adj_mode & 4) {
+                    // through m' = N(v) of the step that ends here
+                    const A3 k1 = a3_ld(p.adj_fk1, n, i), k2 = a3_ld(p.adj_fk2, n, i), k3 = a3_ld(p.adj_fk3, n, i),
+                             k4 = a3_ld(p.adj_fk4, n, i);
+                    const A3 s = {k1.x + 2.f * k2.x + 2.f * k3.x + k4.x, k1.y + 2.f * k2.y + 2.f * k3.y + k4.y,
+                                  k1.z + 2.f * k2.z + 2.f * k3.z + k4.z};
+                    const A3 v = a3_axpy(p.adj_h6, s, a3_ld(p.adj_fy0, n, i)), lam = a3_ld(p.adj_lam_y0, n, i);
+                    const float nn = sqrtf(a3_dot(v, v));
+                    A3 mu{0.f, 0.f, 0.f};
+                    if (nn > 0.f) {
+                        const float inv = 1.0f / nn;
+                        const A3 u{v.x * inv, v.y * inv, v.z * inv};
+                        const A3 t = a3_axpy(-a3_dot(u, lam), u, lam);
+                        mu = {t.x * inv, t.y * inv, t.z * inv};
+                    }
+                    a3_st(p.adj_lam_y0, n, i, mu);
+                    w = {p.adj_h6 * mu.x, p.adj_h6 * mu.y, p.adj_h6 * mu.z};
+                    const A3 w2{2.f * p.adj_h6 * mu.x, 2.f * p.adj_h6 * mu.y, 2.f * p.adj_h6 * mu.z};
+                    a3_st(p.adj_lk1, n, i, w);
+                    a3_st(p.adj_lk2, n, i, w2);
+                    a3_st(p.adj_lk3, n, i, w2);
+                } else {
+                    w = a3_ld(p.adj_w, n, i);
+                }
                 const A3 q = a3_axpy(M.alpha, a3_cross(w, m), A3{M.prec * w.x, M.prec * w.y, M.prec * w.z});
                 const A3 pv = a3_cross(m, H);
                 const A3 t = a3_axpy(M.alpha, a3_cross(pv, w), a3_cross(H, q));
@@ -955,6 +992,8 @@ __global__ void __launch_bounds__(kThreads, row_ctas(HALF)) row_pass_kernel(cons
 
 template <int HALF>
 __global__ void __launch_bounds__(kThreads) row_pass_adj_kernel(const RowPass p) {
+    pdl_wait();
+    if (p.early) pdl_trigger();
     row_pass_body<HALF, false, true, false>(p, blockIdx.x, gridDim.x);
 }
 
