@@ -1606,7 +1606,8 @@ struct Engine {
     // Tiles for batched rounds.  The autotuner picks tiles that make one small grid fill
     // the GPU (many thin CTAs); in a batched round the problems fill the GPU together, so
     // each CTA takes more work instead: row passes of at least ~512 cells, and the widest
-    // kx tile of the fused column pass within 64 KB of shared memory.
+    // kx tile of the fused column pass within 96 KB of shared memory (24 films, a block of
+    // 64 rounds: 24.0 ms, 64 KB 24.7, 32 KB 28.6; row passes of 256 cells 26.3).
     void batch_tiling() {
         const int nrows = g.ny * g.nz;
         int r = 1;
@@ -1625,7 +1626,7 @@ struct Engine {
         if (!demag) return;
         int tx = 1;
         auto smem = [&](int t) { return g.thin ? y_convolve_2d_smem(g, t) : yz_convolve_smem(g, t); };
-        while (tx < 16 && 2 * tx <= g.nkx && smem(2 * tx) <= 64u * 1024u) tx *= 2;
+        while (tx < 16 && 2 * tx <= g.nkx && smem(2 * tx) <= 96u * 1024u) tx *= 2;
         if (g.thin) tx_2d = std::max(tx_2d, tx);
         else if (use_yz) tx_z = std::max(tx_z, tx);
     }
@@ -3354,9 +3355,8 @@ struct FdmBatch {
     std::vector<double> next_dt;  // per problem: suggested step (DP45) or 0 before the first step
     std::string last_error;
     cudaStream_t bstream = nullptr;
-    // Branches of a captured round: the buckets of one pass (row buckets, column groups)
-    // are independent launches, captured as parallel graph branches so that a bucket of
-    // a few dozen CTAs runs beside the large ones instead of after them.
+    // Branches of a captured round: the chains (build_round).
+    static constexpr int kChains = 8;
     static constexpr int kSide = 8;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[kSide] = {};
@@ -3452,9 +3452,59 @@ struct FdmBatch {
         // the old round's pending commits and step control go back to the engines first
         if (!sync_states(err)) return false;
         if (bstream) cudaStreamSynchronize(bstream);
+        // The problems do not depend on one another, so the round is a set of chains, each the
+        // commits, passes, statistics and step control of the problems that share a row-pass class
+        // and a column kernel; a chain's row pass runs beside another's column pass.  With fewer
+        // than kChains kinds the largest chains are cut.  Joining all kernels between phases left
+        // the GPU waiting for the slowest bucket thirteen times a round (24 films, 64 rounds: 35.7
+        // ms against 24.7 at 8 chains, 25.3 at 6, 26.0 at 12, 28.0 at one chain per film).
         const int n = (int)act.size();
-        if (round.members != act) round.release();
-        round.members = act;
+        struct Chain {
+            int cls = 0, kind = -1, first = 0;
+            long long max_n3 = 0;
+            size_t row_smem = 0, col_smem = 0, row_work_at = 0, cols_at = 0, col_work_at = 0;
+            std::vector<size_t> ids;
+            std::vector<int2> row_work, col_work;
+            std::vector<ColPass> cols;
+        };
+        std::vector<Chain> chains;
+        {
+            std::map<std::pair<int, int>, Chain> by_kind;
+            for (size_t i : act) {
+                Engine *e = items[i];
+                const int cls = row_pass_class(e->g, e->demag), kind = e->demag ? col_batched_kind(e->g) : -1;
+                Chain &c = by_kind[{cls, kind}];
+                c.cls = cls;
+                c.kind = kind;
+                c.ids.push_back(i);
+            }
+            for (auto &c : by_kind) chains.push_back(std::move(c.second));
+            auto cells = [&](const Chain &c) {
+                long long t = 0;
+                for (size_t i : c.ids) t += items[i]->g.n;
+                return c.ids.size() > 1 ? t : 0;
+            };
+            while ((int)chains.size() < kChains) {
+                auto big = std::max_element(chains.begin(), chains.end(),
+                                            [&](const Chain &a, const Chain &b) { return cells(a) < cells(b); });
+                if (cells(*big) == 0) break;
+                std::stable_sort(big->ids.begin(), big->ids.end(), [&](size_t a, size_t b) { return items[a]->g.n > items[b]->g.n; });
+                Chain half;
+                half.cls = big->cls;
+                half.kind = big->kind;
+                std::vector<size_t> keep;
+                for (size_t q = 0; q < big->ids.size(); ++q) (q & 1 ? half.ids : keep).push_back(big->ids[q]);
+                big->ids = std::move(keep);
+                chains.push_back(std::move(half));
+            }
+        }
+        std::vector<size_t> order;  // members, chain by chain
+        for (Chain &c : chains) {
+            c.first = (int)order.size();
+            order.insert(order.end(), c.ids.begin(), c.ids.end());
+        }
+        if (round.members != order) round.release();
+        round.members = order;
         if (!round.h_ctl && (cudaMallocHost((void **)&round.h_ctl, sizeof(BatchCtl) * n) != cudaSuccess ||
             cudaMallocHost((void **)&round.h_stats, sizeof(double) * kNumStats * n) != cudaSuccess ||
             cudaMallocHost((void **)&round.h_state, sizeof(BatchState) * n) != cudaSuccess ||
@@ -3464,37 +3514,18 @@ struct FdmBatch {
             err = "batch round allocation failed";
             return false;
         }
-        // Work is bucketed by kernel (class of the row pass, kind of the column pass) and by
-        // shared-memory class, so one large member does not set the occupancy of every CTA.
-        auto smem_class = [](size_t b) {
-            return b <= 24u * 1024u ? 0 : b <= 48u * 1024u ? 1 : b <= 96u * 1024u ? 2 : b <= 150u * 1024u ? 3 : 4;
-        };
-        constexpr int NC = 8;
-        struct RowBucket {
-            int cls = 0;
-            size_t smem = 0, offset = 0;
-            std::vector<int2> work;
-        };
-        struct ColBucket {
-            int kind = 0;
-            size_t smem = 0, offset = 0, work_offset = 0;
-            std::vector<ColPass> passes;
-            std::vector<int2> work;
-        };
         std::vector<RowPass> rows[7];
-        std::map<int, RowBucket> row_buckets;  // x class, smem class
-        std::map<int, ColBucket> col_buckets;  // kind, smem class
         std::vector<FinDesc> fin(n);
         std::vector<CommitDesc> com(n);
         std::vector<RowPass> rec;
         std::vector<int> kinds;
-        for (int k = 0; k < n; ++k) {
-            Engine *e = items[act[k]];
+        for (Chain &ch : chains) for (int k = ch.first; k < ch.first + (int)ch.ids.size(); ++k) {
+            Engine *e = items[order[k]];
             BatchState &st = round.h_state[k];
             memset(&st, 0, sizeof(st));
             st.time = e->time;
             st.t_end = t_end;
-            st.next_dt = next_dt[act[k]];
+            st.next_dt = next_dt[order[k]];
             st.max_error = e->max_error;
             st.dt_min = e->dt_min;
             st.dt_max = e->dt_max;
@@ -3503,7 +3534,7 @@ struct FdmBatch {
             st.done = e->time >= t_end * (1.0 - 1e-12);
             round.h_ctl[k] = BatchCtl{st.done ? 0.0 : std::min(st.next_dt, t_end - e->time), 0, 0};
             if (!e->record_attempt(&round.d_ctl[k].dt, rec, kinds)) {
-                err = "problem " + std::to_string(act[k]) + ": " + (e->last_error.empty() ? "not batchable" : e->last_error);
+                err = "problem " + std::to_string(order[k]) + ": " + (e->last_error.empty() ? "not batchable" : e->last_error);
                 return false;
             }
             size_t rs = 0;
@@ -3511,25 +3542,20 @@ struct FdmBatch {
                 rows[s].push_back(rec[s]);
                 rs = std::max(rs, row_pass_smem(rec[s]));
             }
-            const int cls = row_pass_class(e->g, e->demag);
-            RowBucket &rb = row_buckets[cls * NC + smem_class(rs)];
-            rb.cls = cls;
-            rb.smem = std::max(rb.smem, rs);
+            ch.row_smem = std::max(ch.row_smem, rs);
             const int nb = row_pass_blocks(rec[0]);
-            for (int b = 0; b < nb; ++b) rb.work.push_back(make_int2(k, b));
+            for (int b = 0; b < nb; ++b) ch.row_work.push_back(make_int2(k, b));
             if (e->demag) {
                 const bool thin = e->g.thin != 0;
                 const int tx = thin ? e->tx_2d : e->tx_z;
-                const size_t cs = thin ? y_convolve_2d_smem(e->g, tx) : yz_convolve_smem(e->g, tx);
-                ColBucket &cb = col_buckets[kinds[0] * NC + smem_class(cs)];
-                cb.kind = kinds[0];
-                cb.smem = std::max(cb.smem, cs);
+                ch.col_smem = std::max(ch.col_smem, thin ? y_convolve_2d_smem(e->g, tx) : yz_convolve_smem(e->g, tx));
                 ColPass c = e->col_pass(e->plan_y, tx, e->X, e->X);
                 c.skip_dt = &round.d_ctl[k].dt;
                 const int ntiles = (e->g.nkx + tx - 1) / tx;
-                for (int t = 0; t < ntiles; ++t) cb.work.push_back(make_int2((int)cb.passes.size(), t));
-                cb.passes.push_back(c);
+                for (int t = 0; t < ntiles; ++t) ch.col_work.push_back(make_int2((int)ch.cols.size(), t));
+                ch.cols.push_back(c);
             }
+            ch.max_n3 = std::max(ch.max_n3, 3 * e->g.n);
             fin[k] = FinDesc{e->partials, nb, 0};
             com[k] = CommitDesc{e->S[0], e->S[1], e->K[0], e->K[6], 3 * e->g.n};
         }
@@ -3543,19 +3569,19 @@ struct FdmBatch {
         };
         size_t o_rows[7], o_fin, o_com;
         for (int s = 0; s < 7; ++s) o_rows[s] = place(sizeof(RowPass) * rows[s].size());
-        for (auto &b : row_buckets) b.second.offset = place(sizeof(int2) * b.second.work.size());
-        for (auto &b : col_buckets) {
-            b.second.offset = place(sizeof(ColPass) * b.second.passes.size());
-            b.second.work_offset = place(sizeof(int2) * b.second.work.size());
+        for (Chain &c : chains) {
+            c.row_work_at = place(sizeof(int2) * c.row_work.size());
+            c.cols_at = place(sizeof(ColPass) * c.cols.size());
+            c.col_work_at = place(sizeof(int2) * c.col_work.size());
         }
         o_fin = off; off += al(sizeof(FinDesc) * n);
         o_com = off; off += al(sizeof(CommitDesc) * n);
         std::vector<char> hb(off);
         for (int s = 0; s < 7; ++s) memcpy(hb.data() + o_rows[s], rows[s].data(), sizeof(RowPass) * rows[s].size());
-        for (auto &b : row_buckets) memcpy(hb.data() + b.second.offset, b.second.work.data(), sizeof(int2) * b.second.work.size());
-        for (auto &b : col_buckets) {
-            memcpy(hb.data() + b.second.offset, b.second.passes.data(), sizeof(ColPass) * b.second.passes.size());
-            memcpy(hb.data() + b.second.work_offset, b.second.work.data(), sizeof(int2) * b.second.work.size());
+        for (const Chain &c : chains) {
+            memcpy(hb.data() + c.row_work_at, c.row_work.data(), sizeof(int2) * c.row_work.size());
+            memcpy(hb.data() + c.cols_at, c.cols.data(), sizeof(ColPass) * c.cols.size());
+            memcpy(hb.data() + c.col_work_at, c.col_work.data(), sizeof(int2) * c.col_work.size());
         }
         memcpy(hb.data() + o_fin, fin.data(), sizeof(FinDesc) * n);
         memcpy(hb.data() + o_com, com.data(), sizeof(CommitDesc) * n);
@@ -3582,60 +3608,51 @@ struct FdmBatch {
         }
         if (same) return true;
         round.d_com = (const CommitDesc *)(blob + o_com);
-        // capture the round
-        long long max_n3 = 0;
-        for (auto &c : com) max_n3 = std::max(max_n3, c.n3);
-        // set the shared-memory limits outside the capture
-        std::vector<const RowBucket *> row_ids;
-        std::vector<const ColBucket *> col_ids;
-        for (auto &b : row_buckets) {
-            row_ids.push_back(&b.second);
-            for (bool lean : {false, true})
-                launch_row_pass_batched(nullptr, nullptr, 0, b.second.cls, lean, b.second.smem, bstream);
+        round.max_n3 = 0;
+        for (const Chain &c : chains) {
+            round.max_n3 = std::max(round.max_n3, c.max_n3);
+            // set the shared-memory limits outside the capture
+            for (bool lean : {false, true}) launch_row_pass_batched(nullptr, nullptr, 0, c.cls, lean, c.row_smem, bstream);
+            if (c.kind >= 0) launch_col_batched(nullptr, nullptr, 0, c.kind, c.col_smem, bstream);
         }
-        for (auto &b : col_buckets) {
-            col_ids.push_back(&b.second);
-            launch_col_batched(nullptr, nullptr, 0, b.second.kind, b.second.smem, bstream);
-        }
-        // the largest launches first, so that the small ones run beside them
-        std::stable_sort(row_ids.begin(), row_ids.end(), [](auto *a, auto *b) { return a->work.size() > b->work.size(); });
-        std::stable_sort(col_ids.begin(), col_ids.end(), [](auto *a, auto *b) { return a->work.size() > b->work.size(); });
         cudaGetLastError();
         if (!ensure_branches()) {
             err = "batch stream or event creation failed";
             return false;
         }
+        // capture the round: each chain on a branch of its own
         cudaGraph_t graph = nullptr;
         if (cudaStreamBeginCapture(bstream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             err = "batch capture failed";
             return false;
         }
-        // one round: the previous round's commits, the seven passes of an attempt for every
-        // member, the statistics, and the device step control
-        bool ok = true;
-        round.max_n3 = max_n3;
-        {
-            const unsigned gx = (unsigned)std::min<long long>((max_n3 + 255) / 256, 64);
-            batch_commit_all_kernel<<<dim3(gx, n), 256, 0, bstream>>>((const CommitDesc *)(blob + o_com), round.d_ctl);
-            ok = cudaGetLastError() == cudaSuccess;
-            for (int s = 0; s < 7 && ok; ++s) {
+        std::vector<int> ids(chains.size());
+        for (size_t q = 0; q < ids.size(); ++q) ids[q] = (int)q;
+        const bool ok = fan_out(ids, [&](int q, cudaStream_t st) {
+            const Chain &c = chains[q];
+            const int m = (int)c.ids.size();
+            // the previous round's commits, the seven passes of an attempt, the statistics, and
+            // the device step control
+            const unsigned gx = (unsigned)std::min<long long>((c.max_n3 + 255) / 256, 64);
+            batch_commit_all_kernel<<<dim3(gx, m), 256, 0, st>>>((const CommitDesc *)(blob + o_com) + c.first,
+                                                                 round.d_ctl + c.first);
+            cudaError_t e = cudaGetLastError();
+            for (int s = 0; s < 7 && e == cudaSuccess; ++s) {
                 // passes 1 to 5 are intermediate stages (0 has no right-hand side, 6 the statistics)
-                ok = fan_out(row_ids, [&](const RowBucket *rb, cudaStream_t st) {
-                    return launch_row_pass_batched((const RowPass *)(blob + o_rows[s]), (const int2 *)(blob + rb->offset),
-                                                   (int)rb->work.size(), rb->cls, s > 0 && s < 6, rb->smem, st);
-                });
-                if (ok && s < 6)
-                    ok = fan_out(col_ids, [&](const ColBucket *cb, cudaStream_t st) {
-                        return launch_col_batched((const ColPass *)(blob + cb->offset), (const int2 *)(blob + cb->work_offset),
-                                                  (int)cb->work.size(), cb->kind, cb->smem, st);
-                    });
+                e = launch_row_pass_batched((const RowPass *)(blob + o_rows[s]), (const int2 *)(blob + c.row_work_at),
+                                            (int)c.row_work.size(), c.cls, s > 0 && s < 6, c.row_smem, st);
+                if (e == cudaSuccess && s < 6 && c.kind >= 0)
+                    e = launch_col_batched((const ColPass *)(blob + c.cols_at), (const int2 *)(blob + c.col_work_at),
+                                           (int)c.col_work.size(), c.kind, c.col_smem, st);
             }
-            if (ok) ok = launch_finalize_batched((const FinDesc *)(blob + o_fin), n, round.d_stats, bstream) == cudaSuccess;
-            if (ok) {
-                batch_control_kernel<<<(n + 127) / 128, 128, 0, bstream>>>(round.d_ctl, round.d_state, round.d_stats, n);
-                ok = cudaGetLastError() == cudaSuccess;
-            }
-        }
+            if (e == cudaSuccess)
+                e = launch_finalize_batched((const FinDesc *)(blob + o_fin) + c.first, m,
+                                            round.d_stats + (size_t)c.first * kNumStats, st);
+            if (e != cudaSuccess) return e;
+            batch_control_kernel<<<(m + 127) / 128, 128, 0, st>>>(round.d_ctl + c.first, round.d_state + c.first,
+                                                                  round.d_stats + (size_t)c.first * kNumStats, m);
+            return cudaGetLastError();
+        });
         const cudaError_t ce = cudaStreamEndCapture(bstream, &graph);
         if (!ok || ce != cudaSuccess || !graph) {
             if (graph) cudaGraphDestroy(graph);
