@@ -263,7 +263,9 @@ cudaError_t launch_y_fused(const ColPass &p, cudaStream_t s) {
     const auto fn = INV ? y_inverse_fused_kernel<N1, N2, FULL> : y_forward_fused_kernel<N1, N2, FULL>;
     cudaError_t e = ensure_smem((const void *)fn, sm);
     if (e != cudaSuccess) return e;
-    return launch_pdl(fn, dim3(tiles(p), p.g.nz, 3), dim3(y_threads(N1)), sm, s, p);
+    // a narrower tile takes a smaller CTA (at least 64 threads), so more of them overlap on an SM
+    const int threads = p.tx < 16 ? std::max(64, y_threads(N1) * p.tx / 16) : y_threads(N1);
+    return launch_pdl(fn, dim3(tiles(p), p.g.nz, 3), dim3(threads), sm, s, p);
 }
 // Radix split N = N1 x N2 of the two-level passes: split 0 is the default, split 1 the
 // alternative the autotuner times against it (open powers of two up to 256).
