@@ -768,12 +768,16 @@ struct Engine {
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         bool ok = fn();  // warm-up (also sets shared-memory attributes)
-        cudaEventRecord(e0, stream);
-        for (int r = 0; r < 3 && ok; ++r) ok = fn();
-        cudaEventRecord(e1, stream);
-        cudaEventSynchronize(e1);
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
+        for (int reps : {3, 9}) {  // launches of a few microseconds are timed again, longer
+            cudaEventRecord(e0, stream);
+            for (int r = 0; r < reps && ok; ++r) ok = fn();
+            cudaEventRecord(e1, stream);
+            cudaEventSynchronize(e1);
+            cudaEventElapsedTime(&ms, e0, e1);
+            ms *= 3.f / reps;
+            if (ms > 0.06f) break;
+        }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (!ok) {
@@ -2496,7 +2500,7 @@ bool Engine::autotune() {
         }
     }
     // The fastest tile of one pass timed alone; with early launch (small fixed-step
-    // problems) the widest tile within 5 % of it: fewer CTAs of the next kernel are then
+    // problems) the widest tile within 2 % of it: fewer CTAs of the next kernel are then
     // resident and waiting beside the current one (measured on 256x64x1 RK4: 0.0645 ms/step
     // with 65 thin-film CTAs against 0.0755 with 129, which timed alike on their own).
     auto pick_tile = [&](const std::vector<std::pair<int, float>> &cand, int cur) {
@@ -2510,7 +2514,7 @@ bool Engine::autotune() {
             }
         if (early_launch)
             for (const auto &c : cand)
-                if (c.second <= 1.05f * bt && c.first > best) best = c.first;
+                if (c.second <= 1.02f * bt && c.first > best) best = c.first;
         return best;
     };
     if (demag) {
@@ -2588,10 +2592,9 @@ bool Engine::autotune() {
         }
     }
     if (!std::getenv("FULLMAG_FDM_ROWS_PER_CTA")) {
-        // a full stage pass: inverse x, fields, statistics, combination, forward x
-        int best = row_rows;
-        float bt = 1e30f;
+        // an intermediate stage: inverse x, fields, combination, forward x
         const int nrows = g.ny * g.nz;
+        std::vector<std::pair<int, float>> cand;
         for (int rows : {1, 2, 4, 8, 16}) {
             if (rows > nrows || rows * g.nx > 8192) continue;
             RowPass p = row_base();
@@ -2599,7 +2602,6 @@ bool Engine::autotune() {
             p.x_in = demag ? X : nullptr;
             p.m_in = S[0];
             p.k_out = K[0];
-            p.partials = partials;
             p.m0 = S[1];
             p.m_next = A[0];
             p.n_comb = 1;
@@ -2607,13 +2609,9 @@ bool Engine::autotune() {
             p.comb_c[0] = 0.f;
             p.x_out = demag ? X : nullptr;
             if (row_pass_smem(p) > 200u * 1024u) continue;
-            const float t = time_ms([&] { return launch_row_pass(p, stream) == cudaSuccess; });
-            if (t < bt) {
-                bt = t;
-                best = rows;
-            }
+            cand.emplace_back(rows, time_ms([&] { return launch_row_pass(p, stream) == cudaSuccess; }));
         }
-        row_rows = best;
+        row_rows = pick_tile(cand, row_rows);
     }
     row_blocks = (g.ny * g.nz + row_rows - 1) / row_rows;
     // the timed launches only wrote scratch (X, Y, A[0], K[0], partials); every one of

@@ -34,7 +34,8 @@ int row_pass_length(const Grid &g, bool demag) {
 size_t row_pass_smem(const RowPass &p) {
     const bool use_fft = (p.x_in != nullptr) || (p.x_out != nullptr);
     size_t b = 0;
-    if (use_fft) b += 2 * sizeof(float2) * (size_t)p.rows * 3 * skewed_len(p.g.half);
+    // one buffer for the two-level transforms of half lines (in place), else two
+    if (use_fft) b += (row_pass_length(p.g, true) && !(p.g.per & 1) ? 1 : 2) * sizeof(float2) * (size_t)p.rows * 3 * skewed_len(p.g.half);
     b += sizeof(double) * kWarps * kNumStats;
     return b;
 }
@@ -49,7 +50,9 @@ cudaError_t launch_row_pass(const RowPass &p, cudaStream_t s) {
     const int length = row_pass_length(p.g, p.x_in || p.x_out);
     const RowKernels &k = row_kernels_for(length);
     const bool lean = row_lean(p, length > 0);
-    const RowKernel fn = length && (p.g.per & 1) ? k.periodic[lean] : k.open[lean];
+    const RowKernel fn = length && (p.g.per & 1)                                ? k.periodic[lean]
+                         : lean && k.dense && row_pass_blocks(p) >= kDenseCtas ? k.dense
+                                                                               : k.open[lean];
     cudaError_t e = ensure_smem((const void *)fn, sm);
     if (e != cudaSuccess) return e;
     return launch_pdl(fn, dim3(row_pass_blocks(p)), dim3(kThreads), sm, s, p);

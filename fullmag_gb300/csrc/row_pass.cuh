@@ -25,10 +25,10 @@
 namespace fm {
 
 // The kernels of one x length, each length compiled in row_pass_lengths.cu ([0] everything,
-// [1] intermediate stages).
+// [1] intermediate stages, dense those of large grids).
 using RowKernel = void (*)(const RowPass);
 struct RowKernels {
-    RowKernel open[2], periodic[2], adj;
+    RowKernel open[2], periodic[2], adj, dense;
 };
 template <int HALF>
 const RowKernels &row_kernels_of();
@@ -91,12 +91,12 @@ __host__ __device__ __forceinline__ bool row_x_periodic_ok(const Grid &g) {
 }
 
 // X rows (global, nkx = half + 1 values per line) -> H_d samples in
-// hd[line*lsx + sk(x/2)] (.x for even x, .y for odd x), x < nx.  Phase A (line, k1):
+// buf[line*lsx + sk(x/2)] (.x for even x, .y for odd x), x < nx.  Phase A (line, k1):
 // Z[k] = (a + b') + i (a - b') conj(e^{-2 pi i k/px}), a = X[k], b' = conj(X[half-k]),
 // for k = k1 + N1 k2 from global loads, inverse N2-point DFT, conjugate twiddle;
 // phase B (line, n2): outer inverse.
 template <int half, bool FULL>
-__device__ __forceinline__ void row_inverse_x(const RowPass &p, int rows, int row0, float2 *slots, float2 *hd) {
+__device__ __forceinline__ void row_inverse_x(const RowPass &p, int rows, int row0, float2 *buf, float2 *other) {
     constexpr int N1 = split_line(half), N2 = half / N1, H1 = N1 / 2;
     constexpr int lsx = skewed_len(half);
     const Grid &g = p.g;
@@ -117,72 +117,91 @@ __device__ __forceinline__ void row_inverse_x(const RowPass &p, int rows, int ro
             v[k2] = cadd(cadd(a, b), mul_i(O));
         }
         dft_small<N2>(v, true);
-        float2 *sl = slots + line * lsx;
+        float2 *sl = buf + line * lsx;
 #pragma unroll
         for (int n2 = 0; n2 < N2; ++n2) sl[sk(k1 * N2 + n2)] = (n2 && k1) ? cmul(v[n2], cconj(__ldg(tw + n2 * k1))) : v[n2];
     }
     __syncthreads();
-    for (int it = threadIdx.x; it < nl * N2; it += blockDim.x) {
-        const int line = it / N2, n2 = it % N2;
+    // open x, in place: whole lines at a time, all of a line's reads before its writes
+    constexpr int L = kThreads / N2;
+    const int l0 = threadIdx.x / N2, n2 = threadIdx.x % N2;
+    for (int base = 0; base < nl; base += L) {
+        const bool act = l0 < L && base + l0 < nl;
+        float2 *h = other + (base + l0) * lsx;
         float2 e[H1], f[H1];
-        idft_load<N1, N2, FULL>(e, f, n2, slots + line * lsx, tw);
-        float2 *h = hd + line * lsx;
+        if (act) idft_load<N1, N2, FULL>(e, f, n2, buf + (base + l0) * lsx, tw);
+        if (!FULL) __syncthreads();
+        if (act) {
 #pragma unroll
-        for (int j1 = 0; j1 < H1; ++j1) {
-            h[sk(N2 * j1 + n2)] = e[j1];
-            if (FULL) h[sk(N2 * (j1 + H1) + n2)] = f[j1];
+            for (int j1 = 0; j1 < H1; ++j1) {
+                h[sk(N2 * j1 + n2)] = e[j1];
+                if (FULL) h[sk(N2 * (j1 + H1) + n2)] = f[j1];
+            }
         }
     }
     __syncthreads();
 }
 
-// Next-stage samples s[x], x < nx, in pack[line*lsx + sk(x/2)] -> X rows (global).
+// Next-stage samples s[x], x < nx, in buf[line*lsx + sk(x/2)] -> X rows (global).
 // Phase 1 (line, n2): outer DFT of z[j] (open x: j < half/2, samples x >= nx read as
 // zero); phase 2 (line, k1): inner N2-point DFTs into natural order; phase 3
 // (line, k): the real-to-half-spectrum split
 // X[k] = (Z[k] + Z'[k])/2 + e^{-2 pi i k/px} (Z[k] - Z'[k])/(2i), Z'[k] = conj(Z[half-k]).
 template <int half, bool FULL>
-__device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int row0, float2 *pack, float2 *slots) {
+__device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int row0, float2 *buf, float2 *other) {
     constexpr int N1 = split_line(half), N2 = half / N1, H1 = N1 / 2;
     constexpr int lsx = skewed_len(half);
     const Grid &g = p.g;
     constexpr int nkx = half + 1;
     const int nx = g.nx, nrows = g.ny * g.nz, nl = rows * 3;
     const float2 *__restrict__ tw = p.xplan.tw;
-    for (int it = threadIdx.x; it < nl * N2; it += blockDim.x) {
-        const int line = it / N2, n2 = it % N2;
-        const float2 *src = pack + line * lsx;
-        float2 e[H1];
+    {
+        constexpr int L = kThreads / N2;
+        const int l0 = threadIdx.x / N2, n2 = threadIdx.x % N2;
+        for (int base = 0; base < nl; base += L) {
+            const bool act = l0 < L && base + l0 < nl;
+            float2 *line = buf + (base + l0) * lsx;
+            float2 e[H1], f[H1];
+            if (act) {
 #pragma unroll
-        for (int j1 = 0; j1 < H1; ++j1) {
-            const int j = N2 * j1 + n2;
-            float2 v = src[sk(j)];
-            if (!FULL && 2 * j + 1 >= nx) {
-                v.y = 0.f;
-                if (2 * j >= nx) v.x = 0.f;
+                for (int j1 = 0; j1 < H1; ++j1) {
+                    const int j = N2 * j1 + n2;
+                    float2 v = line[sk(j)];
+                    if (!FULL && 2 * j + 1 >= nx) {
+                        v.y = 0.f;
+                        if (2 * j >= nx) v.x = 0.f;
+                    }
+                    e[j1] = v;
+                    if (FULL) f[j1] = line[sk(N2 * (j1 + H1) + n2)];
+                }
             }
-            e[j1] = v;
-        }
-        if constexpr (FULL) {
-            float2 f[H1];
-#pragma unroll
-            for (int j1 = 0; j1 < H1; ++j1) f[j1] = src[sk(N2 * (j1 + H1) + n2)];
-            full_dft_store<N1, N2>(e, f, n2, slots + line * lsx, tw);
-        } else {
-            half_dft_store<N1, N2>(e, n2, slots + line * lsx, tw);
+            if (!FULL) __syncthreads();
+            if (act) {
+                if constexpr (FULL) full_dft_store<N1, N2>(e, f, n2, other + (base + l0) * lsx, tw);
+                else half_dft_store<N1, N2>(e, n2, line, tw);
+            }
         }
     }
     __syncthreads();
-    for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
-        const int line = it / N1, k1 = it % N1;
-        const float2 *sl = slots + line * lsx;
-        float2 v[N2];
+    {
+        constexpr int L = kThreads / N1;
+        const int l0 = threadIdx.x / N1, k1 = threadIdx.x % N1;
+        for (int base = 0; base < nl; base += L) {
+            const bool act = l0 < L && base + l0 < nl;
+            float2 *z = buf + (base + l0) * lsx;
+            const float2 *slots = other + (base + l0) * lsx;
+            float2 v[N2];
+            if (act) {
 #pragma unroll
-        for (int n2 = 0; n2 < N2; ++n2) v[n2] = sl[sk(k1 * N2 + n2)];
-        dft_small<N2>(v, false);
-        float2 *z = pack + line * lsx;
+                for (int n2 = 0; n2 < N2; ++n2) v[n2] = slots[sk(k1 * N2 + n2)];
+                dft_small<N2>(v, false);
+            }
+            if (!FULL) __syncthreads();
+            if (act) {
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) z[sk(k1 + N1 * k2)] = v[k2];
+                for (int k2 = 0; k2 < N2; ++k2) z[sk(k1 + N1 * k2)] = v[k2];
+            }
+        }
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < nl * nkx; idx += blockDim.x) {
@@ -190,7 +209,7 @@ __device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int ro
         const int k = idx - line * nkx;
         const int rr = line / 3;
         const int c = line - rr * 3;
-        const float2 *zl = pack + line * lsx;
+        const float2 *zl = buf + line * lsx;
         const float2 a = zl[sk(k == half ? 0 : k)];
         const float2 b = cconj(zl[sk(k == 0 ? 0 : half - k)]);
         const float2 E = cscale(cadd(a, b), 0.5f);
@@ -204,10 +223,10 @@ __device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int ro
 #define FM_LENGTHS_CLASS1(F) F(16) F(20) F(24) F(28) F(32) F(40) F(48) F(56) F(64)
 #define FM_LENGTHS_CLASS2(F) F(80) F(96) F(112) F(128) F(160) F(192) F(224) F(256)
 template <int HALF, bool PX>
-__device__ __forceinline__ void row_inverse_x_select(const RowPass &p, int rows, int row0, float2 *slots, float2 *hd) {
+__device__ __forceinline__ void row_inverse_x_select(const RowPass &p, int rows, int row0, float2 *buf, float2 *other) {
 #define FM_CASE(n) \
-    case n: row_inverse_x<n, PX>(p, rows, row0, slots, hd); return;
-    if constexpr (HALF > 0) row_inverse_x<HALF, PX>(p, rows, row0, slots, hd);
+    case n: row_inverse_x<n, PX>(p, rows, row0, buf, other); return;
+    if constexpr (HALF > 0) row_inverse_x<HALF, PX>(p, rows, row0, buf, other);
     else if constexpr (HALF == -1)
         switch (p.g.half) { FM_LENGTHS_CLASS1(FM_CASE) }
     else if constexpr (HALF == -2)
@@ -217,10 +236,10 @@ __device__ __forceinline__ void row_inverse_x_select(const RowPass &p, int rows,
 #undef FM_CASE
 }
 template <int HALF, bool PX>
-__device__ __forceinline__ void row_forward_x_select(const RowPass &p, int rows, int row0, float2 *pack, float2 *slots) {
+__device__ __forceinline__ void row_forward_x_select(const RowPass &p, int rows, int row0, float2 *buf, float2 *other) {
 #define FM_CASE(n) \
-    case n: row_forward_x<n, PX>(p, rows, row0, pack, slots); return;
-    if constexpr (HALF > 0) row_forward_x<HALF, PX>(p, rows, row0, pack, slots);
+    case n: row_forward_x<n, PX>(p, rows, row0, buf, other); return;
+    if constexpr (HALF > 0) row_forward_x<HALF, PX>(p, rows, row0, buf, other);
     else if constexpr (HALF == -1)
         switch (p.g.half) { FM_LENGTHS_CLASS1(FM_CASE) }
     else if constexpr (HALF == -2)
@@ -539,7 +558,9 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
     const int lsx = skewed_len(half);  // line stride of the x-transform buffers
     const int flen = p.rows * 3 * lsx;
     float2 *fa = reinterpret_cast<float2 *>(smem);
-    float2 *fb = fa + (use_fft ? flen : 0);
+    // two-level transforms of half lines work in place; full lines would hold twice the values
+    // across the barrier, and spill
+    float2 *fb = HALF && !PX ? fa : fa + (use_fft ? flen : 0);
     float2 *red = fb + (use_fft ? flen : 0);  // per-warp statistics
 
     // ---- (1) inverse x-transform of the demag spectrum ----
@@ -653,12 +674,12 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
                     }
                 }
                 if (hd) {
-                    const float2 a = hd[(rr * 3 + 0) * lsx + sk(x >> 1)];
-                    const float2 b = hd[(rr * 3 + 1) * lsx + sk(x >> 1)];
-                    const float2 c = hd[(rr * 3 + 2) * lsx + sk(x >> 1)];
-                    dx_ = (x & 1) ? a.y : a.x;
-                    dy_ = (x & 1) ? b.y : b.x;
-                    dz_ = (x & 1) ? c.y : c.x;
+                    // (its own half of the pair: the neighbour cell's may already hold the next
+                    // stage's sample)
+                    const float *h = reinterpret_cast<const float *>(hd) + 2 * (rr * 3 * lsx + sk(x >> 1)) + (x & 1);
+                    dx_ = h[0];
+                    dy_ = h[2 * lsx];
+                    dz_ = h[4 * lsx];
                 }
                 hx = ex + dx_;
                 hy = ey + dy_;
@@ -917,7 +938,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
     if constexpr (HALF != 0) {
         if (LEAN || p.x_out) {
             __syncthreads();  // every sample packed, every H_d sample of fb read
-            row_forward_x_select<HALF, PX>(p, rows, row0, pack, fb);
+            row_forward_x_select<HALF, PX>(p, rows, row0, fa, fb);
         }
     } else if (p.x_out) {
         // zero the padded half x in [nx, px) of every packed line
@@ -981,8 +1002,17 @@ __device__ __forceinline__ void finalize_stats(const RowPass &p, const int nblk)
 // SM, the others three of 80.
 constexpr int row_ctas(int half) { return half > 256 || half == -3 ? 2 : 3; }
 
-template <int HALF, bool PX, bool LEAN>
-__global__ void __launch_bounds__(kThreads, row_ctas(HALF)) row_pass_kernel(const RowPass p) {
+// DENSE: intermediate stages of a grid that fills every SM several times over, at four CTAs of
+// 64 registers.  With the transforms in place they leave the L1 cache half of the SM's memory,
+// which the neighbour rows of the stencil need (256x256x64, 4 rows a CTA: 137 us per launch at
+// three CTAs and two buffers, 145 at four and two, 135 at three and one, 125 at four and one).
+// A small grid, bound by the latency of one CTA, is slower with fewer registers (256x64 film, 50
+// RK4 steps: 1.82 ms at 80, 2.04 at 64).
+constexpr bool row_dense_ok(int half) { return half >= 64 && half <= 256; }
+constexpr int kDenseCtas = 152 * 4 * 2;
+
+template <int HALF, bool PX, bool LEAN, bool DENSE = false>
+__global__ void __launch_bounds__(kThreads, DENSE ? 4 : row_ctas(HALF)) row_pass_kernel(const RowPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     row_pass_body<HALF, PX, false, LEAN>(p, blockIdx.x, gridDim.x);
@@ -1007,6 +1037,7 @@ RowKernels row_kernels() {
             k.periodic[lean] = lean ? row_pass_kernel<HALF, true, true> : row_pass_kernel<HALF, true, false>;
     }
     k.adj = row_pass_adj_kernel<HALF>;
+    if constexpr (row_dense_ok(HALF)) k.dense = row_pass_kernel<HALF, false, true, true>;
     return k;
 }
 
