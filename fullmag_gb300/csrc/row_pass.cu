@@ -21,7 +21,7 @@ static const RowKernels &row_kernels_for(int half) {
 
 // an intermediate stage: what LEAN leaves out is not asked for
 static bool row_lean(const RowPass &p, bool transforms) {
-    return p.m_in && p.m0 && !p.partials && !p.n_err && !p.h_ex_out && !p.h_d_out && !p.h_eff_out && !p.adj_mode &&
+    return p.m_in && p.m0 && !p.partials && !p.n_err && !p.h_ex_out && !p.h_d_out && !p.adj_mode &&
            (!transforms || (p.x_in && p.x_out));
 }
 

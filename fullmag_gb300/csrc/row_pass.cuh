@@ -454,7 +454,7 @@ __device__ __forceinline__ void cells_vec(const RowPass &p, int rows, int row0, 
                     mx2[1] = fmaxf(mx2[1], dx_ * dx_ + dy_ * dy_ + dz_ * dz_);
                     mx2[2] = fmaxf(mx2[2], kv[0][j] * kv[0][j] + kv[1][j] * kv[1][j] + kv[2][j] * kv[2][j]);
                 }
-                if (!LEAN && p.h_eff_out) {
+                if (p.h_eff_out) {
                     const long long i = i0 + j;
                     p.h_eff_out[i] = hx;
                     p.h_eff_out[n + i] = hy;
@@ -543,7 +543,7 @@ __device__ __forceinline__ void cells_vec(const RowPass &p, int rows, int row0, 
 // HALF, PX: the x length (0 general, -1 to -3 a class) and whether its lines are full
 // (periodic x).  LEAN: an
 // intermediate stage -- right-hand side, combination and (HALF) both x-transforms, without
-// statistics, error norm or observables.
+// statistics, error norm or observables other than H_eff (which the reverse sweep stores).
 template <int HALF, bool PX, bool ADJ, bool LEAN>
 __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, const int nblk) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -765,7 +765,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
                 p.k_out[n + i] = ky_;
                 p.k_out[2 * n + i] = kz_;
             }
-            if (!LEAN && p.h_eff_out) {
+            if (p.h_eff_out) {
                 p.h_eff_out[i] = hx;
                 p.h_eff_out[n + i] = hy;
                 p.h_eff_out[2 * n + i] = hz;
