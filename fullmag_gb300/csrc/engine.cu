@@ -769,14 +769,19 @@ struct Engine {
         cudaEventCreate(&e1);
         bool ok = fn();  // warm-up (also sets shared-memory attributes)
         float ms = 0.f;
-        for (int reps : {3, 9}) {  // launches of a few microseconds are timed again, longer
+        // launches of a few microseconds are timed in more and longer batches, the fastest of which
+        // counts: the host's launch jitter is of their size
+        for (int b = 0; b < 4; ++b) {
+            const int reps = b ? 6 : 3;
             cudaEventRecord(e0, stream);
             for (int r = 0; r < reps && ok; ++r) ok = fn();
             cudaEventRecord(e1, stream);
             cudaEventSynchronize(e1);
-            cudaEventElapsedTime(&ms, e0, e1);
-            ms *= 3.f / reps;
-            if (ms > 0.06f) break;
+            float t = 0.f;
+            cudaEventElapsedTime(&t, e0, e1);
+            t *= 3.f / reps;
+            ms = b > 1 ? std::min(ms, t) : t;
+            if (b == 0 && ms > 0.06f) break;
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -2499,11 +2504,13 @@ bool Engine::autotune() {
             return true;
         }
     }
-    // The fastest tile of one pass timed alone; with early launch (small fixed-step
-    // problems) the widest tile within 2 % of it: fewer CTAs of the next kernel are then
-    // resident and waiting beside the current one (measured on 256x64x1 RK4: 0.0645 ms/step
-    // with 65 thin-film CTAs against 0.0755 with 129, which timed alike on their own).
-    auto pick_tile = [&](const std::vector<std::pair<int, float>> &cand, int cur) {
+    // The fastest tile of one pass timed alone; with early launch (small fixed-step problems)
+    // the widest tile within 5 % of it that still makes 32 CTAs of the pass's `units` kx columns
+    // or rows: fewer CTAs of the next kernel are then resident and waiting beside the current
+    // one (256x64 film, RK4: 0.0645 ms/step with 65 thin-film CTAs against 0.0755 with 129, which
+    // timed alike on their own; 64x32x4 Heun, 16 steps: 524 us with 64 row-pass CTAs, 550 with
+    // 128; but 256x256 periodic film, 20 RK4 steps: 1.12 ms with 33 thin-film CTAs, 1.25 with 17).
+    auto pick_tile = [&](const std::vector<std::pair<int, float>> &cand, int cur, int units) {
         if (cand.empty()) return cur;
         float bt = 1e30f;
         int best = cur;
@@ -2514,7 +2521,7 @@ bool Engine::autotune() {
             }
         if (early_launch)
             for (const auto &c : cand)
-                if (c.second <= 1.02f * bt && c.first > best) best = c.first;
+                if (c.second <= 1.05f * bt && c.first > best && units / c.first >= 32) best = c.first;
         return best;
     };
     if (demag) {
@@ -2524,14 +2531,14 @@ bool Engine::autotune() {
                 if (tx > std::max(1, g.nkx) || y_convolve_2d_smem(g, tx) > 200u * 1024u) continue;
                 cand.emplace_back(tx, time_ms([&] { return launch_y_convolve_2d(col_pass(plan_y, tx, X, X), stream) == cudaSuccess; }));
             }
-            tx_2d = pick_tile(cand, tx_2d);
+            tx_2d = pick_tile(cand, tx_2d, g.nkx);
         } else if (use_yz) {
             std::vector<std::pair<int, float>> cand;
             for (int tx : {1, 2, 4, 8}) {
                 if (tx > std::max(1, g.nkx) || yz_convolve_smem(g, tx) > 200u * 1024u) continue;
                 cand.emplace_back(tx, time_ms([&] { return launch_yz_convolve(col_pass(plan_y, tx, X, X), stream) == cudaSuccess; }));
             }
-            tx_z = pick_tile(cand, tx_z);
+            tx_z = pick_tile(cand, tx_z, g.nkx);
         } else {
             // tile widths and radix splits of the three column passes, each timed on its own
             // (power-of-two lengths 16..256 have a second split N1 x N2)
@@ -2611,7 +2618,7 @@ bool Engine::autotune() {
             if (row_pass_smem(p) > 200u * 1024u) continue;
             cand.emplace_back(rows, time_ms([&] { return launch_row_pass(p, stream) == cudaSuccess; }));
         }
-        row_rows = pick_tile(cand, row_rows);
+        row_rows = pick_tile(cand, row_rows, nrows);
     }
     row_blocks = (g.ny * g.nz + row_rows - 1) / row_rows;
     // the timed launches only wrote scratch (X, Y, A[0], K[0], partials); every one of
