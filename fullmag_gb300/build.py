@@ -20,7 +20,7 @@ SOURCES = ["row_pass.cu", "row_pass_batched.cu", "columns.cu", "columns_z.cu", "
            "newell.cu", "noalloc.cu", "extra_field.cu", "fp64.cu"]
 # kernels per transform length, compiled in groups (FM_GROUP) so that they build in parallel
 GROUPED = ["row_pass_lengths.cu", "columns_lengths.cu"]
-GROUPS = range(7)
+GROUPS = range(9)
 # the cuFFT + unfused measurement baseline: a separate library, never linked into the product
 PLAIN_SOURCES = ["plain_baseline.cu"]
 PLAIN_LIB = OUT / "libfullmag_fdm_plain.so"

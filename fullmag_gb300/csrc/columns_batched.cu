@@ -8,7 +8,7 @@ namespace {
 // work[blockIdx.x] = (problem, kx tile); KIND: see col_batched_kind -- one kernel per kind, so
 // each gets its own register allocation
 template <int KIND>
-__global__ void __launch_bounds__(kThreads, KIND >= 9 ? 4 : KIND >= 6 ? 1 : 2) col_batched_kernel(
+__global__ void __launch_bounds__(kThreads, KIND >= 9 ? 4 : KIND >= 6 || KIND == 2 ? 1 : 2) col_batched_kernel(
     const ColPass *__restrict__ ps, const int2 *__restrict__ work) {
     __shared__ __align__(16) unsigned char desc[sizeof(ColPass)];  // descriptor staged once per CTA
     const int2 w = work[blockIdx.x];

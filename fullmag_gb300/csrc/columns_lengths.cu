@@ -6,9 +6,9 @@ namespace fm {
 
 namespace {
 
-// (from 320 on the inner pass of a film holds up to 3 x 16 complex values a thread)
+// (from 320 on the inner pass of a film holds 3 x 10 to 3 x 32 complex values a thread)
 template <int N, bool FULL, bool PER>
-__global__ void __launch_bounds__(kThreads, 2) y_convolve_2d_kernel(const ColPass p) {
+__global__ void __launch_bounds__(kThreads, N > 512 ? 1 : 2) y_convolve_2d_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     y_convolve_2d_fused<N, FULL, PER>(p, blockIdx.x);
@@ -40,8 +40,12 @@ ConvKernels conv_kernels() {
 #define FM_GROUP_LENGTHS(F) F(128) F(160) F(192)
 #elif FM_GROUP == 5
 #define FM_GROUP_LENGTHS(F) F(224) F(256) F(320)
-#else
+#elif FM_GROUP == 6
 #define FM_GROUP_LENGTHS(F) F(384) F(448) F(512)
+#elif FM_GROUP == 7
+#define FM_GROUP_LENGTHS(F) F(640) F(768)
+#else
+#define FM_GROUP_LENGTHS(F) F(896) F(1024)
 #endif
 
 #define FM_ENTRY(n) \

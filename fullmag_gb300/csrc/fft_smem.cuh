@@ -301,6 +301,42 @@ __device__ __forceinline__ void dft_small<14>(float2 *v, bool inv) {
     dft_coprime<2, 7>(v, inv);
 }
 
+template <>
+__device__ __forceinline__ void dft_small<20>(float2 *v, bool inv) {
+    dft_coprime<4, 5>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<24>(float2 *v, bool inv) {
+    dft_coprime<8, 3>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<28>(float2 *v, bool inv) {
+    dft_coprime<4, 7>(v, inv);
+}
+template <>
+__device__ __forceinline__ void dft_small<32>(float2 *v, bool inv) {
+    // even outputs from v[n] + v[n + 16], odd ones from (v[n] - v[n + 16]) W32^n
+    const float c32[16] = {1.0f,           0.98078528040323043f,  0.92387953251128674f,  0.83146961230254524f,
+                           0.70710678118654752f,  0.55557023301960218f,  0.38268343236508977f,  0.19509032201612825f,
+                           0.0f,           -0.19509032201612825f, -0.38268343236508977f, -0.55557023301960218f,
+                           -0.70710678118654752f, -0.83146961230254524f, -0.92387953251128674f, -0.98078528040323043f};
+    float2 a[16], b[16];
+#pragma unroll
+    for (int n = 0; n < 16; ++n) {
+        a[n] = cadd(v[n], v[n + 16]);
+        const float2 d = csub(v[n], v[n + 16]);
+        const float s = c32[n < 8 ? 8 - n : n - 8];  // sin(2 pi n / 32)
+        b[n] = n == 0 ? d : n == 8 ? mul_mi(d, inv) : cmul(d, make_float2(c32[n], inv ? s : -s));
+    }
+    dft_small<16>(a, inv);
+    dft_small<16>(b, inv);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        v[2 * k] = a[k];
+        v[2 * k + 1] = b[k];
+    }
+}
+
 // radix of the next power-of-two stage given the remaining length 2^m:
 // radix 16 where possible, never a lone radix-2 stage (2^5 -> 8 x 4, 2^9 -> 16 x 8 x 4)
 __host__ __device__ constexpr int pow2_radix(int rem) {
@@ -315,19 +351,19 @@ __host__ __device__ constexpr int pow2_radix(int rem) {
 // along a periodic axis (no padding) they run on full ones.  tw holds the N twiddles
 // e^{-2 pi i e / N}.
 //
-// Lengths: 2^a, 5/4 2^a, 3/2 2^a and 7/4 2^a from 16 to 512, so that padding 2n - 1 samples
+// Lengths: 2^a, 5/4 2^a, 3/2 2^a and 7/4 2^a from 16 to 1024, so that padding 2n - 1 samples
 // up to the next one costs at most a quarter (11 % on average over log-uniform n) where a
 // power of two costs up to a factor of two per axis.  A 150 x 150 x 10 box takes 320 x 320
 // x 20 points instead of 512 x 512 x 32.
 __host__ __device__ constexpr bool two_level_length(int n) {
     return n == 16 || n == 20 || n == 24 || n == 28 || n == 32 || n == 40 || n == 48 || n == 56 || n == 64 || n == 80 ||
            n == 96 || n == 112 || n == 128 || n == 160 || n == 192 || n == 224 || n == 256 || n == 320 || n == 384 ||
-           n == 448 || n == 512;
+           n == 448 || n == 512 || n == 640 || n == 768 || n == 896 || n == 1024;
 }
 // Outer length N1 of a pass whose inner pass holds one line of N2 = n / N1 values a thread:
-// both at most 16 (N1 counts half on open axes) up to n = 256.
+// both at most 16 (N1 counts half on open axes) up to n = 256, 32 beyond.
 __host__ __device__ constexpr int split_line(int n) {
-    return n <= 28 ? 4 : n <= 64 ? 8 : n <= 256 ? 16 : n / 16;
+    return n <= 28 ? 4 : n <= 64 ? 8 : n <= 256 ? 16 : n <= 512 ? n / 16 : 32;
 }
 // The same for a convolution pass, whose inner pass holds three lines: N2 <= 8 up to 256.
 __host__ __device__ constexpr int split_conv(int n) {
@@ -402,10 +438,10 @@ __device__ __forceinline__ void half_idft_load(float2 (&e)[N1 / 2], int n2, cons
     idft_load<N1, N2, false>(e, o, n2, line, tw);
 }
 
-// case labels of the two-level lengths: F(n) for each
+// case labels of the two-level lengths: F(n) for each (the long ones hold up to 32 complex values a thread)
 #define FM_LENGTHS_TO_256(F) \
     F(16) F(20) F(24) F(28) F(32) F(40) F(48) F(56) F(64) F(80) F(96) F(112) F(128) F(160) F(192) F(224) F(256)
-#define FM_LENGTHS_LONG(F) F(320) F(384) F(448) F(512)
+#define FM_LENGTHS_LONG(F) F(320) F(384) F(448) F(512) F(640) F(768) F(896) F(1024)
 
 // ---- runtime-length path ----
 

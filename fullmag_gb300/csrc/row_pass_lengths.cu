@@ -16,8 +16,12 @@ namespace fm {
 #define FM_GROUP_LENGTHS(F) F(128) F(160) F(192)
 #elif FM_GROUP == 5
 #define FM_GROUP_LENGTHS(F) F(224) F(256) F(320)
-#else
+#elif FM_GROUP == 6
 #define FM_GROUP_LENGTHS(F) F(384) F(448) F(512)
+#elif FM_GROUP == 7
+#define FM_GROUP_LENGTHS(F) F(640) F(768)
+#else
+#define FM_GROUP_LENGTHS(F) F(896) F(1024)
 #endif
 
 #define FM_ENTRY(n) \

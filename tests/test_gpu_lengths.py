@@ -1,5 +1,5 @@
 """The single-precision line transforms at every two-level length (2^a times 1, 5/4, 3/2, 7/4
-from 16 to 512) of each axis: rows, thin films, the three-pass and the fused column passes,
+from 16 to 1024) of each axis: rows, thin films, the three-pass and the fused column passes,
 the register, packed and shared-memory z passes, the unpadded (periodic) forms, the batched
 kernels and the reverse sweep.  Against the FP64 oracle within 1e-6 relative L2: an FP32
 transform of length N rounds about 3 log2 N times per axis and direction by 2^-24, at random,
@@ -34,7 +34,8 @@ def open_box(oracle, nx, ny, nz, seed=41):
 FILMS = [(17, 9, 20, 20), (23, 11, 24, 24), (28, 14, 28, 28), (32, 16, 32, 32), (33, 17, 40, 40), (47, 24, 48, 48),
          (50, 28, 56, 56), (64, 31, 64, 64), (65, 33, 80, 80), (96, 41, 96, 96), (110, 56, 112, 112),
          (128, 57, 128, 128), (129, 65, 160, 160), (190, 96, 192, 192), (193, 97, 224, 224), (256, 128, 256, 256),
-         (257, 129, 320, 320), (384, 161, 384, 384), (385, 193, 448, 448), (511, 256, 512, 512), (513, 257, 1024, 1024)]
+         (257, 129, 320, 320), (384, 161, 384, 384), (385, 193, 448, 448), (511, 256, 512, 512), (513, 257, 640, 640),
+         (768, 380, 768, 768), (770, 448, 896, 896), (1000, 500, 1024, 1024), (1025, 513, 2048, 2048)]
 
 
 @pytest.mark.parametrize("nx,ny,half,py", FILMS)
@@ -43,7 +44,7 @@ def test_films(gpu_lib, oracle, nx, ny, half, py):
     assert (px, p) == (2 * half, py)
 
 
-@pytest.mark.parametrize("ny", [1, 9, 12, 13, 17, 21, 28, 32, 40, 48, 50, 64, 70, 90, 100, 128, 150, 192, 200, 256])
+@pytest.mark.parametrize("ny", [1, 9, 12, 13, 17, 21, 28, 32, 40, 48, 50, 64, 70, 90, 100, 128, 150, 192, 200, 256, 300, 384, 400, 512])
 @pytest.mark.parametrize("fused", [True, False])
 def test_y_passes(gpu_lib, oracle, monkeypatch, ny, fused):
     if not fused:
@@ -64,7 +65,7 @@ def test_z_in_registers(gpu_lib, oracle, monkeypatch, nz, fused):
 @pytest.mark.parametrize("pair", ["0", "1"])
 def test_z_in_shared_memory(gpu_lib, oracle, monkeypatch, nz, pair):
     monkeypatch.setenv("FULLMAG_FDM_Z_PAIR", pair)
-    open_box(oracle, 9, 260, nz)  # py = 640 rounds to 1024: the plane does not fit the fused pass
+    open_box(oracle, 9, 260, nz)  # py = 640: the plane does not fit the fused pass
 
 
 def test_small_plane_beyond_the_register_lengths(gpu_lib, oracle):
@@ -75,7 +76,8 @@ def test_small_plane_beyond_the_register_lengths(gpu_lib, oracle):
 
 @pytest.mark.parametrize("shape,periodic", [((2 * h, n, 1), (1, 1, 0)) for h, n in
                                             [(16, 16), (20, 24), (28, 40), (48, 56), (80, 96), (112, 128), (160, 192),
-                                             (224, 256), (256, 320), (320, 384), (24, 448), (33, 34)]] +
+                                             (224, 256), (256, 320), (320, 384), (24, 448), (24, 640),
+                                             (20, 768), (16, 896), (16, 1024), (33, 34)]] +
                          [((40, 17, 1), (1, 0, 0)), ((48, 200, 1), (1, 0, 0)), ((33, 64, 1), (0, 1, 0)),
                           ((32, 20, 4), (1, 1, 0)), ((18, 24, 3), (0, 1, 0)), ((40, 11, 10), (1, 0, 0)),
                           ((20, 12, 14), (1, 1, 0))])
@@ -90,7 +92,7 @@ def test_batched_lengths(gpu_lib):
     """Films and small volumes of every batched kernel in one batch against the same problems
     alone: the two sides run the same step control on transforms that differ only in how the
     work is tiled, so after twenty small steps they agree to a few FP32 roundings."""
-    shapes = [(300, 8, 1), (20, 170, 1), (33, 17, 1), (8, 8, 5), (9, 170, 2), (24, 40, 3), (400, 20, 2), (13, 20, 13)]
+    shapes = [(300, 8, 1), (20, 170, 1), (33, 17, 1), (8, 8, 5), (9, 170, 2), (24, 40, 3), (400, 20, 2), (13, 20, 13), (600, 9, 1), (10, 300, 1), (10, 260, 2)]
     plans = [dict(problem(*s, seed=50 + i, alpha=0.1), integrator=_abi.INTEGRATOR_DP45, adaptive_max_error=1e-5,
                   adaptive_dt_max=5e-14) for i, s in enumerate(shapes)]
     batch = FdmBatch(plans)
