@@ -771,8 +771,8 @@ struct Engine {
         float ms = 0.f;
         // launches of a few microseconds are timed in more and longer batches, the fastest of which
         // counts: the host's launch jitter is of their size
-        for (int b = 0; b < 4; ++b) {
-            const int reps = b ? 6 : 3;
+        for (int b = 0; b < 3; ++b) {
+            const int reps = b ? 5 : 3;
             cudaEventRecord(e0, stream);
             for (int r = 0; r < reps && ok; ++r) ok = fn();
             cudaEventRecord(e1, stream);

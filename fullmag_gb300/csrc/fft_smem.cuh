@@ -11,7 +11,7 @@
 // is a power of two) take a compile-time path: radix-16 stages where possible,
 // then radix 8 or 4 (pow2_radix: never a lone radix-2 stage), all index
 // arithmetic folded to shifts and masks.  Other lengths use the runtime path
-// with radices 8, 4, 2 and an O(R^2) loop for any other prime factor.  Twiddles are FP64-computed host-side and stored as
+// with radices 8, 4, 2, 3, 5, 7 and an O(R^2) loop for any other prime factor.  Twiddles are FP64-computed host-side and stored as
 // float2 e^{-2 pi i e / n}; the inverse conjugates them.
 //
 // The passes over engine-built tensors take the two-level transforms further down at the
@@ -584,6 +584,9 @@ __device__ __forceinline__ float2 *fft_lines(float2 *a, float2 *b, int nlines, i
         if (R == 8) stage_fixed<8>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
         else if (R == 4) stage_fixed<4>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
         else if (R == 2) stage_fixed<2>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
+        else if (R == 3) stage_fixed<3>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
+        else if (R == 5) stage_fixed<5>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
+        else if (R == 7) stage_fixed<7>(a, b, nlines, ls, p.n, Ns, p.tw, inv);
         else stage_generic(a, b, nlines, ls, p.n, Ns, R, p.tw, inv);
         __syncthreads();
         float2 *t = a;
