@@ -78,7 +78,7 @@ def test_small_plane_beyond_the_register_lengths(gpu_lib, oracle):
                                             [(16, 16), (20, 24), (28, 40), (48, 56), (80, 96), (112, 128), (160, 192),
                                              (224, 256), (256, 320), (320, 384), (24, 448), (24, 640),
                                              (20, 768), (16, 896), (16, 1024), (33, 34),
-                                             (45, 105), (98, 75)]]  # the last: no table lengths, radices 2, 3, 5, 7, 11, 17 +
+                                             (45, 105), (98, 75)]] +
                          [((40, 17, 1), (1, 0, 0)), ((48, 200, 1), (1, 0, 0)), ((33, 64, 1), (0, 1, 0)),
                           ((32, 20, 4), (1, 1, 0)), ((18, 24, 3), (0, 1, 0)), ((40, 11, 10), (1, 0, 0)),
                           ((20, 12, 14), (1, 1, 0))])
