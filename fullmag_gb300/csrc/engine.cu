@@ -842,6 +842,9 @@ struct Engine {
     // RHS at the committed state -> K[0], statistics, optionally observables.
     bool eval_state(bool write_fields) {
         if (!set_oersted(time, time) || !set_thermal(th_step, th_step)) return false;
+        // the state or the field changed: a stage prepared before belongs to the old one (with
+        // demag the pass below clears it too, without it no pass writes X)
+        if (!k1_valid) prep_ready = false;
         if (!pass_forward(S[cur])) return false;
         bool fields_written = false;
         if (write_fields && has_torque) {
