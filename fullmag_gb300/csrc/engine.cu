@@ -2451,11 +2451,13 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
 }
 
 namespace {
+// Everything the search depends on: the shape, the column passes that run (yz), the tile rule of
+// early launch, which follows the integrator, and the choices forced through the environment.
 struct TuneKey {
-    int nx, ny, nz, px, py, pz, thin, masked, per;
+    int nx, ny, nz, px, py, pz, thin, masked, per, yz, early, z_forced, rows_forced;
     bool operator<(const TuneKey &o) const {
-        return std::tie(nx, ny, nz, px, py, pz, thin, masked, per) <
-               std::tie(o.nx, o.ny, o.nz, o.px, o.py, o.pz, o.thin, o.masked, o.per);
+        return std::tie(nx, ny, nz, px, py, pz, thin, masked, per, yz, early, z_forced, rows_forced) <
+               std::tie(o.nx, o.ny, o.nz, o.px, o.py, o.pz, o.thin, o.masked, o.per, o.yz, o.early, o.z_forced, o.rows_forced);
     }
 };
 struct TuneChoice {
@@ -2466,11 +2468,15 @@ std::map<TuneKey, TuneChoice> g_tune_cache;
 }  // namespace
 
 // Picks the kx tile width of each column pass and the rows per CTA of the row pass
-// by timing the candidates (3 launches each, CUDA events on the engine stream) on
-// the live, still-unused buffers.  Results are cached per grid shape in the process,
+// by timing the candidates (time_ms, CUDA events on the engine stream) on the live,
+// still-unused buffers.  Results are cached in the process by TuneKey,
 // so batched problems of the same shape pay for the search once.
 bool Engine::autotune() {
-    const TuneKey key{g.nx, g.ny, g.nz, g.px, g.py, g.pz, g.thin, has_mask ? 1 : 0, g.per};
+    // FULLMAG_FDM_Z_PAIR=0 or 1 forces the choice of the packed z pass
+    const char *zp_env = std::getenv("FULLMAG_FDM_Z_PAIR"), *rows_env = std::getenv("FULLMAG_FDM_ROWS_PER_CTA");
+    const int z_forced = zp_env && (zp_env[0] == '0' || zp_env[0] == '1') ? zp_env[0] - '0' : -1;
+    const TuneKey key{g.nx, g.ny,  g.nz,           g.px, g.py, g.pz, g.thin, has_mask ? 1 : 0,
+                      g.per, use_yz, early_launch, z_forced, rows_env ? row_rows : 0};
     // FULLMAG_FDM_TUNE="rows,tx_yf,tx_z,tx_yi,tx_2d,z_pair,split_yf,split_z,split_yi" fixes every
     // choice (the values fullmag_fdm_backend_tuning reports), e.g. so that a profiler run uses
     // the launch shapes of an unprofiled one
@@ -2502,7 +2508,7 @@ bool Engine::autotune() {
             split_yf = it->second.split_yf;
             split_z = it->second.split_z;
             split_yi = it->second.split_yi;
-            if (!std::getenv("FULLMAG_FDM_ROWS_PER_CTA")) row_rows = it->second.rows;
+            row_rows = it->second.rows;
             row_blocks = (g.ny * g.nz + row_rows - 1) / row_rows;
             return true;
         }
@@ -2577,15 +2583,13 @@ bool Engine::autotune() {
             } else {
                 tx_z = tune(tx_z, split_z, two_splits(g.pz), [&](int tx) { return z_convolve_smem(g, tx); },
                             [&](int tx, int sp) { return launch_z_convolve(cp(plan_z, tx, sp, Y, Y), stream) == cudaSuccess; });
-                // the packed ky-pair z pass (tile 8) against the best unpaired launch;
-                // FULLMAG_FDM_Z_PAIR=0 or 1 forces the choice
+                // the packed ky-pair z pass (tile 8) against the best unpaired launch
                 z_pair = 0;
-                const char *zp_env = std::getenv("FULLMAG_FDM_Z_PAIR");
-                if (z_convolve_pair_ok(g, 8) && zp_env && zp_env[0] == '1') {
+                if (z_convolve_pair_ok(g, 8) && z_forced == 1) {
                     tx_z = 8;
                     z_pair = 1;
                     split_z = 0;
-                } else if (z_convolve_pair_ok(g, 8) && !(zp_env && zp_env[0] == '0')) {
+                } else if (z_convolve_pair_ok(g, 8) && z_forced != 0) {
                     ColPass best = cp(plan_z, tx_z, split_z, Y, Y), paired = col_pass(plan_z, 8, Y, Y);
                     paired.pipe = 1;
                     const float t_best = time_ms([&] { return launch_z_convolve(best, stream) == cudaSuccess; });
@@ -2601,7 +2605,7 @@ bool Engine::autotune() {
                          [&](int tx, int sp) { return launch_y_inverse(cp(plan_y, tx, sp, Y, X), stream) == cudaSuccess; });
         }
     }
-    if (!std::getenv("FULLMAG_FDM_ROWS_PER_CTA")) {
+    if (!rows_env) {
         // an intermediate stage: inverse x, fields, combination, forward x
         const int nrows = g.ny * g.nz;
         std::vector<std::pair<int, float>> cand;
