@@ -1,9 +1,10 @@
 // columns.cu -- y transforms of the demag convolution, plus the deterministic final
-// reduction of the per-block statistics of batched problems.
+// reduction of the per-block statistics of large grids and of batched problems.
 //
 // Reference behaviour restated (paths in mzrptu/fullmag):
 //   multi-pass FP64 reductions                 native/backends/fdm/src/reductions_fp64.cu:30-84,354-393
 #include "columns.cuh"
+#include "stats.cuh"
 
 namespace fm {
 
@@ -239,6 +240,14 @@ __device__ __forceinline__ void finalize_body(const float2 *__restrict__ partial
     }
 }
 
+// One problem; up to kFinInPass CTAs in the order of the row pass that reduces its own.
+__global__ void __launch_bounds__(kFinThreads) finalize_stats_kernel(const float2 *__restrict__ partials, int nblocks,
+                                                                     double *__restrict__ out, int early) {
+    pdl_wait();
+    if (early) pdl_trigger();
+    if (nblocks > kFinInPass) finalize_body(partials, nblocks, out);
+    else if (threadIdx.x >> 5 < kNumStats) finalize_stat(partials, nblocks, threadIdx.x >> 5, out);
+}
 // One block per problem; statistics land in out[problem * kNumStats + s].
 __global__ void __launch_bounds__(kFinThreads) finalize_batched_kernel(const FinDesc *__restrict__ fd, double *__restrict__ out) {
     const FinDesc d = fd[blockIdx.x];
@@ -305,6 +314,10 @@ cudaError_t launch_y_inverse(const ColPass &p, cudaStream_t s) {
     cudaError_t e = ensure_smem((const void *)y_inverse_kernel, sm);
     if (e != cudaSuccess) return e;
     return launch_pdl(y_inverse_kernel, dim3(tiles(p), p.g.nz, 3), dim3(kThreads), sm, s, p);
+}
+
+cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early) {
+    return launch_pdl(finalize_stats_kernel, dim3(1), dim3(kFinThreads), 0, s, partials, nblocks, out, early);
 }
 
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s) {

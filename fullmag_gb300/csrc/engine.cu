@@ -679,7 +679,7 @@ struct Engine {
             rec_rows->push_back(p);
             return true;
         }
-        if (p.partials) {
+        if (p.partials && fin_in_pass()) {
             p.fin_out = hstats;
             p.fin_count = fin_count;
         }
@@ -804,10 +804,19 @@ struct Engine {
         return run_row(p) && run_columns();
     }
 
-    // The row pass that collects statistics finalizes them itself, into the pinned hstats; the
-    // extra pass before it left per-CTA sums of its own.
+    // A row pass of few CTAs finalizes its statistics itself, into the pinned hstats; the extra
+    // pass before it left per-CTA sums of its own.
+    bool fin_in_pass() const { return row_blocks <= kFinInPass; }
     bool enqueue_stats() {
-        if (rec_rows || !has_extra) return true;  // a batched round finalizes all problems at once
+        if (rec_rows) return true;  // a batched round finalizes all problems at once
+        if (!fin_in_pass()) {
+            launches += 1;
+            kt_begin(KT_FIN);
+            const cudaError_t rc = launch_finalize_stats(partials, row_blocks, hstats, stream, early_launch ? 1 : 0);
+            kt_end();
+            if (cuda_fail("finalize", rc)) return false;
+        }
+        if (!has_extra) return true;
         launches += 1;
         return !cuda_fail("extra finalize", launch_extra_finalize(xpart, extra_field_blocks(g), hstats + kNumStats + 1, stream,
                                                                   early_launch ? 1 : 0));

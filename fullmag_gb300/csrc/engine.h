@@ -300,6 +300,13 @@ int row_pass_length(const Grid &g, bool demag);  // x half length of the row-pas
 int row_pass_class(const Grid &g, bool demag);   // its class: 0 general, 1 up to 64, 2 up to 256, 3 longer
 cudaError_t launch_col_batched(const ColPass *ps, const int2 *work, int nwork, int kind, size_t smem, cudaStream_t s);
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s);
+// the nine sums / maxima of nblocks CTAs' partials into out
+cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early = 0);
+// Most row-pass CTAs whose statistics the last of them reduces; beyond, the reduction is a launch
+// of its own.  Every CTA of a pass that reduces waits for its fence and its count, which a CTA
+// cannot hide: Heun steps without demag, in the pass against a launch: 128 CTAs 20.0 / 23.5 us,
+// 512 28.5 / 29.4, 1024 37.5 / 36.2, 4096 88.6 / 72.5, 16384 393 / 318.
+constexpr int kFinInPass = 512;
 int row_pass_blocks(const RowPass &p);
 // Kernel of the batched column pass for a grid: 3 k + c with k = 0 thin film two-level, 1 fused
 // y+z two-level, 2 its longer z lengths and c the class of py (0 up to 64, 1 up to 256, 2

@@ -18,7 +18,7 @@
 // y/z transforms and the tensor multiply live in column passes, and no
 // padded real-space array or cuFFT plan exists.
 #pragma once
-#include "engine.h"
+#include "stats.cuh"
 
 #include <cfloat>
 
@@ -50,27 +50,6 @@ __device__ __forceinline__ float2 div2i(float2 a) { return make_float2(0.5f * a.
 __device__ __forceinline__ float2 mul_i(float2 a) { return make_float2(-a.y, a.x); }
 
 __device__ __forceinline__ bool cell_active(const uint8_t *mask, long long i) { return mask == nullptr || mask[i] != 0; }
-
-// butterfly all-reduce of a float-float value; every lane ends with the same bits
-// because each level combines the pair in lane order
-__device__ __forceinline__ void warp_ff_sum(float &h, float &l) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float oh = __shfl_xor_sync(0xffffffffu, h, o);
-        const float ol = __shfl_xor_sync(0xffffffffu, l, o);
-        const bool low = (threadIdx.x & o) == 0;
-        float ah = low ? h : oh, al = low ? l : ol;
-        const float bh = low ? oh : h, bl = low ? ol : l;
-        ff_add(ah, al, bh);
-        h = ah;
-        l = al + bl;
-    }
-}
-__device__ __forceinline__ float warp_maxf(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 // ---- x-transforms in the two-level form (half = px/2 = N1 * N2) ----
 // The real x line of length px is carried as the half-length complex line
@@ -967,11 +946,10 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
     }
 }
 
-// Final reduction of the CTAs' partials by the CTA that finishes last: one warp per statistic,
-// lanes striding over the CTAs with compensated sums (or maxima) and one butterfly, a fixed
-// order whichever CTA it is.  The nine results go straight to pinned host memory, so a step
-// with statistics ends with its row pass instead of with a one-CTA kernel and a copy behind
-// it (64 x 32 x 4 Heun: 39.7 -> 33.5 us a step).
+// Final reduction of the CTAs' partials by the CTA that finishes last, on grids of up to
+// kFinInPass CTAs.  The nine results go straight to pinned host memory, so a step with
+// statistics ends with its row pass instead of with a one-CTA kernel and a copy behind it
+// (64 x 32 x 4 Heun: 39.7 -> 33.5 us a step).
 __device__ __forceinline__ void finalize_stats(const RowPass &p, const int nblk) {
     __shared__ bool last;
     __syncthreads();
@@ -979,22 +957,7 @@ __device__ __forceinline__ void finalize_stats(const RowPass &p, const int nblk)
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const int lane = threadIdx.x & 31;
-    for (int s = threadIdx.x >> 5; s < kNumStats; s += kWarps) {
-        float h = 0.f, l = 0.f;
-        for (int b = lane; b < nblk; b += 32) {
-            const float2 v = __ldcg(p.partials + (size_t)s * nblk + b);
-            if (s < 5) {
-                ff_add(h, l, v.x);
-                l += v.y;
-            } else {
-                h = fmaxf(h, v.x);
-            }
-        }
-        if (s < 5) warp_ff_sum(h, l);
-        else h = warp_maxf(h);
-        if (lane == 0) p.fin_out[s] = (double)h + (double)l;
-    }
+    for (int s = threadIdx.x >> 5; s < kNumStats; s += kWarps) finalize_stat(p.partials, nblk, s, p.fin_out);
     if (threadIdx.x == 0) *p.fin_count = 0;  // for the next launch
 }
 
