@@ -806,7 +806,8 @@ struct Engine {
 
     // A row pass of few CTAs finalizes its statistics itself, into the pinned hstats; the extra
     // pass before it left per-CTA sums of its own.
-    bool fin_in_pass() const { return row_blocks <= kFinInPass; }
+    // With kernel timing on it is a launch of its own, with the same bits, so that both are timed.
+    bool fin_in_pass() const { return row_blocks <= kFinInPass && !ktime; }
     bool enqueue_stats() {
         if (rec_rows) return true;  // a batched round finalizes all problems at once
         if (!fin_in_pass()) {

@@ -384,7 +384,8 @@ int fullmag_fdm_backend_fft_shape(fullmag_fdm_backend *handle, uint32_t *out_px,
  * disabling resets the totals.  kernel_times fills n_kinds entries in the order
  * row pass, y forward, z convolve, y inverse, fused y+z, thin-film y, statistics
  * finalize, extra-field pass: total milliseconds and launch counts since timing was
- * enabled. */
+ * enabled.  With timing on, the statistics are always reduced by a launch of their own
+ * (without it the row pass of a small grid reduces them itself, with the same bits). */
 int fullmag_fdm_backend_set_kernel_timing(fullmag_fdm_backend *handle, int enable);
 int fullmag_fdm_backend_kernel_times(fullmag_fdm_backend *handle, double *total_ms, uint64_t *counts, uint32_t n_kinds);
 

@@ -37,3 +37,18 @@ def test_sums_at_any_number_of_ctas(gpu_lib, monkeypatch, rows, integrator):
         be.close()
     for a, b in zip(*got):
         compare(a, b, 1e-10)
+
+
+@pytest.mark.parametrize("rows,integrator", [(20, _abi.INTEGRATOR_HEUN), (20, _abi.INTEGRATOR_DP45), (600, _abi.INTEGRATOR_RK4)])
+def test_kernel_timing_covers_the_reduction(gpu_lib, rows, integrator):
+    kw = problem(8, rows, 1, seed=92)
+    kw.update(integrator=integrator, adaptive_max_error=1e-3, adaptive_dt_max=5e-14)
+    plain, timed = FdmBackend(**kw), FdmBackend(**kw)
+    timed.set_kernel_timing(True)
+    for n in range(1, 4):
+        a, b = plain.step(5e-14), timed.step(5e-14)
+        assert [a[k] for k in ENERGIES + MAXIMA] == [b[k] for k in ENERGIES + MAXIMA]  # the same bits
+        ms, count = timed.kernel_times()["finalize_stats"]
+        assert count == n and ms > 0
+    plain.close()
+    timed.close()
