@@ -481,6 +481,8 @@ __device__ __forceinline__ void store_lines64(double2 *__restrict__ dst, size_t 
 }
 
 constexpr int kTC = 128;  // threads of a column pass
+// Line strides: one element of padding against bank conflicts, where shared memory holds it
+__host__ __device__ inline int conv_ls64(int len) { return (size_t)6 * sizeof(double2) * (len + 1) <= kMaxSmem ? len + 1 : len; }
 __host__ __device__ inline int y_ls64(const Conv64 &C, int tx) { return C.py + (tx > 1 ? 1 : 0); }  // one line fills the limit
 
 // X[c][z][y < ny][kx] -> Y[c][z][ky][kx]
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(kTC) convolve64(const Col64 P) {
     if (P.early) pdl_trigger();
     extern __shared__ double2 sm64[];
     const Conv64 &C = P.C;
-    const int L = THIN ? C.py : C.pz, cnt = THIN ? C.ny : C.nz, ls = L + 1;
+    const int L = THIN ? C.py : C.pz, cnt = THIN ? C.ny : C.nz, ls = conv_ls64(L);
     const bool prune = (THIN ? C.yprune : C.zprune) != 0;
     const Plan64 &pl = THIN ? C.ply : C.plz;
     const int kx0 = blockIdx.x * P.tx, ncol = min(P.tx, C.nkx - kx0), ky = THIN ? 0 : blockIdx.y;
@@ -1111,7 +1113,7 @@ struct Fp64Engine {
         }
         return !fail("demag column passes", e);
     }
-    size_t conv_smem(int tx) const { return sizeof(double2) * 6 * (size_t)tx * ((conv.thin ? conv.py : conv.pz) + 1); }
+    size_t conv_smem(int tx) const { return sizeof(double2) * 6 * (size_t)tx * conv_ls64(conv.thin ? conv.py : conv.pz); }
     size_t y_smem(int tx) const { return sizeof(double2) * 2 * (size_t)tx * y_ls64(conv, tx); }
     size_t row_smem(int r, int l) const {
         if (!demag) return 0;
