@@ -82,8 +82,9 @@ __device__ __forceinline__ void ff_add(float &hi, float &lo, float v) {
     lo += e;
 }
 __host__ __device__ constexpr int skewed_len(int n) {
-    // odd, so that neighbouring lines start in different banks
-    return (n + (n >> 4) + 1) | 1;
+    // odd, so that neighbouring lines start in different banks; lines of which one column fills the
+    // shared memory keep the last element instead (a film of 4557 periodic rows needs it)
+    return (n + (n >> 4) + 1) | (n <= 4096 ? 1 : 0);
 }
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {

@@ -1,5 +1,5 @@
 """Periodic lines that fill the shared memory of a CTA to the last element: the longest odd film
-and z lines of the double-precision path."""
+and z lines of the double-precision path, the longest odd film line of the single-precision one."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("shape,periodic,precision,tol", [
     ((3, 2421, 1), (0, 1, 0), _abi.PRECISION_DOUBLE, 1e-9),
-    ((2, 2, 2421), (0, 0, 1), _abi.PRECISION_DOUBLE, 1e-9)])
+    ((2, 2, 2421), (0, 0, 1), _abi.PRECISION_DOUBLE, 1e-9),
+    # FP32: 3 log2 N roundings of 2^-24 per axis and direction, and the tensor's own
+    ((4, 4557, 1), (0, 1, 0), _abi.PRECISION_SINGLE, 1e-6)])
 def test_fields(gpu_lib, oracle, shape, periodic, precision, tol):
     kw = problem(*shape, seed=95)
     images = tuple(1 if p else 0 for p in periodic)
