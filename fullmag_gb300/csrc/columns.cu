@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(kThreads) y_forward_kernel(const ColPass p) {
 }
 
 // Y[c][z][ky][kx] -> X[c][z][y<ny][kx] (inverse along y, only physical rows kept)
-__global__ void __launch_bounds__(kThreads) y_inverse_kernel(const ColPass p) {
+// (two CTAs named: columns_conv.cu; the forward pass loads in batches and needs no such help)
+__global__ void __launch_bounds__(kThreads, 2) y_inverse_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem[];

@@ -12,12 +12,16 @@ FM_LENGTHS_TO_256(FM_DECLARE) FM_LENGTHS_LONG(FM_DECLARE)
 
 namespace {
 
-__global__ void __launch_bounds__(kThreads) yz_convolve_general_kernel(const ColPass p) {
+// The general passes wait for shared memory and twiddles; with two CTAs named (what their buffers
+// leave room for) the compiler keeps the loads of a radix-16 butterfly in flight together, in 96
+// registers, instead of 54 to 64 (y+z of 60x45x6: 24.7 -> 22.8 us, y inverse of 30x600x30 in
+// columns.cu: 69.6 -> 61.3 us per launch).
+__global__ void __launch_bounds__(kThreads, 2) yz_convolve_general_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     yz_convolve_general_body(p, blockIdx.x);
 }
-__global__ void __launch_bounds__(kThreads) y_convolve_2d_general_kernel(const ColPass p) {
+__global__ void __launch_bounds__(kThreads, 2) y_convolve_2d_general_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     y_convolve_2d_general_body(p, blockIdx.x);
