@@ -37,6 +37,8 @@ static constexpr double kMu0 = 4.0 * M_PI * 1e-7;
 // five sums (ExtraSums: Zeeman m.(H_ext + H_map), DMI,
 // uniaxial and cubic energy densities, region exchange pair sum)
 static constexpr int kStatSlots = kNumStats + 6;
+// shared memory of a CTA that the choice of tiles stays within
+static constexpr size_t kTileSmem = 200u * 1024u;
 
 bool newell_spectrum_gpu(const Grid &g, double dx, double dy, double dz, double ms, float *kern, cudaStream_t s,
                          std::string &err);
@@ -2073,7 +2075,7 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
         Grid t = g;
         t.py = pow2_extent(2 * g.ny - 1);
         t.pz = pow2_extent(2 * g.nz - 1);
-        if (yz_convolve_smem(t, 1) <= 200u * 1024u) {
+        if (yz_convolve_smem(t, 1) <= kTileSmem) {
             g.py = t.py;
             g.pz = t.pz;
         }
@@ -2081,7 +2083,7 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     if (g.px < 2) g.px = 2;
     g.half = g.px / 2;
     g.nkx = g.half + 1;
-    g.xs = x_pitch(g.nkx);
+    g.xs = demag && thin && y_convolve_2d_smem(g, 2) > kTileSmem ? g.nkx : x_pitch(g.nkx);
     g.nky = g.py / 2 + 1;
     g.nkz = g.pz / 2 + 1;
     grid_dividers(g);
@@ -2547,14 +2549,14 @@ bool Engine::autotune() {
         if (g.thin) {
             std::vector<std::pair<int, float>> cand;
             for (int tx : {1, 2, 4, 8, 16}) {
-                if (tx > std::max(1, g.nkx) || y_convolve_2d_smem(g, tx) > 200u * 1024u) continue;
+                if (tx > std::max(1, g.nkx) || y_convolve_2d_smem(g, tx) > kTileSmem) continue;
                 cand.emplace_back(tx, time_ms([&] { return launch_y_convolve_2d(col_pass(plan_y, tx, X, X), stream) == cudaSuccess; }));
             }
             tx_2d = pick_tile(cand, tx_2d, g.nkx);
         } else if (use_yz) {
             std::vector<std::pair<int, float>> cand;
             for (int tx : {1, 2, 4, 8}) {
-                if (tx > std::max(1, g.nkx) || yz_convolve_smem(g, tx) > 200u * 1024u) continue;
+                if (tx > std::max(1, g.nkx) || yz_convolve_smem(g, tx) > kTileSmem) continue;
                 cand.emplace_back(tx, time_ms([&] { return launch_yz_convolve(col_pass(plan_y, tx, X, X), stream) == cudaSuccess; }));
             }
             tx_z = pick_tile(cand, tx_z, g.nkx);
@@ -2568,7 +2570,7 @@ bool Engine::autotune() {
                 float bt = 1e30f;
                 for (int sp = 0; sp < (alt ? 2 : 1); ++sp)
                     for (int tx : {1, 2, 4, 8, 16}) {
-                        if (tx > std::max(1, g.nkx) || smem(tx) > 200u * 1024u) continue;
+                        if (tx > std::max(1, g.nkx) || smem(tx) > kTileSmem) continue;
                         const float t = time_ms([&] { return run(tx, sp); });
                         if (t < bt) {
                             bt = t;
@@ -2632,7 +2634,7 @@ bool Engine::autotune() {
             p.comb_k[0] = nullptr;
             p.comb_c[0] = 0.f;
             p.x_out = demag ? X : nullptr;
-            if (row_pass_smem(p) > 200u * 1024u) continue;
+            if (row_pass_smem(p) > kTileSmem) continue;
             cand.emplace_back(rows, time_ms([&] { return launch_row_pass(p, stream) == cudaSuccess; }));
         }
         row_rows = pick_tile(cand, row_rows, nrows);

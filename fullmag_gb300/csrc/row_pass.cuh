@@ -85,7 +85,7 @@ __device__ __forceinline__ void row_inverse_x(const RowPass &p, int rows, int ro
     for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
         const int line = it / N1, k1 = it % N1;
         const int rr = line / 3, c = line - 3 * rr;
-        const float2 *X = p.x_in + ((size_t)c * nrows + row0 + rr) * x_pitch(nkx);
+        const float2 *X = p.x_in + ((size_t)c * nrows + row0 + rr) * g.xs;
         float2 v[N2];
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
@@ -193,7 +193,7 @@ __device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int ro
         const float2 b = cconj(zl[sk(k == 0 ? 0 : half - k)]);
         const float2 E = cscale(cadd(a, b), 0.5f);
         const float2 O = div2i(csub(a, b));
-        p.x_out[((size_t)c * nrows + row0 + rr) * x_pitch(nkx) + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
+        p.x_out[((size_t)c * nrows + row0 + rr) * g.xs + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
     }
 }
 
@@ -556,7 +556,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
             [&](int idx) {
                 const int line = g.fd_nkx.div(idx), k = idx - line * nkx;
                 const int rr = line / 3, c = line - 3 * rr;
-                return p.x_in[((size_t)c * nrows + row0 + rr) * x_pitch(nkx) + k];
+                return p.x_in[((size_t)c * nrows + row0 + rr) * g.xs + k];
             },
             [&](int idx, float2 v) {
                 const int line = g.fd_nkx.div(idx), k = idx - line * nkx;
@@ -941,7 +941,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
             const float2 b = cconj(zl[sk(k == 0 ? 0 : half - k)]);
             const float2 E = cscale(cadd(a, b), 0.5f);
             const float2 O = div2i(csub(a, b));
-            p.x_out[((size_t)c * nrows + row0 + rr) * x_pitch(nkx) + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
+            p.x_out[((size_t)c * nrows + row0 + rr) * g.xs + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
         }
     }
 }
