@@ -56,13 +56,17 @@ cudaError_t launch_yz_convolve(const ColPass &p, cudaStream_t s) {
 
 size_t y_convolve_2d_smem(const Grid &g, int tx) {
     const size_t one = sizeof(float2) * (size_t)3 * tx * skewed_len(g.py);
-    return y2d_fused_ok(g) ? one : 2 * one;
+    return y2d_two_level(g) ? one : 2 * one;
+}
+size_t y_convolve_2d_batched_smem(const Grid &g, int tx) {
+    const size_t one = sizeof(float2) * (size_t)3 * tx * skewed_len(g.py);
+    return y2d_fused_ok(g) && !g.per ? one : 2 * one;
 }
 
 cudaError_t launch_y_convolve_2d(const ColPass &p, cudaStream_t s) {
     const size_t sm = y_convolve_2d_smem(p.g, p.tx);
     const ConvKernels &k = conv_kernels_for(p.g.py);
-    const ColKernel fn = !y2d_fused_ok(p.g) ? y_convolve_2d_general_kernel
+    const ColKernel fn = !y2d_two_level(p.g) ? y_convolve_2d_general_kernel
                          : (p.g.per & 2)    ? k.film_full
                          : p.g.per          ? k.film_per
                                             : k.film;

@@ -349,6 +349,15 @@ __host__ __device__ __forceinline__ bool y2d_fused_ok(const Grid &g) {
     return two_level_length(g.py) && ((g.per & 2) ? g.ny == g.py : 2 * g.ny <= g.py);
 }
 
+// ... and is the better one for a film alone: not for long lines (film_y_long, engine.h) of no more kx
+// columns than one wave of CTAs.  The two-level form of these lengths holds 3 x 28 to 3 x 32
+// complex values a thread and is one long chain; a CTA per column has its time whatever the
+// other SMs do.  us per launch, two-level / general at 1024: ny = 500, nx = 8: 18.5 / 16.1, nx = 100:
+// 19.4 / 17.2, nx = 150 (161 columns): 20.5 / 22.4, nx = 300: 22.5 / 32.9.
+__host__ __device__ __forceinline__ bool y2d_two_level(const Grid &g) {
+    return y2d_fused_ok(g) && !(film_y_long(g.py, (g.per & 2) != 0) && g.nkx <= kFilmWave);
+}
+
 // Thin film, any py: Stockham transforms in shared memory.
 __device__ __forceinline__ void y_convolve_2d_general_body(const ColPass &p, const int tile) {
     extern __shared__ __align__(16) unsigned char smem[];

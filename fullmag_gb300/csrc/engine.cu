@@ -498,6 +498,7 @@ struct Engine {
     }
 
     bool use_gpu_newell = false;
+    bool batch_member = false;  // set before setup
     // small fixed-step problems: each kernel lets the next one launch as soon as its own
     // last CTAs have started (programmatic dependent launch, engine.h)
     bool early_launch = false;
@@ -535,8 +536,13 @@ struct Engine {
     }
     // x: the half length is the one transformed
     static int pad_x(int nx) { return 2 * pad_extent(nx); }
-    // y of a 3-D grid: at least the shortest two-level length (the fused y+z pass)
-    static int pad_y(int ny, bool thin) { return thin ? pad_extent(2 * ny - 1) : std::max(16, pad_extent(2 * ny - 1)); }
+    // y of a 3-D grid: at least the shortest two-level length (the fused y+z pass); of a film of
+    // few columns alone: the power of two where the general pass is the faster (film_y_long)
+    int pad_y(int ny, bool thin) const {
+        const int n = pad_extent(2 * ny - 1);
+        if (!thin) return std::max(16, n);
+        return film_y_long(n, false) && g.px / 2 + 1 <= kFilmWave && !batch_member ? pow2_extent(n) : n;
+    }
     // z: every even length up to 16 (the register z passes take them); beyond those, the
     // z pass over the periodic kernel is the general one, fast at powers of two only
     static int pad_z(int nz, bool periodic) {
@@ -1649,7 +1655,7 @@ struct Engine {
         }
         if (!demag) return;
         int tx = 1;
-        auto smem = [&](int t) { return g.thin ? y_convolve_2d_smem(g, t) : yz_convolve_smem(g, t); };
+        auto smem = [&](int t) { return g.thin ? y_convolve_2d_batched_smem(g, t) : yz_convolve_smem(g, t); };
         while (tx < 16 && 2 * tx <= g.nkx && smem(2 * tx) <= 96u * 1024u) tx *= 2;
         if (g.thin) tx_2d = std::max(tx_2d, tx);
         else if (use_yz) tx_z = std::max(tx_z, tx);
@@ -3572,7 +3578,7 @@ struct FdmBatch {
             if (e->demag) {
                 const bool thin = e->g.thin != 0;
                 const int tx = thin ? e->tx_2d : e->tx_z;
-                ch.col_smem = std::max(ch.col_smem, thin ? y_convolve_2d_smem(e->g, tx) : yz_convolve_smem(e->g, tx));
+                ch.col_smem = std::max(ch.col_smem, thin ? y_convolve_2d_batched_smem(e->g, tx) : yz_convolve_smem(e->g, tx));
                 ColPass c = e->col_pass(e->plan_y, tx, e->X, e->X);
                 c.skip_dt = &round.d_ctl[k].dt;
                 const int ntiles = (e->g.nkx + tx - 1) / tx;
@@ -3708,6 +3714,7 @@ fullmag_fdm_batch *fullmag_fdm_batch_create(const fullmag_fdm_plan_desc *plans, 
             break;
         }
         b->items.push_back(e);
+        e->batch_member = true;
         if (!e->setup(&plans[i]) || !e->upload<double>(plans[i].initial_magnetization_xyz) || !e->eval_state(false)) {
             b->last_error = "problem " + std::to_string(i) + ": " + e->last_error;
             break;
