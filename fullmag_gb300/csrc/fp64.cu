@@ -958,21 +958,35 @@ int pad_extent64(int n) {
     return best;
 }
 
-// One FP64 line of length p per CTA along an axis of layout [outer][p][inner] (real
-// input in_re with zero imaginary part, or complex c_in), forward transform
-// e^{-2 pi i k a / p}, the first nout outputs written to out[outer][nout][inner].
+__host__ __device__ inline int axis_ls64(int p, int nl) { return p + (nl > 1 ? 1 : 0); }
+
+// FP64 lines of length p along an axis of layout [outer][p][inner] (real input in_re with zero
+// imaginary part, or complex c_in), nl per CTA: forward transform e^{-2 pi i k a / p}, the first
+// nout outputs written to out[outer][nout][inner].  One line of 64 points has eight radix-8
+// butterflies for 128 threads; with up to 16 lines a CTA every thread has one, and neighbouring
+// lines are read together (periodic tensor of 128x128x30: create 5.2 -> 3.9 ms).
 __global__ void fft_axis64_kernel(const double *__restrict__ in_re, const double2 *__restrict__ c_in,
-                                  double2 *__restrict__ out, int p, int nout, int inner, const Plan64 plan) {
+                                  double2 *__restrict__ out, int p, int nout, int inner, unsigned lines, int nl,
+                                  const Plan64 plan) {
     extern __shared__ double2 sm64[];
-    double2 *a = sm64, *b = sm64 + p;
-    const long long line = blockIdx.x;
-    const long long o = line / inner, q = line - o * inner;
-    const long long base = o * p * inner + q;
-    for (int i = threadIdx.x; i < p; i += blockDim.x)
-        a[i] = in_re ? make_double2(in_re[base + (long long)i * inner], 0.0) : c_in[base + (long long)i * inner];
+    const int ls = axis_ls64(p, nl);
+    double2 *a = sm64, *b = sm64 + nl * ls;
+    const unsigned line0 = blockIdx.x * (unsigned)nl;
+    const int n = (int)min((unsigned)nl, lines - line0);
+    for (int idx = threadIdx.x; idx < n * p; idx += blockDim.x) {
+        // neighbouring threads on neighbouring addresses: along the line, or across the lines
+        const int l = inner == 1 ? idx / p : idx % n, i = inner == 1 ? idx - l * p : idx / n;
+        const unsigned o = (line0 + l) / inner, q = line0 + l - o * inner;
+        const long long at = ((long long)o * p + i) * inner + q;
+        a[l * ls + i] = in_re ? make_double2(in_re[at], 0.0) : c_in[at];
+    }
     __syncthreads();
-    const double2 *r = fft_lines64<false>(a, b, 1, p, plan, false);
-    for (int k = threadIdx.x; k < nout; k += blockDim.x) out[(o * nout + k) * inner + q] = r[k];
+    const double2 *r = fft_lines64<false>(a, b, n, ls, plan, false);
+    for (int idx = threadIdx.x; idx < n * nout; idx += blockDim.x) {
+        const int l = inner == 1 ? idx / nout : idx % n, k = inner == 1 ? idx - l * nout : idx / n;
+        const unsigned o = (line0 + l) / inner, q = line0 + l - o * inner;
+        out[((long long)o * nout + k) * inner + q] = r[l * ls + k];
+    }
 }
 
 }  // namespace
@@ -983,8 +997,12 @@ bool fft64_axis(const double *in_re, const double2 *c_in, double2 *out, long lon
     std::vector<size_t> off;
     Plan64 plan;
     if (!make_plan64(p, tw, off, plan)) return err = "FFT length has too many factors", false;
-    const size_t smem = sizeof(double2) * 2 * (size_t)p;
-    if (smem > 227 * 1024) return err = "FFT length too large for the double-precision lines", false;
+    const long long lines = outer * inner;
+    if (sizeof(double2) * 2 * (size_t)p > kMaxSmem) return err = "FFT length too large for the double-precision lines", false;
+    int nl = 16;
+    auto bytes = [&](int k) { return sizeof(double2) * 2 * (size_t)k * axis_ls64(p, k); };
+    while (nl > 1 && (bytes(nl) > 48 * 1024 || lines / nl < 304)) nl /= 2;
+    const size_t smem = bytes(nl);
     double2 *dtw = nullptr;
     cudaError_t e = cudaMalloc(&dtw, sizeof(double2) * tw.size());
     if (e == cudaSuccess) e = cudaMemcpyAsync(dtw, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice, s);
@@ -992,8 +1010,8 @@ bool fft64_axis(const double *in_re, const double2 *c_in, double2 *out, long lon
         e = cudaFuncSetAttribute((const void *)fft_axis64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) {
         plan.tw = dtw;
-        const long long lines = outer * inner;
-        fft_axis64_kernel<<<(unsigned)lines, 128, smem, s>>>(in_re, c_in, out, p, nout, inner, plan);
+        fft_axis64_kernel<<<(unsigned)((lines + nl - 1) / nl), 128, smem, s>>>(in_re, c_in, out, p, nout, inner,
+                                                                               (unsigned)lines, nl, plan);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
