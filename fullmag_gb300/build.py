@@ -25,7 +25,10 @@ GROUPS = range(9)
 PLAIN_SOURCES = ["plain_baseline.cu"]
 PLAIN_LIB = OUT / "libfullmag_fdm_plain.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
+# Kernels are stored uncompressed: the first use of a length in a process loads its module, and
+# unpacking the y passes' took 12 ms of the 22 ms of a first create (150x150x10 disk; 9.7 ms so;
+# the library grows from 120 to 151 MB).
+FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--compress-mode=none"]
 
 
 def nvcc() -> str:
