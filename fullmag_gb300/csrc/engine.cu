@@ -445,6 +445,7 @@ struct Engine {
 
     bool cuda_fail(const char *what, cudaError_t e) {
         if (e == cudaSuccess) return false;
+        cudaGetLastError();  // reported here: the next check is not to find it again
         last_error = std::string(what) + ": " + cudaGetErrorString(e);
         return true;
     }

@@ -1082,6 +1082,7 @@ struct Fp64Engine {
 
     bool fail(const char *what, cudaError_t e) {
         if (e == cudaSuccess) return false;
+        cudaGetLastError();  // reported here: the next check is not to find it again
         err = std::string(what) + ": " + cudaGetErrorString(e);
         return true;
     }

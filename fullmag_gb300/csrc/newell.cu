@@ -196,6 +196,7 @@ unsigned grid_for(long long n) { return (unsigned)std::min<long long>((n + 255) 
 
 static bool ck(cudaError_t e, const char *what, std::string &err) {
     if (e == cudaSuccess) return true;
+    cudaGetLastError();  // reported here: the next check is not to find it again
     err = std::string(what) + ": " + cudaGetErrorString(e);
     return false;
 }
