@@ -2470,14 +2470,14 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
 }
 
 namespace {
-// Everything the search depends on: the shape, the column passes that run (yz), the tile rule of
-// early launch, which follows the integrator, and the choices forced through the environment.
+// Everything the search depends on: the shape, the column passes that run (demag, yz), the tile
+// rule of early launch, which follows the integrator, and the choices forced through the environment.
 struct TuneKey {
-    int nx, ny, nz, px, py, pz, thin, masked, per, yz, early, z_forced, rows_forced;
-    bool operator<(const TuneKey &o) const {
-        return std::tie(nx, ny, nz, px, py, pz, thin, masked, per, yz, early, z_forced, rows_forced) <
-               std::tie(o.nx, o.ny, o.nz, o.px, o.py, o.pz, o.thin, o.masked, o.per, o.yz, o.early, o.z_forced, o.rows_forced);
+    int nx, ny, nz, px, py, pz, thin, masked, per, demag, yz, early, z_forced, rows_forced;
+    auto tied() const {
+        return std::tie(nx, ny, nz, px, py, pz, thin, masked, per, demag, yz, early, z_forced, rows_forced);
     }
+    bool operator<(const TuneKey &o) const { return tied() < o.tied(); }
 };
 struct TuneChoice {
     int tx_yf, tx_z, tx_yi, tx_2d, rows, z_pair, split_yf, split_z, split_yi;
@@ -2494,8 +2494,8 @@ bool Engine::autotune() {
     // FULLMAG_FDM_Z_PAIR=0 or 1 forces the choice of the packed z pass
     const char *zp_env = std::getenv("FULLMAG_FDM_Z_PAIR"), *rows_env = std::getenv("FULLMAG_FDM_ROWS_PER_CTA");
     const int z_forced = zp_env && (zp_env[0] == '0' || zp_env[0] == '1') ? zp_env[0] - '0' : -1;
-    const TuneKey key{g.nx, g.ny,  g.nz,           g.px, g.py, g.pz, g.thin, has_mask ? 1 : 0,
-                      g.per, use_yz, early_launch, z_forced, rows_env ? row_rows : 0};
+    const TuneKey key{g.nx, g.ny, g.nz, g.px, g.py, g.pz, g.thin, has_mask ? 1 : 0, g.per, demag ? 1 : 0, use_yz ? 1 : 0,
+                      early_launch ? 1 : 0, z_forced, rows_env ? row_rows : 0};
     // FULLMAG_FDM_TUNE="rows,tx_yf,tx_z,tx_yi,tx_2d,z_pair,split_yf,split_z,split_yi" fixes every
     // choice (the values fullmag_fdm_backend_tuning reports), e.g. so that a profiler run uses
     // the launch shapes of an unprofiled one

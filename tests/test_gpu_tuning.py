@@ -8,8 +8,8 @@ from helpers import problem
 pytestmark = pytest.mark.gpu
 
 
-def make(nx, ny, nz):
-    return FdmBackend(**problem(nx, ny, nz, seed=81), integrator=_abi.INTEGRATOR_RK4)
+def make(nx, ny, nz, **terms):
+    return FdmBackend(**problem(nx, ny, nz, seed=81, **terms), integrator=_abi.INTEGRATOR_RK4)
 
 
 def test_three_passes_after_the_fused_pass(gpu_lib, monkeypatch):
@@ -21,6 +21,12 @@ def test_three_passes_after_the_fused_pass(gpu_lib, monkeypatch):
     be.refresh()
     assert be.kernel_times()["z_convolve"][1] == 1 and be.kernel_times()["yz_convolve"][1] == 0
     be.close()
+
+
+def test_z_pass_after_a_problem_without_demag(gpu_lib, monkeypatch):
+    monkeypatch.setenv("FULLMAG_FDM_Z_PAIR", "1")
+    assert make(16, 512, 20, enable_demag=False).tuning()["z_pair"] == 0  # same extents, no z pass
+    assert make(16, 512, 20).tuning()["z_pair"] == 1
 
 
 # pz 32 to 128; the plane of 260 rows does not fit the fused pass
