@@ -2645,6 +2645,13 @@ bool Engine::autotune() {
             cand.emplace_back(rows, time_ms([&] { return launch_row_pass(p, stream) == cudaSuccess; }));
         }
         row_rows = pick_tile(cand, row_rows, nrows);
+        // of near-equals on a large grid the most rows: the pass with statistics, not timed here, has
+        // fewer partials then (256x256x64 without demag: 62.3 us at 4 rows, 63.7 at 8 for this pass,
+        // 190 and 178 us a Heun step)
+        float bt = 1e30f;
+        for (const auto &c : cand) bt = std::min(bt, c.second);
+        for (const auto &c : cand)
+            if (!early_launch && c.second <= 1.03f * bt && c.first > row_rows && nrows / c.first > kFinInPass) row_rows = c.first;
     }
     row_blocks = (g.ny * g.nz + row_rows - 1) / row_rows;
     // the timed launches only wrote scratch (X, Y, A[0], K[0], partials); every one of
