@@ -514,12 +514,6 @@ struct Engine {
         for (int q : {2, 3, 5, 7}) while (m % q == 0) m /= q;
         return m == 1;
     }
-    static int next_smooth(int n, bool even) {
-        for (int m = std::max(n, 1);; ++m) {
-            if (even && (m & 1)) continue;
-            if (smooth_enough(m)) return m;
-        }
-    }
     // Padded extent >= n when the engine builds the tensor: the next power of two, or the
     // next length of the two-level transforms (two_level_length) where there is one.  They
     // run at the speed per point of the powers of two, several times faster than the runtime
@@ -2025,7 +2019,8 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     // With caller spectra the padded grid is the reference's (2nx, 2ny, 2nz) or, for
     // nz == 1 and 2-D spectra, (2nx, 2ny).  When the engine builds the tensor itself
     // any extent p >= 2n - 1 keeps the circular convolution exact on the physical
-    // cells, so awkward sizes are rounded up to 2,3,5,7-smooth FFT lengths.
+    // cells, so every extent is rounded up to a length of the two-level transforms or a power
+    // of two (pad_extent).
     bool thin = false;
     use_gpu_newell = false;
     g.px = 2 * g.nx;
@@ -2066,7 +2061,7 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
                 return false;
             }
             // the given spectra fix P = 2n; lengths with a prime factor the shared-memory
-            // FFT does not handle are rebuilt on the GPU at smooth extents instead
+            // FFT does not handle are rebuilt on the GPU at those extents instead
             if (!smooth_enough(2 * g.nx) || !smooth_enough(2 * g.ny) || (!thin && !smooth_enough(2 * g.nz)))
                 use_gpu_newell = true;
         }
@@ -3346,10 +3341,10 @@ int fullmag_fdm_backend_fft_shape(fullmag_fdm_backend *handle, uint32_t *out_px,
 // Batched sweeps: many independent problems of uneven size
 // =====================================================================
 
-// One round of a batched sweep: the attempt of every member problem, executed as
-// 7 batched row passes + 6 batched column passes (one launch per pass and column
-// kind for all problems, through (problem, block) work tables) + one batched
-// finalize, captured once as a CUDA graph and replayed every round.
+// One round of a batched sweep: the attempt of every member problem, executed as 7 batched row
+// passes + 6 batched column passes through (problem, block) work tables, the batched finalize
+// and the step control, on independent chains of problems (build_round), captured once as a CUDA
+// graph and replayed every round.
 struct BatchRound {
     std::vector<size_t> members;
     BatchCtl *h_ctl = nullptr;  // pinned [n]
@@ -3743,12 +3738,9 @@ uint32_t fullmag_fdm_batch_size(fullmag_fdm_batch *batch) {
     return batch ? (uint32_t)reinterpret_cast<FdmBatch *>(batch)->items.size() : 0u;
 }
 
-// Batched-kernel path (all problems DP45 and small enough for the fused column
-// passes).  Each round replays one graph for all unfinished problems, waits once,
-// then applies the accept/reject rule per problem on the host.  Problems that reached
-// t_end stay in the round's work tables with step size 0, which makes their row and
-// column CTAs return at once, until the round is rebuilt without them (when a tenth
-// of its members have finished).  Returns 1 when not batchable.
+// Batched-kernel path (all problems DP45 and small enough for the fused column passes; returns
+// 1 when they are not).  Problems that reached t_end stay in the round's work tables with step
+// size 0, which makes their row and column CTAs return at once.
 // Batched DP45 rounds: each look at the state follows up to BatchRound::kRounds rounds with the step
 // control on the device (batch_control_kernel); the host reads the control state after them
 // to see which problems reached t_end, and rebuilds the round for the remaining
