@@ -51,6 +51,10 @@ __device__ __forceinline__ float2 mul_i(float2 a) { return make_float2(-a.y, a.x
 
 __device__ __forceinline__ bool cell_active(const uint8_t *mask, long long i) { return mask == nullptr || mask[i] != 0; }
 
+// start of spectrum row r (component, row) in X: a widening product of 32-bit factors, since the
+// pitch is the grid's (a 64-bit one made the stages of x half length 1024 2 % slower)
+__device__ __forceinline__ size_t x_row(const Grid &g, int r) { return (size_t)(unsigned)r * (unsigned)g.xs; }
+
 // ---- x-transforms in the two-level form (half = px/2 = N1 * N2) ----
 // The real x line of length px is carried as the half-length complex line
 // z[j] = s[2j] + i s[2j+1].  On an open x its nonzero samples are j < half/2 and only those
@@ -85,7 +89,7 @@ __device__ __forceinline__ void row_inverse_x(const RowPass &p, int rows, int ro
     for (int it = threadIdx.x; it < nl * N1; it += blockDim.x) {
         const int line = it / N1, k1 = it % N1;
         const int rr = line / 3, c = line - 3 * rr;
-        const float2 *X = p.x_in + ((size_t)c * nrows + row0 + rr) * g.xs;
+        const float2 *X = p.x_in + x_row(g, c * nrows + row0 + rr);
         float2 v[N2];
 #pragma unroll
         for (int k2 = 0; k2 < N2; ++k2) {
@@ -193,7 +197,7 @@ __device__ __forceinline__ void row_forward_x(const RowPass &p, int rows, int ro
         const float2 b = cconj(zl[sk(k == 0 ? 0 : half - k)]);
         const float2 E = cscale(cadd(a, b), 0.5f);
         const float2 O = div2i(csub(a, b));
-        p.x_out[((size_t)c * nrows + row0 + rr) * g.xs + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
+        p.x_out[x_row(g, c * nrows + row0 + rr) + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
     }
 }
 
@@ -556,7 +560,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
             [&](int idx) {
                 const int line = g.fd_nkx.div(idx), k = idx - line * nkx;
                 const int rr = line / 3, c = line - 3 * rr;
-                return p.x_in[((size_t)c * nrows + row0 + rr) * g.xs + k];
+                return p.x_in[x_row(g, c * nrows + row0 + rr) + k];
             },
             [&](int idx, float2 v) {
                 const int line = g.fd_nkx.div(idx), k = idx - line * nkx;
@@ -941,7 +945,7 @@ __device__ __forceinline__ void row_pass_body(const RowPass &p, const int bid, c
             const float2 b = cconj(zl[sk(k == 0 ? 0 : half - k)]);
             const float2 E = cscale(cadd(a, b), 0.5f);
             const float2 O = div2i(csub(a, b));
-            p.x_out[((size_t)c * nrows + row0 + rr) * g.xs + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
+            p.x_out[x_row(g, c * nrows + row0 + rr) + k] = cadd(E, cmul(__ldg(p.xpost + k), O));
         }
     }
 }
