@@ -317,6 +317,11 @@ cudaError_t launch_y_inverse(const ColPass &p, cudaStream_t s) {
     return launch_pdl(y_inverse_kernel, dim3(tiles(p), p.g.nz, 3), dim3(kThreads), sm, s, p);
 }
 
+cudaError_t load_finalize_stats() {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, (const void *)finalize_stats_kernel);
+}
+
 cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early) {
     return launch_pdl(finalize_stats_kernel, dim3(1), dim3(kFinThreads), 0, s, partials, nblocks, out, early);
 }

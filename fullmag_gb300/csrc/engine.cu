@@ -3279,6 +3279,7 @@ int fullmag_fdm_backend_set_kernel_timing(fullmag_fdm_backend *handle, int enabl
     Engine *e = eng(handle);
     if (!e || !e->arena) return FULLMAG_FDM_ERR_INVALID;
     if (cudaStreamSynchronize(e->stream) != cudaSuccess) return FULLMAG_FDM_ERR_CUDA;
+    if (enable && e->cuda_fail("finalize kernel", load_finalize_stats())) return FULLMAG_FDM_ERR_CUDA;
     e->kt_collect();
     e->ktime = enable != 0;
     for (int k = 0; k < Engine::KT_N; ++k) {

@@ -311,6 +311,8 @@ cudaError_t launch_col_batched(const ColPass *ps, const int2 *work, int nwork, i
 cudaError_t launch_finalize_batched(const FinDesc *fd, int nproblems, double *out, cudaStream_t s);
 // the nine sums / maxima of nblocks CTAs' partials into out
 cudaError_t launch_finalize_stats(const float2 *partials, int nblocks, double *out, cudaStream_t s, int early = 0);
+// loads its kernel, so that the first timed launch does not
+cudaError_t load_finalize_stats();
 // Most row-pass CTAs whose statistics the last of them reduces; beyond, the reduction is a launch
 // of its own.  Every CTA of a pass that reduces waits for its fence and its count, which a CTA
 // cannot hide: Heun steps without demag, in the pass against a launch: 128 CTAs 20.0 / 23.5 us,
