@@ -2300,7 +2300,11 @@ bool Engine::setup(const fullmag_fdm_plan_desc *plan) {
     tx_2d = col_tile(g, 3, g.py);
     {
         const char *no_yz = std::getenv("FULLMAG_FDM_NO_FUSED_YZ");
-        // beyond pz = 8 the fused pass needs two CTAs per SM to be worth it
+        // beyond pz = 8 the fused pass needs two CTAs per SM to be worth it, in its general form too
+        // (caller spectra; RK4 steps, three passes / fused: 120x60x8 at 107 KB a column 158 / 176 us,
+        // 30x120x6 117 / 197, 32x50x12 101 / 147).  A batch with such a member runs its problems as
+        // single ones side by side (24 and 96 films and one such: a block of 20 rounds 8.7 and 31.2 ms,
+        // with it fused and batched 9.0 and 30.4).
         const size_t yz_limit = (z_register_length_ok(g.pz) && g.pz > 8 ? 100u : 200u) * 1024u;
         use_yz = demag && !thin && !g.per && !(no_yz && *no_yz && *no_yz != '0') && yz_convolve_smem(g, 1) <= yz_limit;
         z_pair = demag && !thin && !use_yz && z_convolve_register_ok(g) ? 2 : 0;

@@ -38,3 +38,22 @@ def test_values_after_every_call(gpu_lib):
     for s in singles:
         s[0].close()
     batch.close()
+
+
+def test_a_member_beyond_the_batched_passes(gpu_lib, oracle):
+    """A caller's 3 x 60 x 8 spectra: a column of that plane takes more shared memory than the fused y+z
+    pass is used for, so the batch runs its problems one by one on their streams."""
+    plans = [dict(problem(*s, seed=60 + i, alpha=0.1), integrator=_abi.INTEGRATOR_DP45, adaptive_max_error=1e-5,
+                  adaptive_dt_max=5e-14) for i, s in enumerate([(3, 60, 8), (17, 9, 1), (12, 20, 4)])]
+    plans[0]["spectra"] = oracle.newell_spectra(3, 60, 8, *[plans[0][k] for k in ("dx", "dy", "dz")])
+    batch = FdmBatch(plans)
+    singles = [[FdmBackend(**kw), 0.0, 5e-14] for kw in plans]
+    assert singles[0][0].fft_shape() == (6, 120, 16)
+    for call, t_end in enumerate((5e-13, 1e-12)):
+        batch.step_until(t_end, 5e-14)
+        for i, s in enumerate(singles):
+            s[1], s[2] = alone(*s, t_end)
+            assert np.abs(batch.copy_field(i) - s[0].copy_field(_abi.OBSERVABLE_M)).max() < 1e-6 * (call + 1), (call, i)
+    for s in singles:
+        s[0].close()
+    batch.close()
