@@ -349,13 +349,13 @@ __host__ __device__ __forceinline__ bool y2d_fused_ok(const Grid &g) {
     return two_level_length(g.py) && ((g.per & 2) ? g.ny == g.py : 2 * g.ny <= g.py);
 }
 
-// ... and is the better one for a film alone: not for long lines (film_y_long, engine.h) of no more kx
-// columns than one wave of CTAs.  The two-level form of these lengths holds 3 x 28 to 3 x 32
-// complex values a thread and is one long chain; a CTA per column has its time whatever the
-// other SMs do.  us per launch, two-level / general at 1024: ny = 500, nx = 8: 18.5 / 16.1, nx = 100:
-// 19.4 / 17.2, nx = 150 (161 columns): 20.5 / 22.4, nx = 300: 22.5 / 32.9.
+// ... and is the better one for a film alone: not for long lines (film_y_long, engine.h) of few kx
+// columns.  The two-level form of these lengths holds 3 x 28 to 3 x 32 complex values a thread and is
+// one long chain, which a few CTAs only wait for; from about 40 columns its fewer instructions count.
+// RK4 steps in one call, us, two-level / general at 1024: ny = 500, nx = 4: 99 / 65, nx = 32: 85 / 73,
+// nx = 48: 84 / 91, nx = 64: 86 / 91; ny = 400: nx = 32: 80 / 68, nx = 48: 81 / 68, nx = 64: 80 / 83.
 __host__ __device__ __forceinline__ bool y2d_two_level(const Grid &g) {
-    return y2d_fused_ok(g) && !(film_y_long(g.py, (g.per & 2) != 0) && g.nkx <= kFilmWave);
+    return y2d_fused_ok(g) && !(film_y_long(g.py, (g.per & 2) != 0) && g.nkx <= kFilmColumns);
 }
 
 // Thin film, any py: Stockham transforms in shared memory.

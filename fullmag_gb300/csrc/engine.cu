@@ -536,7 +536,7 @@ struct Engine {
     int pad_y(int ny, bool thin) const {
         const int n = pad_extent(2 * ny - 1);
         if (!thin) return std::max(16, n);
-        return film_y_long(n, false) && g.px / 2 + 1 <= kFilmWave && !batch_member ? pow2_extent(n) : n;
+        return film_y_long(n, false) && g.px / 2 + 1 <= kFilmColumns && !batch_member ? pow2_extent(n) : n;
     }
     // z: every even length up to 16 (the register z passes take them); beyond those, the
     // z pass over the periodic kernel is the general one, fast at powers of two only

@@ -217,10 +217,10 @@ size_t y_pass_smem(const Grid &g, int tx);
 size_t y_convolve_2d_smem(const Grid &g, int tx);
 size_t y_convolve_2d_batched_smem(const Grid &g, int tx);  // of the pass over many films
 
-// Film y lines whose two-level form is slower than the general one while the kx columns are no
-// more than kFilmWave CTAs (y2d_two_level, columns_conv.cuh): open from 896 points, periodic (full
-// lines) at 512 and from 896.
-constexpr int kFilmWave = 152;
+// Film y lines whose two-level form is slower than the general one while the kx columns are no more
+// than kFilmColumns (y2d_two_level, columns_conv.cuh): open from 896 points, periodic (full lines) at
+// 512 and from 896.
+constexpr int kFilmColumns = 40;
 __host__ __device__ constexpr bool film_y_long(int py, bool periodic) { return py >= 896 || (periodic && py == 512); }
 
 // Field terms computed by a pass of their own before each right-hand-side row pass

@@ -13,10 +13,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nx,ny,periodic,py", [
-    (8, 440, None, 1024), (128, 448, None, 1024), (130, 448, None, 896), (128, 512, None, 1024), (130, 500, None, 1024),
-    (8, 380, None, 768), (32, 450, (1, 0, 0), 1024), (320, 440, (1, 0, 0), 896),
-    (8, 512, (0, 1, 0), 512), (256, 512, (1, 1, 0), 512), (320, 512, (1, 1, 0), 512), (300, 896, (1, 1, 0), 896),
-    (320, 896, (1, 1, 0), 896), (16, 1024, (1, 1, 0), 1024), (320, 1024, (1, 1, 0), 1024),
+    (8, 440, None, 1024), (32, 448, None, 1024), (40, 448, None, 896), (32, 512, None, 1024), (40, 500, None, 1024),
+    (8, 380, None, 768), (32, 450, (1, 0, 0), 1024), (80, 440, (1, 0, 0), 896), (320, 440, (1, 0, 0), 896),
+    (8, 512, (0, 1, 0), 512), (64, 512, (1, 1, 0), 512), (80, 512, (1, 1, 0), 512), (320, 512, (1, 1, 0), 512),
+    (64, 896, (1, 1, 0), 896), (320, 896, (1, 1, 0), 896), (16, 1024, (1, 1, 0), 1024), (320, 1024, (1, 1, 0), 1024),
     (20, 600, None, 2048), (300, 1030, None, 4096), (60, 700, (1, 0, 0), 2048)])
 def test_fields(gpu_lib, oracle, nx, ny, periodic, py):
     kw = problem(nx, ny, 1, d=(3e-9, 2.5e-9, 2e-9), seed=97)
