@@ -44,8 +44,9 @@ __global__ void __launch_bounds__(kThreads) y_forward_kernel(const ColPass p) {
 }
 
 // Y[c][z][ky][kx] -> X[c][z][y<ny][kx] (inverse along y, only physical rows kept)
-// (two CTAs named: columns_conv.cu; the forward pass loads in batches and needs no such help)
-__global__ void __launch_bounds__(kThreads, 2) y_inverse_kernel(const ColPass p) {
+// (WIDE: long_butterflies, columns.cuh; the forward pass loads in batches and needs no such help)
+template <bool WIDE>
+__global__ void __launch_bounds__(kThreads, general_ctas(WIDE)) y_inverse_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     extern __shared__ __align__(16) unsigned char smem[];
@@ -312,9 +313,10 @@ cudaError_t launch_y_forward(const ColPass &p, cudaStream_t s) {
 cudaError_t launch_y_inverse(const ColPass &p, cudaStream_t s) {
     if (y_fused_ok(p.g)) return (p.g.per & 2) ? launch_y_dispatch<true, true>(p, s) : launch_y_dispatch<true, false>(p, s);
     const size_t sm = 2 * sizeof(float2) * (size_t)p.tx * skewed_len(p.g.py);
-    cudaError_t e = ensure_smem((const void *)y_inverse_kernel, sm);
+    const auto fn = long_butterflies(p.plan) ? y_inverse_kernel<true> : y_inverse_kernel<false>;
+    cudaError_t e = ensure_smem((const void *)fn, sm);
     if (e != cudaSuccess) return e;
-    return launch_pdl(y_inverse_kernel, dim3(tiles(p), p.g.nz, 3), dim3(kThreads), sm, s, p);
+    return launch_pdl(fn, dim3(tiles(p), p.g.nz, 3), dim3(kThreads), sm, s, p);
 }
 
 cudaError_t load_finalize_stats() {

@@ -12,16 +12,15 @@ FM_LENGTHS_TO_256(FM_DECLARE) FM_LENGTHS_LONG(FM_DECLARE)
 
 namespace {
 
-// The general passes wait for shared memory and twiddles; with two CTAs named (what their buffers
-// leave room for) the compiler keeps the loads of a radix-16 butterfly in flight together, in 96
-// registers, instead of 54 to 64 (y+z of 60x45x6: 24.7 -> 22.8 us, y inverse of 30x600x30 in
-// columns.cu: 69.6 -> 61.3 us per launch).
+// (two CTAs named as in long_butterflies; the y+z pass gains at every length: 60x45x6 24.7 -> 22.8 us
+// per launch, 100x90x5 32.1 -> 30.9)
 __global__ void __launch_bounds__(kThreads, 2) yz_convolve_general_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     yz_convolve_general_body(p, blockIdx.x);
 }
-__global__ void __launch_bounds__(kThreads, 2) y_convolve_2d_general_kernel(const ColPass p) {
+template <bool WIDE>
+__global__ void __launch_bounds__(kThreads, general_ctas(WIDE)) y_convolve_2d_general_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     y_convolve_2d_general_body(p, blockIdx.x);
@@ -66,7 +65,8 @@ size_t y_convolve_2d_batched_smem(const Grid &g, int tx) {
 cudaError_t launch_y_convolve_2d(const ColPass &p, cudaStream_t s) {
     const size_t sm = y_convolve_2d_smem(p.g, p.tx);
     const ConvKernels &k = conv_kernels_for(p.g.py);
-    const ColKernel fn = !y2d_two_level(p.g) ? y_convolve_2d_general_kernel
+    const ColKernel general = long_butterflies(p.plan) ? y_convolve_2d_general_kernel<true> : y_convolve_2d_general_kernel<false>;
+    const ColKernel fn = !y2d_two_level(p.g) ? general
                          : (p.g.per & 2)    ? k.film_full
                          : p.g.per          ? k.film_per
                                             : k.film;

@@ -2537,6 +2537,10 @@ bool Engine::autotune() {
     // one (256x64 film, RK4: 0.0645 ms/step with 65 thin-film CTAs against 0.0755 with 129, which
     // timed alike on their own; 64x32x4 Heun, 16 steps: 524 us with 64 row-pass CTAs, 550 with
     // 128; but 256x256 periodic film, 20 RK4 steps: 1.12 ms with 33 thin-film CTAs, 1.25 with 17).
+    // Passes of more than 30 us take the fastest: they do not wait for one another's launch
+    // (464x34x4 periodic, x half length 8 x 29: a row pass of 104 us with 136 CTAs and 107 with 68,
+    // an RK4 step of 611 and 715 us).
+    constexpr float kEarlyTile = 3 * 0.030f;  // ms of the three launches that time_ms returns
     auto pick_tile = [&](const std::vector<std::pair<int, float>> &cand, int cur, int units) {
         if (cand.empty()) return cur;
         float bt = 1e30f;
@@ -2546,7 +2550,7 @@ bool Engine::autotune() {
                 bt = c.second;
                 best = c.first;
             }
-        if (early_launch)
+        if (early_launch && bt <= kEarlyTile)
             for (const auto &c : cand)
                 if (c.second <= 1.05f * bt && c.first > best && units / c.first >= 32) best = c.first;
         return best;

@@ -208,6 +208,19 @@ bool newell_periodic_spectrum_gpu(const Grid &g, double dx, double dy, double dz
                                   float2 *kern, double2 *kern64, cudaStream_t s, std::string &err);
 // K[c][kz][ky][kx] -> K[c][kz][kx][ky] (the fused y+z path's layout), out of place
 cudaError_t launch_kern_ky_fast(const float *in, float *out, int ncomp, int nkz, int nky, int nkx, cudaStream_t s);
+// CTAs per SM that a general pass is compiled for, by the line's plan.  Powers of two (radix 16) and
+// prime radices above 7 wait for shared memory and twiddles: two CTAs, which their buffers leave room
+// for, give the compiler 96 registers for the loads of a whole butterfly.  Lengths of radices 2 to 8
+// are shorter chains and gain from more CTAs.  y inverse, us per launch at 96 and 54 registers: 2048
+// points (200x700x8) 107 and 123, 77 points (64x77x4) 15.7 and 20.9; 500 points (400x500x4) 24.9 and
+// 20.8, 200 points (256x100x16) 29.0 and 25.0.
+inline bool long_butterflies(const FftPlan &p) {
+    for (int s = 0; s < p.nstages; ++s)
+        if (p.radix[s] > 8) return true;
+    return p.log2n >= 4;
+}
+__host__ __device__ constexpr int general_ctas(bool wide) { return wide ? 2 : 0; }  // 0: left to the compiler
+
 size_t z_convolve_smem(const Grid &g, int tx);
 // the packed ky-pair z pass exists for this grid at tile tx / the register z pass exists
 bool z_convolve_pair_ok(const Grid &g, int tx);

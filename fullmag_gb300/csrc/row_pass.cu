@@ -51,6 +51,7 @@ cudaError_t launch_row_pass(const RowPass &p, cudaStream_t s) {
     const RowKernels &k = row_kernels_for(length);
     const bool lean = row_lean(p, length > 0);
     const RowKernel fn = length && (p.g.per & 1)                                ? k.periodic[lean]
+                         : !length && (p.x_in || p.x_out) && long_butterflies(p.xplan) ? k.wide[lean]
                          : lean && k.dense && row_pass_blocks(p) >= kDenseCtas ? k.dense
                                                                                : k.open[lean];
     cudaError_t e = ensure_smem((const void *)fn, sm);

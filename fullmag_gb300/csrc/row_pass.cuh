@@ -25,10 +25,10 @@
 namespace fm {
 
 // The kernels of one x length, each length compiled in row_pass_lengths.cu ([0] everything,
-// [1] intermediate stages, dense those of large grids).
+// [1] intermediate stages, dense those of large grids; any length: wide, long_butterflies).
 using RowKernel = void (*)(const RowPass);
 struct RowKernels {
-    RowKernel open[2], periodic[2], adj, dense;
+    RowKernel open[2], periodic[2], adj, dense, wide[2];
 };
 template <int HALF>
 const RowKernels &row_kernels_of();
@@ -978,8 +978,8 @@ constexpr int row_ctas(int half) { return half > 256 || half == -3 ? 2 : 3; }
 constexpr bool row_dense_ok(int half) { return half >= 64 && half <= 256; }
 constexpr int kDenseCtas = 152 * 4 * 2;
 
-template <int HALF, bool PX, bool LEAN, bool DENSE = false>
-__global__ void __launch_bounds__(kThreads, DENSE ? 4 : row_ctas(HALF)) row_pass_kernel(const RowPass p) {
+template <int HALF, bool PX, bool LEAN, bool DENSE = false, bool WIDE = false>
+__global__ void __launch_bounds__(kThreads, DENSE ? 4 : WIDE ? 2 : row_ctas(HALF)) row_pass_kernel(const RowPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     row_pass_body<HALF, PX, false, LEAN>(p, blockIdx.x, gridDim.x);
@@ -1004,6 +1004,10 @@ RowKernels row_kernels() {
             k.periodic[lean] = lean ? row_pass_kernel<HALF, true, true> : row_pass_kernel<HALF, true, false>;
     }
     k.adj = row_pass_adj_kernel<HALF>;
+    if constexpr (HALF == 0) {
+        k.wide[0] = row_pass_kernel<0, false, false, false, true>;
+        k.wide[1] = row_pass_kernel<0, false, true, false, true>;
+    }
     if constexpr (row_dense_ok(HALF)) k.dense = row_pass_kernel<HALF, false, true, true>;
     return k;
 }
