@@ -18,6 +18,7 @@ namespace fm {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory of an SM that CTAs can have
 
 __device__ __forceinline__ void kernel_mirror(int k, int p, int &km, float &sg) {
     if (k > p / 2) {

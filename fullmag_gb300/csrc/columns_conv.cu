@@ -12,9 +12,11 @@ FM_LENGTHS_TO_256(FM_DECLARE) FM_LENGTHS_LONG(FM_DECLARE)
 
 namespace {
 
-// (two CTAs named as in long_butterflies; the y+z pass gains at every length: 60x45x6 24.7 -> 22.8 us
-// per launch, 100x90x5 32.1 -> 30.9)
-__global__ void __launch_bounds__(kThreads, 2) yz_convolve_general_kernel(const ColPass p) {
+// (two CTAs named as in long_butterflies; the y+z pass gains at every length, 60x45x6 24.7 -> 22.8 us
+// per launch, 100x90x5 32.1 -> 30.9, unless its CTAs want more than two per SM: 300x2x20, 321 CTAs of
+// 10 KB, 12.3 us at 64 registers and 16.3 at 96)
+template <bool WIDE>
+__global__ void __launch_bounds__(kThreads, general_ctas(WIDE)) yz_convolve_general_kernel(const ColPass p) {
     pdl_wait();
     if (p.early) pdl_trigger();
     yz_convolve_general_body(p, blockIdx.x);
@@ -47,7 +49,10 @@ cudaError_t launch_yz_convolve(const ColPass &p, cudaStream_t s) {
     if (p.g.per) return cudaErrorInvalidValue;  // the fused y+z pass reads the octant kernel only
     const size_t sm = yz_convolve_smem(p.g, p.tx);
     const ConvKernels &k = conv_kernels_for(p.g.py);
-    const ColKernel fn = yz_fused_ok(p.g) ? (p.g.pz <= 8 ? k.yz : k.yz_big) : yz_convolve_general_kernel;
+    const bool wide = tiles(p) <= 2 * 152 || sm > kMaxSmem / 3;
+    const ColKernel fn = yz_fused_ok(p.g) ? (p.g.pz <= 8 ? k.yz : k.yz_big)
+                         : wide           ? yz_convolve_general_kernel<true>
+                                          : yz_convolve_general_kernel<false>;
     cudaError_t e = ensure_smem((const void *)fn, sm);
     if (e != cudaSuccess) return e;
     return launch_pdl(fn, dim3(tiles(p)), dim3(kThreads), sm, s, p);
