@@ -395,8 +395,10 @@ cudaError_t launch_z_register(const ColPass &p, cudaStream_t s) {
 }
 }  // namespace
 
-// the packed ky-pair z pass: tile 8, inner radix 4 to 8
-bool z_convolve_pair_ok(const Grid &g, int tx) { return tx == 8 && z_fused_ok(g) && g.pz >= 32 && g.pz <= 128; }
+// the packed ky-pair z pass: tile 8, inner radix 4 to 8, kernel rows at 16-byte boundaries (cp.async)
+bool z_convolve_pair_ok(const Grid &g, int tx) {
+    return tx == 8 && z_fused_ok(g) && g.pz >= 32 && g.pz <= 128 && g.ks % 4 == 0;
+}
 bool z_register_length_ok(int pz) { return z_register_length(pz); }
 bool z_convolve_register_ok(const Grid &g) {
     return !(g.per & 4) && z_register_length(g.pz) && 2 * g.nz <= g.pz && (long long)g.py * g.nkx < (1ll << 30);
